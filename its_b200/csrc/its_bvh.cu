@@ -40,7 +40,7 @@ struct BvhDevice {
 //     (area-weighted centroid sum / area), squared radius (+inf for a node without area, which
 //     the far-field test then never accepts), normal sum, the second-order tensor's trace,
 //     diagonal and summed off-diagonal pairs (all that the expansion uses), and the children.
-//   * the leaves' triangles (9 doubles each, in leaf order).
+//   * the leaves' triangles in leaf order.
 struct __align__(16) WideSlot {
   float lo[3], hi[3];
   int32_t code;    // a wide node's index, or the first leaf of a bucket
@@ -71,6 +71,7 @@ struct NodeSums {
   double lo[3], hi[3], an[3], ac[3], area, sm[9];
 };
 constexpr int kSumWords = sizeof(NodeSums) / 8;
+constexpr int kTriWords = 10;  // a leaf triangle's nine coordinates, padded to whole 16-byte loads
 
 __global__ void kCentroidBounds(const double* __restrict__ V, const int32_t* __restrict__ F, int64_t nf,
                                 double* __restrict__ partial) {
@@ -154,39 +155,106 @@ __global__ void kBuildInternal(const uint32_t* __restrict__ codes, int64_t n, in
   parent[R < 0 ? (n - 1) + (-R - 1) : R] = (int32_t)i;
 }
 
-// Leaf data, then climb: the second child to arrive at a node merges both, writes the node's
-// box and expansion and goes on. A block's leaves are consecutive, so a node whose range lies
-// inside them is merged by the block's own threads, the first arrival's sums waiting in shared
-// memory ([word][slot]; slot = 2 (node - first leaf) + side: Karras numbers a node by an end of
-// its range, so the node's index lies in the block too). Only the maximal subtrees of a block
-// (a dozen of 128 leaves) climb on through global memory, where the first arrival's sums wait
-// at its first leaf's place: a node's place is its left child's, whose sums the merging thread
-// has read by then. One thread per leaf climbing through global memory all the way, with the
-// sums in arrays of their own and a packing pass over them, moved 0.9 GB and took 823 + 110 us
-// at 1,048,576 triangles.
+// The node's box, rounded outward.
+__device__ __forceinline__ BoxF outwardBox(const NodeSums& S) {
+  BoxF b;
+  for (int a = 0; a < 3; ++a) {
+    b.lo[a] = __double2float_rd(S.lo[a]);
+    b.hi[a] = __double2float_ru(S.hi[a]);
+  }
+  return b;
+}
+__device__ __forceinline__ void mergeSums(NodeSums& S, const NodeSums& O) {
+  for (int a = 0; a < 3; ++a) {
+    S.lo[a] = fmin(S.lo[a], O.lo[a]);
+    S.hi[a] = fmax(S.hi[a], O.hi[a]);
+    S.an[a] = S.an[a] + O.an[a];
+    S.ac[a] = S.ac[a] + O.ac[a];
+  }
+  S.area = S.area + O.area;
+  for (int e = 0; e < 9; ++e) S.sm[e] = S.sm[e] + O.sm[e];
+}
+__device__ __forceinline__ FwnNode fwnNode(const NodeSums& S, int32_t left, int32_t right) {
+  FwnNode f;
+  f.r2 = __longlong_as_double(0x7ff0000000000000ll);  // +inf: no far-field term without area
+  for (int a = 0; a < 3; ++a) {
+    f.an[a] = S.an[a];
+    f.c[a] = S.area > 0.0 ? S.ac[a] / S.area : 0.0;
+  }
+  if (S.area > 0.0) {
+    double r2 = 0.0;
+    for (int a = 0; a < 3; ++a) {
+      const double e = fmax(f.c[a] - S.lo[a], S.hi[a] - f.c[a]);
+      r2 += e * e;
+    }
+    f.r2 = r2;
+  }
+  double m[9];
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j) m[3 * i + j] = S.sm[3 * i + j] - f.an[i] * f.c[j];
+  f.tr = m[0] + m[4] + m[8];
+  f.dg[0] = m[0];
+  f.dg[1] = m[4];
+  f.dg[2] = m[8];
+  f.of[0] = m[1] + m[3];
+  f.of[1] = m[2] + m[6];
+  f.of[2] = m[5] + m[7];
+  f.child[0] = left;
+  f.child[1] = right;
+  f.pad[0] = f.pad[1] = 0;
+  return f;
+}
+
+// Leaf data, then climb: the second child to arrive at a node merges both and goes on. A block's
+// leaves are consecutive, so a node whose range lies inside them is merged by the block's own
+// threads, every node's sums in shared memory ([word][slot]: the leaves, then the inner nodes,
+// whose indices lie in the block too, since Karras numbers a node by an end of its range). The
+// tree's links come in beforehand, and the winding records are formed afterwards, a thread per
+// node, so that a step of the climb is a merge and nothing else. The maximal subtrees of a block
+// (a dozen of 128 leaves) are left for kClimbTop, their sums at their first leaf's place in raw
+// and their node and first leaf listed in top. One thread per leaf climbing through global memory all the way, with
+// the sums in arrays of their own and a packing pass over them, moved 0.9 GB and took 823 + 110
+// us at 1,048,576 triangles; now 183 us and kClimbTop.
 constexpr int kUpLeaves = 128;
 __global__ void __launch_bounds__(kUpLeaves) kBottomUp(const double* __restrict__ V, const int32_t* __restrict__ F,
-                                                       BvhDevice B, double* __restrict__ raw, BoxF* __restrict__ box,
+                                                       BvhDevice B, double* __restrict__ raw, int2* __restrict__ top,
+                                                       unsigned* __restrict__ topCount, BoxF* __restrict__ box,
                                                        FwnNode* __restrict__ fwn, double* __restrict__ tris) {
   __shared__ double sSum[kSumWords][2 * kUpLeaves];
   __shared__ unsigned sFlag[kUpLeaves];
+  __shared__ int32_t sParent[2 * kUpLeaves], sLeft[kUpLeaves], sRight[kUpLeaves];
+  __shared__ int2 sRange[kUpLeaves];
+  __shared__ int sTops, sTopBase;
   const int64_t n = B.nf;
-  const int64_t k0 = (int64_t)blockIdx.x * kUpLeaves, k = k0 + threadIdx.x;
+  const int64_t k0 = (int64_t)blockIdx.x * kUpLeaves;
+  const int i = threadIdx.x;
+  const int64_t k = k0 + i;
   const int64_t kEnd = k0 + kUpLeaves < n ? k0 + kUpLeaves : n;
-  sFlag[threadIdx.x] = 0;
-  __syncthreads();
-  if (k >= n) return;
+  sFlag[i] = 0;
+  if (i == 0) sTops = 0;
+  sRange[i] = make_int2(-1, -1);
+  if (k < n - 1) {
+    sParent[kUpLeaves + i] = B.parent[k];
+    sLeft[i] = B.left[k];
+    sRight[i] = B.right[k];
+    sRange[i] = ((const int2*)B.range)[k];
+  }
   NodeSums S;
-  int64_t node = (n - 1) + k, first = k, last = k;
-  {
+  const double* mine = (const double*)&S;
+  if (k < n) {
+    sParent[i] = B.parent[(n - 1) + k];
     const uint32_t t = B.leafTri[k];
     double p[3][3];
     for (int c = 0; c < 3; ++c) {
       const int64_t vi = F[3 * (int64_t)t + c];
       for (int a = 0; a < 3; ++a) p[c][a] = V[3 * vi + a];
     }
-    for (int c = 0; c < 3; ++c)
-      for (int a = 0; a < 3; ++a) tris[9 * k + 3 * c + a] = p[c][a];
+    double2* dst = (double2*)(tris + kTriWords * k);
+    dst[0] = make_double2(p[0][0], p[0][1]);
+    dst[1] = make_double2(p[0][2], p[1][0]);
+    dst[2] = make_double2(p[1][1], p[1][2]);
+    dst[3] = make_double2(p[2][0], p[2][1]);
+    dst[4] = make_double2(p[2][2], 0.0);
     const double u[3] = {p[1][0] - p[0][0], p[1][1] - p[0][1], p[1][2] - p[0][2]};
     const double v[3] = {p[2][0] - p[0][0], p[2][1] - p[0][1], p[2][2] - p[0][2]};
     const double an[3] = {0.5 * (u[1] * v[2] - u[2] * v[1]), 0.5 * (u[2] * v[0] - u[0] * v[2]),
@@ -198,85 +266,100 @@ __global__ void __launch_bounds__(kUpLeaves) kBottomUp(const double* __restrict_
       S.ac[a] = ar * (p[0][a] + p[1][a] + p[2][a]) / 3.0;
       S.an[a] = an[a];
     }
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) S.sm[3 * i + j] = an[i] * ((p[0][j] + p[1][j] + p[2][j]) / 3.0);
+    for (int r = 0; r < 3; ++r)
+      for (int j = 0; j < 3; ++j) S.sm[3 * r + j] = an[r] * ((p[0][j] + p[1][j] + p[2][j]) / 3.0);
     S.area = ar;
+    box[(n - 1) + k] = outwardBox(S);
   }
-  if (n == 1) return;
-  while (true) {
-    // this node's box for the wide tree's slots
-    BoxF bf;
-    for (int a = 0; a < 3; ++a) {
-      bf.lo[a] = __double2float_rd(S.lo[a]);
-      bf.hi[a] = __double2float_ru(S.hi[a]);
+  __syncthreads();
+  int place = -1;  // of the maximal subtree that this thread ends at
+  int2 found = make_int2(0, 0);
+  if (k < n) {
+    int slot = i;
+    int64_t first = k;
+    while (true) {
+      const int32_t par = sParent[slot];
+      if (par < 0) break;  // the root
+      const bool inside = par >= k0 && par < kEnd && sRange[par - k0].x >= k0 && sRange[par - k0].y < kEnd;
+      if (!inside) {
+        double* dst = raw + kSumWords * first;
+#pragma unroll
+        for (int w = 0; w < kSumWords; ++w) dst[w] = mine[w];
+        place = atomicAdd(&sTops, 1);
+        found = make_int2((int32_t)(slot < kUpLeaves ? (n - 1) + k0 + slot : k0 + slot - kUpLeaves), (int32_t)first);
+        break;
+      }
+      const int pi = (int)(par - k0);
+      if (slot < kUpLeaves) {  // an inner node's sums went in when it was merged
+#pragma unroll
+        for (int w = 0; w < kSumWords; ++w) sSum[w][slot] = mine[w];
+      }
+      __threadfence_block();
+      if (atomicAdd(&sFlag[pi], 1u) == 0) break;  // first arrival: the sibling merges
+      __threadfence_block();
+      const int32_t l = sLeft[pi], r = sRight[pi];
+      const int ls = l < 0 ? (int)(-(int64_t)l - 1 - k0) : (int)(l - k0) + kUpLeaves;
+      const int rs = r < 0 ? (int)(-(int64_t)r - 1 - k0) : (int)(r - k0) + kUpLeaves;
+      const int os = ls == slot ? rs : ls;
+      NodeSums O;
+      double* other = (double*)&O;
+#pragma unroll
+      for (int w = 0; w < kSumWords; ++w) other[w] = ((volatile double*)sSum[w])[os];
+      mergeSums(S, O);
+      slot = kUpLeaves + pi;
+      first = sRange[pi].x;
+#pragma unroll
+      for (int w = 0; w < kSumWords; ++w) sSum[w][slot] = mine[w];
     }
-    box[node] = bf;
+  }
+  __syncthreads();
+  if (i == 0 && sTops) sTopBase = (int)atomicAdd(topCount, (unsigned)sTops);
+  if (sRange[i].x >= k0 && sRange[i].y < kEnd) {
+    NodeSums N;
+    double* to = (double*)&N;
+#pragma unroll
+    for (int w = 0; w < kSumWords; ++w) to[w] = sSum[w][kUpLeaves + i];
+    box[k] = outwardBox(N);
+    fwn[k] = fwnNode(N, sLeft[i], sRight[i]);
+  }
+  __syncthreads();
+  if (place >= 0) top[sTopBase + place] = found;
+}
+
+// The nodes above the blocks' maximal subtrees, a thread per subtree: the first arrival's sums
+// wait at its first leaf's place; a node's place is its left child's, whose sums the merging
+// thread has read by then.
+__global__ void __launch_bounds__(128) kClimbTop(BvhDevice B, double* __restrict__ raw, const int2* __restrict__ top,
+                                                 const unsigned* __restrict__ topCount, BoxF* __restrict__ box,
+                                                 FwnNode* __restrict__ fwn) {
+  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (k >= *topCount) return;
+  int64_t node = top[k].x, first = top[k].y;
+  NodeSums S;
+  double* mine = (double*)&S;
+#pragma unroll
+  for (int w = 0; w < kSumWords; ++w) mine[w] = raw[kSumWords * first + w];
+  while (true) {
     const int32_t par = B.parent[node];
     if (par < 0) return;
-    const int32_t r0 = B.range[2 * par], r1 = B.range[2 * par + 1];
-    const int side = first != r0;  // 0: the left child
-    const double* mine = (const double*)&S;
+    __threadfence();
+    if (atomicAdd(B.flag + par, 1u) == 0) return;  // first arrival: the sibling merges
+    __threadfence();
+    const int32_t r0 = B.range[2 * (int64_t)par], l = B.left[par], r = B.right[par];
+    const int64_t rFirst = r < 0 ? -(int64_t)r - 1 : B.range[2 * (int64_t)r];
+    const volatile double* src = raw + kSumWords * (first == r0 ? rFirst : (int64_t)r0);
     NodeSums O;
     double* other = (double*)&O;
-    if (r0 >= k0 && r1 < kEnd) {
-      const int slot = 2 * (int)(par - k0);
 #pragma unroll
-      for (int w = 0; w < kSumWords; ++w) sSum[w][slot + side] = mine[w];
-      __threadfence_block();
-      if (atomicAdd(&sFlag[par - k0], 1u) == 0) return;  // first arrival: the sibling merges
-      __threadfence_block();
-#pragma unroll
-      for (int w = 0; w < kSumWords; ++w) other[w] = ((volatile double*)sSum[w])[slot + 1 - side];
-    } else {
-      double* dst = raw + kSumWords * first;
-#pragma unroll
-      for (int w = 0; w < kSumWords; ++w) dst[w] = mine[w];
-      __threadfence();
-      if (atomicAdd(B.flag + par, 1u) == 0) return;
-      __threadfence();
-      const volatile double* src = raw + kSumWords * (int64_t)(side ? r0 : last + 1);
-#pragma unroll
-      for (int w = 0; w < kSumWords; ++w) other[w] = src[w];
-    }
-    for (int a = 0; a < 3; ++a) {
-      S.lo[a] = fmin(S.lo[a], O.lo[a]);
-      S.hi[a] = fmax(S.hi[a], O.hi[a]);
-      S.an[a] = S.an[a] + O.an[a];
-      S.ac[a] = S.ac[a] + O.ac[a];
-    }
-    S.area = S.area + O.area;
-    for (int e = 0; e < 9; ++e) S.sm[e] = S.sm[e] + O.sm[e];
+    for (int w = 0; w < kSumWords; ++w) other[w] = src[w];
+    mergeSums(S, O);
     node = par;
     first = r0;
-    last = r1;
-    FwnNode f;
-    f.r2 = __longlong_as_double(0x7ff0000000000000ll);  // +inf: no far-field term without area
-    for (int a = 0; a < 3; ++a) {
-      f.an[a] = S.an[a];
-      f.c[a] = S.area > 0.0 ? S.ac[a] / S.area : 0.0;
-    }
-    if (S.area > 0.0) {
-      double r2 = 0.0;
-      for (int a = 0; a < 3; ++a) {
-        const double e = fmax(f.c[a] - S.lo[a], S.hi[a] - f.c[a]);
-        r2 += e * e;
-      }
-      f.r2 = r2;
-    }
-    double m[9];
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) m[3 * i + j] = S.sm[3 * i + j] - f.an[i] * f.c[j];
-    f.tr = m[0] + m[4] + m[8];
-    f.dg[0] = m[0];
-    f.dg[1] = m[4];
-    f.dg[2] = m[8];
-    f.of[0] = m[1] + m[3];
-    f.of[1] = m[2] + m[6];
-    f.of[2] = m[5] + m[7];
-    f.child[0] = B.left[par];
-    f.child[1] = B.right[par];
-    f.pad[0] = f.pad[1] = 0;
-    fwn[par] = f;
+    volatile double* dst = raw + kSumWords * first;
+#pragma unroll
+    for (int w = 0; w < kSumWords; ++w) dst[w] = mine[w];
+    box[par] = outwardBox(S);
+    fwn[par] = fwnNode(S, l, r);
   }
 }
 
@@ -345,30 +428,39 @@ __global__ void __launch_bounds__(128) kWideNodes(BvhDevice B, const BoxF* __res
 }
 
 // ---- the walks: eight lanes per query ------------------------------------------------------
-// A warp walks four queries at a time, eight lanes each, taken in the Morton order of their
-// positions from a run of kRun queries of its own: a group that has finished takes the run's
-// next query while the others go on (queries differ tenfold in their visits: far from the
-// surface many boxes are about equally near). A thread per query kept 7.6 of 32 lanes busy and
-// waited on its dependent node loads: 7.57 ms at 196,681 queries against 1,048,576 triangles.
-constexpr int kWalkThreads = 128, kGroups = kWalkThreads / 8, kRun = 16;
+// A warp walks four queries at a time, eight lanes each, in the Morton order of their positions:
+// a group that has finished takes the next query from a counter while the others go on (queries
+// differ tenfold in their visits: far from the surface many boxes are about equally near). A
+// thread per query kept 7.6 of 32 lanes busy and waited on its dependent node loads: 7.57 ms at
+// 196,681 queries against 1,048,576 triangles. A fixed run of 16 queries per warp left the SMs
+// idle for 38 % of the nearest walk, waiting for the runs with many far queries.
+constexpr int kWalkThreads = 128, kGroups = kWalkThreads / 8;
 // The tree's keys are 30 bits of position and an index: at most 62 binary levels. A wide node
-// spans at least three of them and leaves seven others on the stack; the winding walk takes
-// eight nodes from the top, so no level but the two on top keeps more than eight.
-constexpr int kNearStack = 7 * 21 + 8, kFwnStack = 8 * 62 + 16;
+// spans at least three of them and leaves seven others on the stack. The winding walk takes eight
+// nodes at a time (each may leave two) while its stack is short, else one at a time, which adds
+// at most one entry per level (short below 32, 64, 128, 256 or 400 entries: 5.8, 4.6, 4.6, 5.0,
+// 5.5 ms for the call: a longer stack takes shared memory from the L1 and the resident blocks).
+constexpr int kTreeLevels = 62, kNearStack = 7 * ((kTreeLevels + 2) / 3) + 8;
+constexpr int kWideFwn = 64, kFwnStack = kWideFwn + 16 + kTreeLevels + 2;
 
-struct QueryRun {  // the next query of the warp's run for each group that needs one
-  int64_t next, end;
-  __device__ QueryRun(int64_t m) {
-    next = ((int64_t)blockIdx.x * (kWalkThreads / 32) + (threadIdx.x >> 5)) * kRun;
-    end = next + kRun < m ? next + kRun : m;
-  }
-  __device__ int64_t take(bool need, int lane) {
-    const unsigned b = __ballot_sync(0xffffffffu, need && (lane & 7) == 0);
-    const int64_t q = next + __popc(b & ((1u << (lane & 24)) - 1u));
-    next += __popc(b);
-    return need && q < end ? q : -1;
-  }
-};
+// The next query of each of the warp's groups that needs one, or -1.
+__device__ __forceinline__ int64_t takeQuery(bool need, int lane, int64_t m, unsigned long long* counter) {
+  const unsigned b = __ballot_sync(0xffffffffu, need && (lane & 7) == 0);
+  if (!b) return -1;
+  unsigned long long base = 0;
+  if (lane == 0) base = atomicAdd(counter, (unsigned long long)__popc(b));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  const int64_t q = (int64_t)base + __popc(b & ((1u << (lane & 24)) - 1u));
+  return need && q < m ? q : -1;
+}
+// A leaf triangle.
+__device__ __forceinline__ void loadTri(const double* __restrict__ tris, int64_t leaf, D3& a, D3& b, D3& c) {
+  const double2* v = (const double2*)(tris + kTriWords * leaf);
+  const double2 v0 = __ldg(v), v1 = __ldg(v + 1), v2 = __ldg(v + 2), v3 = __ldg(v + 3), v4 = __ldg(v + 4);
+  a = D3{v0.x, v0.y, v1.x};
+  b = D3{v1.y, v2.x, v2.y};
+  c = D3{v3.x, v3.y, v4.x};
+}
 
 __device__ __forceinline__ double groupMin(double v) {
 #pragma unroll
@@ -385,22 +477,24 @@ __device__ __forceinline__ double groupSum(double v) {
 // bound of its box's squared distance (FP32, every operation rounded down) is beyond the best
 // squared distance times (1 + 1e-12), so the minimum is the IEEE value the brute force finds.
 // A bucket's triangles are tested together, one per lane.
-__global__ void __launch_bounds__(kWalkThreads) kNearest(const double* __restrict__ P, int64_t m,
+__global__ void __launch_bounds__(kWalkThreads, 6) kNearest(const double* __restrict__ P, int64_t m,
                                                          const uint32_t* __restrict__ order,
                                                          const WideNode* __restrict__ wide,
-                                                         const double* __restrict__ tris, double* __restrict__ out) {
+                                                         const double* __restrict__ tris, double* __restrict__ out,
+                                                         unsigned long long* __restrict__ counter) {
   __shared__ int2 sStack[kGroups][kNearStack];  // wide node, lower bound
   const int lane = threadIdx.x & 31, j = lane & 7, shift = lane & 24;
   int2* stack = sStack[threadIdx.x >> 3];
-  QueryRun run(m);
   int64_t qi = -1;
+  bool drained = false;  // no query is left for this group
   D3 q{0, 0, 0};
   float qlo[3] = {0, 0, 0}, qhi[3] = {0, 0, 0};
   double best = 0.0;
   float bound = 0.0f;
   int sp = 0;
   while (true) {
-    const int64_t got = run.take(qi < 0, lane);
+    const int64_t got = takeQuery(qi < 0 && !drained, lane, m, counter);
+    drained = drained || (qi < 0 && got < 0);
     if (got >= 0) {
       qi = order[got];
       q = D3{P[3 * qi], P[3 * qi + 1], P[3 * qi + 2]};
@@ -451,8 +545,8 @@ __global__ void __launch_bounds__(kWalkThreads) kNearest(const double* __restric
       const bool mine = qi >= 0 && count > 0 && j < count && db <= bound;
       double t2 = 1.7976931348623157e308;
       if (mine) {
-        const double* v = tris + 9 * ((int64_t)first + j);
-        const D3 a{v[0], v[1], v[2]}, b{v[3], v[4], v[5]}, c{v[6], v[7], v[8]};
+        D3 a, b, c;
+        loadTri(tris, (int64_t)first + j, a, b, c);
         t2 = fmin(t2, pointTriSqDist(q, a, b, c));
       }
       best = fmin(best, groupMin(t2));
@@ -482,23 +576,27 @@ __global__ void __launch_bounds__(kWalkThreads) kNearest(const double* __restric
 // inner children back on the stack and its leaves on a list, whose exact solid angles are formed
 // eight at a time. The nodes accepted and opened are those of a walk one node at a time; the sum
 // is over lanes.
-__global__ void __launch_bounds__(kWalkThreads) kWinding(const double* __restrict__ P, int64_t m,
+__global__ void __launch_bounds__(kWalkThreads, 6) kWinding(const double* __restrict__ P, int64_t m,
                                                          const uint32_t* __restrict__ order,
                                                          const FwnNode* __restrict__ W, const double* __restrict__ tris,
-                                                         int64_t n, double* __restrict__ out) {
+                                                         int64_t n, double* __restrict__ out,
+                                                         unsigned long long* __restrict__ counter) {
   __shared__ int32_t sStack[kGroups][kFwnStack];
+  __shared__ double2 sRec[kGroups][64];    // eight records; piece p of record r at p ^ r
   __shared__ int32_t sLeaves[kGroups][24];  // fewer than eight are left before sixteen more can come
   const int lane = threadIdx.x & 31, j = lane & 7, shift = lane & 24;
   const unsigned below = (1u << j) - 1u;
   int32_t* stack = sStack[threadIdx.x >> 3];
   int32_t* leaves = sLeaves[threadIdx.x >> 3];
-  QueryRun run(m);
+  double2* rec = sRec[threadIdx.x >> 3];
   int64_t qi = -1;
+  bool drained = false;  // no query is left for this group
   D3 q{0, 0, 0};
   double w = 0.0;
   int sp = 0, nl = 0;
   while (true) {
-    const int64_t got = run.take(qi < 0, lane);
+    const int64_t got = takeQuery(qi < 0 && !drained, lane, m, counter);
+    drained = drained || (qi < 0 && got < 0);
     if (got >= 0) {
       qi = order[got];
       q = D3{P[3 * qi], P[3 * qi + 1], P[3 * qi + 2]};
@@ -512,15 +610,25 @@ __global__ void __launch_bounds__(kWalkThreads) kWinding(const double* __restric
     }
     if (!__any_sync(0xffffffffu, qi >= 0)) break;
     __syncwarp();
-    const int take = sp < 8 ? sp : 8;
+    const int take = sp > kWideFwn ? 1 : (sp < 8 ? sp : 8);
     const bool have = j < take;
     const int32_t node = have ? stack[sp - take + j] : 0;
     sp -= take;
     __syncwarp();
+    // the records come in a line at a time, a lane per 16 bytes (a lane loading its own record
+    // touches a line per lane and load: the L1 ran at 74 % and held the walk up)
+#pragma unroll
+    for (int o = 0; o < 8; ++o) {
+      const int32_t no = __shfl_sync(0xffffffffu, node, o, 8);
+      if (o < take) rec[8 * o + (j ^ o)] = __ldg((const double2*)(W + no) + j);
+    }
+    __syncwarp();
     bool near = false;
     int32_t c0 = 0, c1 = 0;
     if (have) {
-      const FwnNode& nd = W[node];
+      FwnNode nd;
+#pragma unroll
+      for (int p = 0; p < 8; ++p) ((double2*)&nd)[p] = rec[8 * j + (p ^ j)];
       const double d[3] = {nd.c[0] - q.x, nd.c[1] - q.y, nd.c[2] - q.z};
       const double R2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
       if (R2 > kFwnBeta * kFwnBeta * nd.r2) {  // the powers of 1/R from one reciprocal
@@ -553,8 +661,9 @@ __global__ void __launch_bounds__(kWalkThreads) kWinding(const double* __restric
     while (__any_sync(0xffffffffu, nl >= 8 || (sp == 0 && nl > 0))) {
       const int t = nl < 8 ? nl : 8;
       if (j < t) {
-        const double* v = tris + 9 * (int64_t)leaves[nl - t + j];
-        w += solidAngle(q, D3{v[0], v[1], v[2]}, D3{v[3], v[4], v[5]}, D3{v[6], v[7], v[8]});
+        D3 a, b, c;
+        loadTri(tris, leaves[nl - t + j], a, b, c);
+        w += solidAngle(q, a, b, c);
       }
       nl -= t;
       __syncwarp();
@@ -629,15 +738,24 @@ its_status sdfBvh(its_ctx* ctx, const double* dP, int64_t m, const double* dV, c
     ITS_LAUNCHED(ctx);
   }
   DevBuf<double> raw, tris;
+  DevBuf<int2> top;
+  DevBuf<unsigned> topCount;
+  DevBuf<unsigned long long> counters;
   DevBuf<BoxF> box;
   DevBuf<FwnNode> fwn;
   DevBuf<WideNode> wide;
-  if ((st = raw.alloc(ctx, kSumWords * nf)) != ITS_OK || (st = tris.alloc(ctx, 9 * nf)) != ITS_OK ||
+  if ((st = raw.alloc(ctx, kSumWords * nf)) != ITS_OK || (st = tris.alloc(ctx, kTriWords * nf)) != ITS_OK ||
+      (st = top.alloc(ctx, nf)) != ITS_OK || (st = topCount.zeros(ctx, 1)) != ITS_OK || (st = counters.zeros(ctx, 2)) != ITS_OK ||
       (st = box.alloc(ctx, nodes)) != ITS_OK || (st = fwn.alloc(ctx, inner)) != ITS_OK ||
       (st = wide.alloc(ctx, inner)) != ITS_OK)
     return st;
-  kBottomUp<<<gridFor(nf, kUpLeaves), kUpLeaves, 0, ctx->stream>>>(dV, dF, B, raw.p, box.p, fwn.p, tris.p);
+  kBottomUp<<<gridFor(nf, kUpLeaves), kUpLeaves, 0, ctx->stream>>>(dV, dF, B, raw.p, top.p, topCount.p, box.p, fwn.p,
+                                                               tris.p);
   ITS_LAUNCHED(ctx);
+  if (nf > kUpLeaves) {
+    kClimbTop<<<gridFor(nf, 128), 128, 0, ctx->stream>>>(B, raw.p, top.p, topCount.p, box.p, fwn.p);
+    ITS_LAUNCHED(ctx);
+  }
   kWideNodes<<<gridFor(inner, 128), 128, 0, ctx->stream>>>(B, box.p, wide.p);
   ITS_LAUNCHED(ctx);
   // the queries in Morton order
@@ -649,10 +767,10 @@ its_status sdfBvh(its_ctx* ctx, const double* dP, int64_t m, const double* dV, c
                                                        make_double3(inv[0], inv[1], inv[2]), qc.p, qi.p);
   ITS_LAUNCHED(ctx);
   if ((st = radixSortPairs(ctx, qc.p, qi.p, qsc.p, qorder.p, qtk.p, qtv.p, m, 30)) != ITS_OK) return st;
-  const unsigned blocks = gridFor(m, kRun * (kWalkThreads / 32));
-  kNearest<<<blocks, kWalkThreads, 0, ctx->stream>>>(dP, m, qorder.p, wide.p, tris.p, dOut);
+  const unsigned blocks = (unsigned)std::min<int64_t>(gridFor(m, kGroups), 6ll * ctx->numSMs);  // six fit an SM
+  kNearest<<<blocks, kWalkThreads, 0, ctx->stream>>>(dP, m, qorder.p, wide.p, tris.p, dOut, counters.p);
   ITS_LAUNCHED(ctx);
-  kWinding<<<blocks, kWalkThreads, 0, ctx->stream>>>(dP, m, qorder.p, fwn.p, tris.p, nf, dOut);
+  kWinding<<<blocks, kWalkThreads, 0, ctx->stream>>>(dP, m, qorder.p, fwn.p, tris.p, nf, dOut, counters.p + 1);
   ITS_LAUNCHED(ctx);
   return ITS_OK;
 }
