@@ -341,7 +341,11 @@ __global__ void __launch_bounds__(kBrickThreads, 2)
 // corners -- fieldAt's additions in fieldAt's order, so the field is bit-identical, at a few
 // table reads and three FP64 operations per term (the x*y factor is shared by a column's
 // points where they lie in one cell).
-constexpr int kSepX = 32, kSepY = 8, kSepThreads = kSepX * kSepY, kSepTileCap = 1024, kSepStageCap = 2048;
+constexpr int kSepX = 32, kSepY = 8, kSepThreads = kSepX * kSepY;
+// Staged corners per depth and in all. Grids at least twice as fine as the octree need at most
+// kSepTileCap; coarser ones (a point per finest cell: 34 x 10 x 10 corners a brick) get the larger
+// pair, 72 KB of shared memory and three blocks per SM instead of four.
+constexpr int kSepTileCap = 1024, kSepStageCap = 2048, kCoarseTileCap = 4608, kCoarseStageCap = 5632;
 template <typename T> struct Pair { typedef double2 type; };
 template <> struct Pair<float> { typedef float2 type; };
 
@@ -361,10 +365,13 @@ __global__ void kSepTables(const __grid_constant__ EvalParams P, double3 o, doub
   const double ga = a == 0 ? P.g.x : a == 1 ? P.g.y : P.g.z;
   const double pa = oa + (double)idx * va;
   const int64_t c = (int64_t)floor(divRn(pa - ga, w, wi));
+  // a cell outside the depth's lattice touches no corner: kept next to it, so that boxes stay small
+  const int64_t lim = (int64_t)(P.res >> d);
+  const int64_t cc = c < -2 ? -2 : (c > lim + 1 ? lim + 1 : c);
   double h[4];
 #pragma unroll
   for (int side = 0; side < 2; ++side) {
-    const int64_t X = c + side;
+    const int64_t X = cc + side;
     const double pA = latticePos(ga, w, (uint32_t)(X < 0 ? 0 : X));
     const double pB = X >= 1 ? latticePos(ga, w, (uint32_t)(X - 1)) + w : pA;
     h[2 * side] = hat1r(pa, pA, w, wi);
@@ -373,7 +380,7 @@ __global__ void kSepTables(const __grid_constant__ EvalParams P, double3 o, doub
   double2* dst = (double2*)(tabH + 4 * item);
   dst[0] = make_double2(h[0], h[1]);
   dst[1] = make_double2(h[2], h[3]);
-  tabC[item] = (int)c;
+  tabC[item] = (int)cc;
 }
 
 // One brick's hat tables and cell boxes: the hat factors and cells of the brick's coordinates
@@ -381,18 +388,20 @@ __global__ void kSepTables(const __grid_constant__ EvalParams P, double3 o, doub
 // corner's factors for a thread's points lie side by side and come in pairs), and the corner
 // boxes of every depth staged together in one pass (their lattice lookups are dependent loads:
 // in one pass their latencies overlap).
-template <typename T, int kSepZ>
+template <typename T, int kSepZ, bool kCoarse>
 struct alignas(16) SepStage {
+  static constexpr int kTile = kCoarse ? kCoarseTileCap : kSepTileCap;
+  static constexpr int kStage = kCoarse ? kCoarseStageCap : kSepStageCap;
   T hX[kMaxDepth][4][kSepX];  // [depth][corner side * 2 + corner bit][x]: a warp's x run reads side by side
   T hY[kMaxDepth][kSepY][4];
   T hZ[kMaxDepth][4][kSepZ];
-  T tLam[kSepStageCap];
+  T tLam[kStage];
   int cX[kMaxDepth][kSepX], cY[kMaxDepth][kSepY], cZ[kMaxDepth][kSepZ];
   int tOff[kMaxDepth], tEnd[kMaxDepth];  // depth d's tile: [tOff[d], tEnd[d]); tOff -1: per-point
   int cOff[kMaxDepth], cEnd[kMaxDepth];  // its (x, y) columns: [cOff[d], cEnd[d])
   int bny[kMaxDepth], bnz[kMaxDepth];  // the box's corners along y and z
-  int tAny[kMaxDepth], tCols;
-  unsigned char tFlag[kSepStageCap];
+  int tAny[kMaxDepth], tOdd[kMaxDepth], tCols;  // any corner; a coefficient that is not finite (kCoarse)
+  unsigned char tFlag[kStage];
   __device__ int boxOf(int d, int& nx, int& ny, int& nz) const {
     nx = cX[d][kSepX - 1] - cX[d][0] + 2;
     ny = cY[d][kSepY - 1] - cY[d][0] + 2;
@@ -402,8 +411,8 @@ struct alignas(16) SepStage {
 };
 
 // The brick's slices of kSepTables' tables (threads i = 0, n, 2n, ... of the calling group).
-template <typename T, int kSepZ>
-__device__ void sepTables(SepStage<T, kSepZ>& S, int D, int64_t M, int64_t x0, int64_t y0, int64_t z0,
+template <typename T, int kSepZ, bool kCoarse>
+__device__ void sepTables(SepStage<T, kSepZ, kCoarse>& S, int D, int64_t M, int64_t x0, int64_t y0, int64_t z0,
                           const double* __restrict__ tabH, const int* __restrict__ tabC, int i, int n) {
   constexpr int kCoords = kSepX + kSepY + kSepZ, kBatch = 4;  // a thread's items in batches, loads first
   const int total = kCoords * D;
@@ -456,18 +465,19 @@ __device__ void sepTables(SepStage<T, kSepZ>& S, int D, int64_t M, int64_t x0, i
 // Where each depth's box goes (a box over the capacity: per-point lookups), by one warp: lane d
 // sizes depth d's box, then every lane runs the greedy placement in depth order on the
 // shuffled sizes (registers only) and lane d keeps depth d's place.
-template <typename T, int kSepZ>
-__device__ void sepPlace(SepStage<T, kSepZ>& S, int D, int lane) {
+template <typename T, int kSepZ, bool kCoarse>
+__device__ void sepPlace(SepStage<T, kSepZ, kCoarse>& S, int D, int lane) {
   int n = 0, c = 0, ny = 0, nz = 0;
   if (lane < D) {
     int nx;
     n = S.boxOf(lane, nx, ny, nz);
-    c = nx * ny;
+    c = nx > 1 && ny > 1 && nz > 1 ? nx * ny : 0;
   }
   int off = 0, cols = 0, myOff = -1, myCol = 0, myEnd = 0, myColEnd = 0;
   for (int d = 0; d < D; ++d) {
     const int nd = __shfl_sync(0xffffffffu, n, d), cd = __shfl_sync(0xffffffffu, c, d);
-    const bool fits = nd <= kSepTileCap && off + nd <= kSepStageCap;
+    // (a lattice that runs backwards has no box)
+    const bool fits = cd > 0 && nd > 0 && nd <= S.kTile && off + nd <= S.kStage;
     if (lane == d) {
       myOff = fits ? off : -1;
       myCol = cols;
@@ -489,6 +499,7 @@ __device__ void sepPlace(SepStage<T, kSepZ>& S, int D, int lane) {
     S.bny[lane] = ny;
     S.bnz[lane] = nz;
     S.tAny[lane] = 0;
+    S.tOdd[lane] = 0;
   }
   if (lane == 0) S.tCols = cols;
 }
@@ -498,8 +509,8 @@ __device__ void sepPlace(SepStage<T, kSepZ>& S, int D, int lane) {
 // box, eight z entries at a time: their lattice indices are consecutive, so they lie in one or
 // two words of the lattice bits, and the loads of those words, then of the present corners'
 // coefficients and keys, go out together. The box entry (x, y, z) sits at (x ny + y) nz + z.
-template <typename T, int kSepZ>
-__device__ void sepStageBoxes(SepStage<T, kSepZ>& S, const EvalParams& P, const double* __restrict__ lambda, int i,
+template <typename T, int kSepZ, bool kCoarse>
+__device__ void sepStageBoxes(SepStage<T, kSepZ, kCoarse>& S, const EvalParams& P, const double* __restrict__ lambda, int i,
                               int n) {
   for (int e = i; e < S.tCols; e += n) {
     // the columns lie in depth order (a depth without a tile: an empty range): e's depth is the
@@ -565,6 +576,7 @@ __device__ void sepStageBoxes(SepStage<T, kSepZ>& S, const EvalParams& P, const 
         unsigned char f = 0;
         if (hasMask >> j & 1u) {
           S.tLam[t] = (T)lv[j];
+          if (kCoarse && !isfinite((T)lv[j])) S.tOdd[d] = 1;
           f = (unsigned char)(1u | (((keyHi[j] >> 5) & 7u) << 1));
         }
         S.tFlag[t] = f;
@@ -579,8 +591,8 @@ __device__ void sepStageBoxes(SepStage<T, kSepZ>& S, const EvalParams& P, const 
 // z cell rz): each present corner's coefficient, bits and x*y factor are read once for them,
 // and each point adds lambda * ((hx * hy) * hz) in corner order. colT[c]: the box entry of the
 // (x, y) corner column c = x | y << 1 at z = 0.
-template <int G, typename T, int kSepZ>
-__device__ __forceinline__ void sepCellTerms(const SepStage<T, kSepZ>& S, int d, const T* hx, const T* hy,
+template <int G, typename T, int kSepZ, bool kCoarse>
+__device__ __forceinline__ void sepCellTerms(const SepStage<T, kSepZ, kCoarse>& S, int d, const T* hx, const T* hy,
                                              const T* lamT, const unsigned char* flagT, const int (&colT)[4], int rz,
                                              int q0, T (&sum)[kSepZ]) {
 #pragma unroll
@@ -599,36 +611,45 @@ __device__ __forceinline__ void sepCellTerms(const SepStage<T, kSepZ>& S, int d,
 
 // The terms of one thread's column of kSepZ points (brick column tx, ty) over every depth, in
 // fieldAt's order: for d = 0..D-1 and k = x|y<<1|z<<2, lambda * ((hx * hy) * hz).
-template <typename T, int kSepZ>
-__device__ void sepTerms(const SepStage<T, kSepZ>& S, const EvalParams& P, const double* __restrict__ lambda,
-                         double3 o, double3 vs, int tx, int ty, int64_t xi, int64_t yj, int64_t z0, T (&sum)[kSepZ]) {
+template <typename T, int kSepZ, bool kCoarse>
+__device__ void sepTerms(const SepStage<T, kSepZ, kCoarse>& S, const EvalParams& P, const double* __restrict__ lambda,
+                         int tx, int ty, T (&sum)[kSepZ]) {
 #pragma unroll
   for (int q = 0; q < kSepZ; ++q) sum[q] = T(0);
   for (int d = 0; d < P.depth; ++d) {
-    const double w = P.w0 * (double)(1u << d), wi = P.winv[d];
     const int ny = S.bny[d], nz = S.bnz[d];
-    if (S.tOff[d] < 0) {  // the box does not fit the tile: per-point lookups
+    if (S.tOff[d] < 0 || (kCoarse && S.tOdd[d])) {
+      // The box does not fit the tile: each point looks its corners up, the four (x, y) corner
+      // columns' two z neighbours in one or two words of the lattice bits, most of them empty. A
+      // factor that is not positive ends its term here, as in the point-wise kernel, so that a
+      // coefficient that is not finite stays within its own cells (where one is staged, a coarse
+      // grid's depth comes this way too).
       const LatticeIndex& L = P.lat[d];
-      const int64_t lim = (int64_t)(P.res >> d);
-      const double px = o.x + (double)xi * vs.x, py = o.y + (double)yj * vs.y;
+      const int lim = P.res >> d;
+      const int cx = S.cX[d][tx], cy = S.cY[d][ty];
 #pragma unroll
       for (int q = 0; q < kSepZ; ++q) {
-        const double pz = o.z + (double)(z0 + q) * vs.z;
-        const int64_t cx = S.cX[d][tx], cy = S.cY[d][ty], cz = S.cZ[d][q];
+        const int cz = S.cZ[d][q];
+        unsigned has = 0;  // bit k: corner k is a vertex
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int Lx = cx + (c & 1), Ly = cy + (c >> 1);
+          if (Lx < 0 || Ly < 0 || Lx > lim || Ly > lim) continue;
+          const uint32_t col = ((uint32_t)Lx * L.M + (uint32_t)Ly) * L.M;
+          if (cz >= 0 && cz <= lim && latticeHas(L, col + (uint32_t)cz)) has |= 1u << c;
+          if (cz >= -1 && cz < lim && latticeHas(L, col + (uint32_t)(cz + 1))) has |= 16u << c;
+        }
         T s = sum[q];
-        for (int k = 0; k < 8; ++k) {
-          const int64_t Lx = cx + (k & 1), Ly = cy + ((k >> 1) & 1), Lz = cz + ((k >> 2) & 1);
-          if (Lx < 0 || Ly < 0 || Lz < 0 || Lx > lim || Ly > lim || Lz > lim) continue;
-          const uint32_t lin = (uint32_t)((Lx * L.M + Ly) * L.M + Lz);
-          if (!latticeHas(L, lin)) continue;
-          const uint32_t v = latticeRank(L, lin);
-          const double fx = hat1r(px, P.vertPos[3 * (int64_t)v], w, wi);
-          if (fx <= 0.0) continue;
-          const double fy = hat1r(py, P.vertPos[3 * (int64_t)v + 1], w, wi);
-          if (fy <= 0.0) continue;
-          const double fz = hat1r(pz, P.vertPos[3 * (int64_t)v + 2], w, wi);
-          if (fz <= 0.0) continue;
-          s += (T)lambda[v] * ((T)fx * (T)fy * (T)fz);
+        while (has) {
+          const int k = __ffs(has) - 1, ox = k & 1, oy = (k >> 1) & 1, oz = k >> 2;
+          has &= has - 1;
+          const uint32_t v = latticeRank(
+              L, ((uint32_t)(cx + ox) * L.M + (uint32_t)(cy + oy)) * L.M + (uint32_t)(cz + oz));
+          const unsigned f = (unsigned)(P.vertKey[v] >> 37) & 7u;  // the owner corner bits
+          const T fx = S.hX[d][2 * ox + (f & 1u)][tx], fy = S.hY[d][ty][2 * oy + ((f >> 1) & 1u)],
+                  fz = S.hZ[d][2 * oz + ((f >> 2) & 1u)][q];
+          if (fx <= T(0) || fy <= T(0) || fz <= T(0)) continue;
+          s += (T)lambda[v] * (fx * fy * fz);
         }
         sum[q] = s;
       }
@@ -707,13 +728,12 @@ __device__ void sepTerms(const SepStage<T, kSepZ>& S, const EvalParams& P, const
 
 // T = float is the precision form's FP32 field: the same tables (formed in FP64, rounded once)
 // and the same terms, summed in FP32. One block per brick of kSepX x kSepY x kSepZ points.
-template <typename T, int kSepZ>  // points per thread along z (the brick's depth)
-__global__ void __launch_bounds__(kSepThreads, 4) kEvalGridSep(const __grid_constant__ EvalParams P,
-                                                            const double* __restrict__ lambda, double3 o, double3 vs,
-                                                            const double* __restrict__ tabH,
-                                                            const int* __restrict__ tabC, int R,
-                                                            T* __restrict__ field) {
-  __shared__ SepStage<T, kSepZ> S;
+template <typename T, int kSepZ, bool kCoarse>  // points per thread along z (the brick's depth)
+__global__ void __launch_bounds__(kSepThreads, kCoarse ? 3 : 4)
+    kEvalGridSep(const __grid_constant__ EvalParams P, const double* __restrict__ lambda,
+                 const double* __restrict__ tabH, const int* __restrict__ tabC, int R, T* __restrict__ field) {
+  extern __shared__ __align__(16) unsigned char sepRaw[];
+  SepStage<T, kSepZ, kCoarse>& S = *(SepStage<T, kSepZ, kCoarse>*)sepRaw;
   const int64_t M = (int64_t)R + 1;
   const int tid = threadIdx.x, tx = tid % kSepX, ty = tid / kSepX;
   const int64_t x0 = (int64_t)blockIdx.x * kSepX, y0 = (int64_t)blockIdx.y * kSepY, z0 = (int64_t)blockIdx.z * kSepZ;
@@ -726,11 +746,25 @@ __global__ void __launch_bounds__(kSepThreads, 4) kEvalGridSep(const __grid_cons
   __syncthreads();
   if (xi < M && yj < M) {
     T sum[kSepZ];
-    sepTerms(S, P, lambda, o, vs, tx, ty, xi, yj, z0, sum);
+    sepTerms(S, P, lambda, tx, ty, sum);
 #pragma unroll
     for (int q = 0; q < kSepZ; ++q)
       if (z0 + q < M) field[xi + M * (yj + M * (z0 + q))] = sum[q];
   }
+}
+
+template <typename T, int kSepZ, bool kCoarse>
+static its_status launchSep(its_ctx* ctx, const EvalParams& P, const double* lam, const double* tabH, const int* tabC,
+                            int res, T* field) {
+  const int64_t M = (int64_t)res + 1;
+  const dim3 grid((unsigned)((M + kSepX - 1) / kSepX), (unsigned)((M + kSepY - 1) / kSepY),
+                  (unsigned)((M + kSepZ - 1) / kSepZ));
+  constexpr int bytes = (int)sizeof(SepStage<T, kSepZ, kCoarse>);
+  if (bytes > 48 * 1024)
+    ITS_CU(ctx, cudaFuncSetAttribute(kEvalGridSep<T, kSepZ, kCoarse>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  kEvalGridSep<T, kSepZ, kCoarse><<<grid, kSepThreads, bytes, ctx->stream>>>(P, lam, tabH, tabC, res, field);
+  ITS_LAUNCHED(ctx);
+  return ITS_OK;
 }
 
 // ---- marching cubes in three launches -----------------------------------------------------
@@ -933,56 +967,55 @@ template <typename T>
 static its_status evalGridTuned(its_ctx* ctx, const SvoDevice& d, const double* lam, double3 o, double3 vs, int res,
                                 T* field) {
   const EvalParams P = evalParams(d);
-  // four brick shapes of the point-wise kernel and the separable kernel with 4 or 8 points per
-  // thread along z (FP64, when the brick's cell box fits its tile): every candidate computes
-  // the same bits
-  auto sepFits = [&](int z) {
+  // Every candidate computes the same bits for its type. Grids at least about twice as fine as the
+  // octree (the brick's finest cell box fits the small tile): FP64, four brick shapes of the
+  // point-wise kernel and the separable kernel with 4 or 8 points per thread along z; FP32, the
+  // separable kernel's two shapes. Coarser grids: the separable kernel with the large tile, the
+  // deeper brick by default where its box fits (torus of 99,000 faces, octree 256, grid 256: 3.52
+  // ms point by point in bricks of 32 x 4 x 8).
+  auto boxFits = [&](int z, int64_t cap) {
     return boxCorners(kSepX, vs.x, d.unit[0]) * boxCorners(kSepY, vs.y, d.unit[0]) * boxCorners(z, vs.z, d.unit[0]) <=
-           kSepTileCap;
+           cap;
   };
-  // Candidates, each computing the same bits for its type: FP64, four brick shapes of the
-  // point-wise kernel and the separable kernel with 4 or 8 points per thread along z (when the
-  // brick's cell box fits its tile); FP32, the separable kernel's two shapes where it fits (its
-  // rounding differs from the point-wise FP32 kernel's), else the brick shapes.
   std::vector<int> cand;
-  if (sizeof(T) == 8 || !sepFits(4)) cand = {0, 1, 2, 3};
-  if (sepFits(4)) cand.push_back(4);
-  if (sepFits(8)) cand.push_back(5);
+  if (boxFits(4, kSepTileCap)) {
+    if (sizeof(T) == 8) cand = {0, 1, 2, 3};
+    cand.push_back(4);
+    if (boxFits(8, kSepTileCap)) cand.push_back(5);
+  } else {
+    cand = {6};
+    if (boxFits(8, kCoarseTileCap)) cand.push_back(7);
+  }
+  // the separable kernel's hat tables, formed once for all its launches here
   DevBuf<double> tabH;
   DevBuf<int> tabC;
-  if (sepFits(4)) {  // the separable kernel's hat tables, formed once for all its launches here
-    const int64_t M = (int64_t)res + 1, n = (int64_t)d.depth * 3 * M;
-    its_status st = tabH.alloc(ctx, 4 * n);
-    if (st == ITS_OK) st = tabC.alloc(ctx, n);
-    if (st != ITS_OK) return st;
-    kSepTables<<<gridFor(n, 256), 256, 0, ctx->stream>>>(P, o, vs, M, tabH.p, tabC.p);
-    ITS_LAUNCHED(ctx);
-  }
+  const int64_t M = (int64_t)res + 1, n = (int64_t)d.depth * 3 * M;
+  its_status st = tabH.alloc(ctx, 4 * n);
+  if (st == ITS_OK) st = tabC.alloc(ctx, n);
+  if (st != ITS_OK) return st;
+  kSepTables<<<gridFor(n, 256), 256, 0, ctx->stream>>>(P, o, vs, M, tabH.p, tabC.p);
+  ITS_LAUNCHED(ctx);
   auto run = [&](int j) -> its_status {
     switch (cand[j]) {
-      case 1: return launchBricks<T, 32, 8, 2>(ctx, P, lam, o, vs, res, field);
-      case 2: return launchBricks<T, 64, 4, 2>(ctx, P, lam, o, vs, res, field);
-      case 3: return launchBricks<T, 16, 4, 4>(ctx, P, lam, o, vs, res, field);
-      case 4:
-      case 5: {
-        const int z = cand[j] == 5 ? 8 : 4;
-        const int64_t M = (int64_t)res + 1;
-        const dim3 grid((unsigned)((M + kSepX - 1) / kSepX), (unsigned)((M + kSepY - 1) / kSepY),
-                        (unsigned)((M + z - 1) / z));
-        if (z == 8)
-          kEvalGridSep<T, 8><<<grid, kSepThreads, 0, ctx->stream>>>(P, lam, o, vs, tabH.p, tabC.p, res, field);
-        else
-          kEvalGridSep<T, 4><<<grid, kSepThreads, 0, ctx->stream>>>(P, lam, o, vs, tabH.p, tabC.p, res, field);
-        ITS_LAUNCHED(ctx);
-        return ITS_OK;
-      }
-      default: return launchBricks<T, 32, 4, 4>(ctx, P, lam, o, vs, res, field);
+      case 4: return launchSep<T, 4, false>(ctx, P, lam, tabH.p, tabC.p, res, field);
+      case 5: return launchSep<T, 8, false>(ctx, P, lam, tabH.p, tabC.p, res, field);
+      case 6: return launchSep<T, 4, true>(ctx, P, lam, tabH.p, tabC.p, res, field);
+      case 7: return launchSep<T, 8, true>(ctx, P, lam, tabH.p, tabC.p, res, field);
     }
+    if constexpr (sizeof(T) == 8) {
+      switch (cand[j]) {
+        case 1: return launchBricks<T, 32, 8, 2>(ctx, P, lam, o, vs, res, field);
+        case 2: return launchBricks<T, 64, 4, 2>(ctx, P, lam, o, vs, res, field);
+        case 3: return launchBricks<T, 16, 4, 4>(ctx, P, lam, o, vs, res, field);
+        default: return launchBricks<T, 32, 4, 4>(ctx, P, lam, o, vs, res, field);
+      }
+    }
+    return ITS_ERR_STATE;
   };
   const std::string key = std::string("eval_grid/") + (sizeof(T) == 8 ? "f64" : "f32") + "/grid=" +
                           std::to_string(res) + "/octree=" + std::to_string(d.res) + "/depth=" + std::to_string(d.depth);
   int choice = 0;
-  its_status st = tuneChoice(ctx, key, (int)cand.size(), cand.back() >= 4 ? (int)cand.size() - 1 : 0, run, &choice);
+  st = tuneChoice(ctx, key, (int)cand.size(), (int)cand.size() - 1, run, &choice);
   if (st != ITS_OK) return st;
   return run(choice);
 }
