@@ -35,32 +35,35 @@ struct CubicGen {
   // Entries of the row whose lattice coordinates at depth dd are u(dd, u).
   template <typename U, typename E>
   __device__ void row(U uOf, E emit) const {
-    for (int dd = 0; dd < depth; ++dd) {
-      double u[3];
-      uOf(dd, u);
-      const LatticeIndex L = lat[dd];
-      const int64_t M = L.M;
-      int64_t base[3];
-      double wt[3][4];
+    for (int dd = 0; dd < depth; ++dd) rowDepth(dd, uOf, emit);
+  }
+  // Those of depth dd.
+  template <typename U, typename E>
+  __device__ void rowDepth(int dd, U uOf, E emit) const {
+    double u[3];
+    uOf(dd, u);
+    const LatticeIndex L = lat[dd];
+    const int64_t M = L.M;
+    int64_t base[3];
+    double wt[3][4];
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        base[a] = (int64_t)floor(u[a]) - 1;
+    for (int a = 0; a < 3; ++a) {
+      base[a] = (int64_t)floor(u[a]) - 1;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) wt[a][j] = bspline3(u[a] - (double)(base[a] + j));
-      }
-      for (int jx = 0; jx < 4; ++jx) {
-        const int64_t kx = base[0] + jx;
-        if (kx < 0 || kx >= M || wt[0][jx] == 0.0) continue;
-        for (int jy = 0; jy < 4; ++jy) {
-          const int64_t ky = base[1] + jy;
-          if (ky < 0 || ky >= M || wt[1][jy] == 0.0) continue;
-          const double wxy = wt[0][jx] * wt[1][jy];
-          for (int jz = 0; jz < 4; ++jz) {
-            const int64_t kz = base[2] + jz;
-            if (kz < 0 || kz >= M || wt[2][jz] == 0.0) continue;
-            const uint32_t lin = (uint32_t)((kx * M + ky) * M + kz);
-            if (latticeHas(L, lin)) emit((int32_t)latticeRank(L, lin), wxy * wt[2][jz]);
-          }
+      for (int j = 0; j < 4; ++j) wt[a][j] = bspline3(u[a] - (double)(base[a] + j));
+    }
+    for (int jx = 0; jx < 4; ++jx) {
+      const int64_t kx = base[0] + jx;
+      if (kx < 0 || kx >= M || wt[0][jx] == 0.0) continue;
+      for (int jy = 0; jy < 4; ++jy) {
+        const int64_t ky = base[1] + jy;
+        if (ky < 0 || ky >= M || wt[1][jy] == 0.0) continue;
+        const double wxy = wt[0][jx] * wt[1][jy];
+        for (int jz = 0; jz < 4; ++jz) {
+          const int64_t kz = base[2] + jz;
+          if (kz < 0 || kz >= M || wt[2][jz] == 0.0) continue;
+          const uint32_t lin = (uint32_t)((kx * M + ky) * M + kz);
+          if (latticeHas(L, lin)) emit((int32_t)latticeRank(L, lin), wxy * wt[2][jz]);
         }
       }
     }
