@@ -16,6 +16,7 @@
 //   compaction pass, no 18 R^3 preallocation).
 #include <algorithm>
 #include <cfloat>
+#include <type_traits>
 #include <vector>
 
 #include "its_mc.cuh"
@@ -767,182 +768,291 @@ static its_status launchSep(its_ctx* ctx, const EvalParams& P, const double* lam
   return ITS_OK;
 }
 
-// ---- marching cubes in three launches -----------------------------------------------------
-// Classify: each thread takes 8 consecutive voxels (x fastest) and slides along x, loading one
-// column of 4 corner values per voxel (each field value is read about once), writes the case
-// bytes and reduces the vertex counts per block. The block sums are scanned (kScanSpine);
-// Emit re-reads only the case bytes, scans the counts inside the block and writes the
-// triangle vertices of the non-empty voxels in voxel order, as the reference's compaction does.
-template <typename T, int ITEMS>
-__global__ void __launch_bounds__(kScanThreads) kMcClassify(const T* __restrict__ field, int R, double iso,
-                                                             uint8_t* __restrict__ cube,
-                                                             unsigned long long* __restrict__ blockSums) {
+// ---- marching cubes -----------------------------------------------------------------------
+// kMcSigns reads the field once, flat and coalesced, and keeps one bit per lattice point
+// (f < iso); everything after works on the bits, which stay in L2 (17 MB at 513^3), and on the
+// field values of crossed voxels only. kMcCases: a thread takes ITEMS consecutive voxels, whose
+// 4 corner rows are windows of ITEMS + 1 bits, writes the case bytes (most windows are all 0 or
+// all 1) and counts the vertices; tiles with any are listed. The tiles' counts are scanned
+// (scanSpine), and kMcEmit writes the listed tiles' triangles, a thread per vertex, in voxel
+// order, as the reference's compaction does. Comparing in the classifying pass itself read
+// every value four times through the L1 and formed each case from four ballots: 356 us for the
+// 512^3 cases of an FP64 field, and a thread per crossed voxel in one block per tile 97 us for
+// 1.25 M vertices; now 154 + 66 us and 38 us.
+constexpr int kSignWords = 16;  // words of 32 lattice points per warp
+template <typename T>
+__global__ void __launch_bounds__(kScanThreads) kMcSigns(const T* __restrict__ field, int64_t total, double iso,
+                                                         uint32_t* __restrict__ signs, unsigned* __restrict__ zero) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *zero = 0u;  // the listed tiles' counter
+  const int lane = threadIdx.x & 31;
+  const int64_t w0 = ((int64_t)blockIdx.x * (kScanThreads / 32) + (threadIdx.x >> 5)) * kSignWords;
+  const int64_t i0 = w0 * 32 + lane;
+  T v[kSignWords];
+  if ((w0 + kSignWords) * 32 <= total) {
+#pragma unroll
+    for (int j = 0; j < kSignWords; ++j) v[j] = field[i0 + 32 * j];
+  } else {
+#pragma unroll
+    for (int j = 0; j < kSignWords; ++j) v[j] = i0 + 32 * j < total ? field[i0 + 32 * j] : field[total - 1];
+  }
+  uint32_t mine = 0;
+#pragma unroll
+  for (int j = 0; j < kSignWords; ++j) {
+    const uint32_t b = __ballot_sync(0xffffffffu, (double)v[j] < iso);
+    if (lane == j) mine = b;
+  }
+  if (lane < kSignWords) signs[w0 + lane] = mine;
+}
+
+// The bit of lattice point p, and the 32 bits from it on.
+__device__ __forceinline__ unsigned signBit(const uint32_t* __restrict__ signs, int64_t p) {
+  return (__ldg(signs + (p >> 5)) >> (p & 31)) & 1u;
+}
+__device__ __forceinline__ uint32_t signWindow(const uint32_t* __restrict__ signs, int64_t p) {
+  const uint32_t* w = signs + (p >> 5);
+  return __funnelshift_r(__ldg(w), __ldg(w + 1), (unsigned)(p & 31));
+}
+// Bits 0..3 of b, one per byte.
+__device__ __forceinline__ uint32_t spread4(uint32_t b) { return ((b & 15u) * 0x00204081u) & 0x01010101u; }
+
+// Division of v < 2^53 by d <= 2048: with m = ceil(2^64 / d), m d = 2^64 + e, e < d, so v m / 2^64 is
+// v / d plus v e / (d 2^64), less than 1 / d: the same whole part.
+struct FastDiv {
+  unsigned long long m;
+  int d;
+  __device__ __forceinline__ int64_t operator()(int64_t v) const {
+    return d == 1 ? v : (int64_t)__umul64hi((unsigned long long)v, m);
+  }
+};
+static FastDiv fastDiv(int d) { return {d > 1 ? ~0ull / (unsigned)d + 1ull : 0ull, d}; }
+
+// A warp takes kTiles consecutive tiles of 32 x ITEMS voxels, their windows loaded together. A run
+// that crosses a row's end joins the windows of the two rows.
+template <int ITEMS, int kTiles>
+__global__ void __launch_bounds__(kScanThreads) kMcCases(const uint32_t* __restrict__ signs, int R, FastDiv byR,
+                                                         uint8_t* __restrict__ cube, int64_t numTiles,
+                                                         unsigned long long* __restrict__ tileSums,
+                                                         uint32_t* __restrict__ listed, unsigned* __restrict__ numListed) {
+  constexpr uint32_t kMask = (1u << ITEMS) - 1u;
+  __shared__ unsigned char sCount[256];
+  const int lane = threadIdx.x & 31;
   const int64_t nvox = (int64_t)R * R * R, M = (int64_t)R + 1;
-  const int64_t base = (int64_t)blockIdx.x * (kScanThreads * ITEMS) + (int64_t)threadIdx.x * ITEMS;
-  unsigned long long cnt = 0;
-  int64_t x = 0, y = 0, z = 0;
-  if (base < nvox) voxelXYZ(base, R, x, y, z);
-  if (base + ITEMS <= nvox && x + ITEMS <= R) {
-    // the run stays in one row: all 4 x (ITEMS + 1) corner values are loaded up front
-    const int64_t r0 = (z * M + y) * M + x, r1 = (z * M + y + 1) * M + x, r2 = ((z + 1) * M + y) * M + x,
-                  r3 = ((z + 1) * M + y + 1) * M + x;
-    double fa[ITEMS + 1], fb[ITEMS + 1], fc[ITEMS + 1], fd[ITEMS + 1];
+  const int64_t tile0 = ((int64_t)blockIdx.x * (kScanThreads / 32) + (threadIdx.x >> 5)) * kTiles;
+  uint32_t c[kTiles][4], n[kTiles][4];  // the corners at x and x + 1 of (y, z), (y+1, z), (y, z+1), (y+1, z+1)
+  bool whole[kTiles];
 #pragma unroll
-    for (int j = 0; j <= ITEMS; ++j) {
-      fa[j] = (double)field[r0 + j];
-      fb[j] = (double)field[r1 + j];
-      fc[j] = (double)field[r2 + j];
-      fd[j] = (double)field[r3 + j];
-    }
-    unsigned long long packed = 0;
+  for (int t = 0; t < kTiles; ++t) {
+    const int64_t base = ((tile0 + t) * 32 + lane) * ITEMS;
+    whole[t] = base + ITEMS <= nvox && ITEMS <= R;
+    if (!whole[t]) continue;
+    const int64_t row = byR(base), z = byR(row), p = base + row + z * M;  // (z M + y) M + x
+    const int left = (int)((row + 1) * R - base);                         // voxels left in the row
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-      const unsigned ci = (unsigned)(fa[j] < iso) | (unsigned)(fb[j] < iso) << 1 | (unsigned)(fb[j + 1] < iso) << 2 |
-                          (unsigned)(fa[j + 1] < iso) << 3 | (unsigned)(fc[j] < iso) << 4 |
-                          (unsigned)(fd[j] < iso) << 5 | (unsigned)(fd[j + 1] < iso) << 6 |
-                          (unsigned)(fc[j + 1] < iso) << 7;
-      cnt += cMcCase[ci] & 15ull;
-      packed |= (unsigned long long)ci << (8 * (j & 7));
-      if (ITEMS != 8 || (((uintptr_t)(cube + base)) & 7u)) cube[base + j] = (uint8_t)ci;
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t w = signWindow(signs, p + (k & 1 ? M : 0) + (k & 2 ? M * M : 0));
+      c[t][k] = w & kMask;
+      n[t][k] = (w >> 1) & kMask;
     }
-    // one 8-byte store when the caller's buffer allows it (base is a multiple of 8)
-    if (ITEMS == 8 && !(((uintptr_t)(cube + base)) & 7u)) *(unsigned long long*)(cube + base) = packed;
-  } else if (base < nvox) {
-    double a = 0, b = 0, c = 0, d = 0;  // column x: (y,z) (y+1,z) (y,z+1) (y+1,z+1)
-    bool have = false;
-    for (int j = 0; j < ITEMS && base + j < nvox; ++j) {
-      const int64_t r0 = (z * M + y) * M, r1 = (z * M + y + 1) * M, r2 = ((z + 1) * M + y) * M,
-                    r3 = ((z + 1) * M + y + 1) * M;
-      if (!have) {
-        a = (double)field[r0 + x];
-        b = (double)field[r1 + x];
-        c = (double)field[r2 + x];
-        d = (double)field[r3 + x];
+    if (left < ITEMS) {
+      const int64_t row2 = row + 1, z2 = byR(row2), p2 = row2 * R + row2 + z2 * M;
+      const uint32_t keep = (1u << left) - 1u;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t w = signWindow(signs, p2 + (k & 1 ? M : 0) + (k & 2 ? M * M : 0));
+        c[t][k] = (c[t][k] & keep) | (w << left & kMask);
+        n[t][k] = (n[t][k] & keep) | ((w >> 1) << left & kMask);
       }
-      const double a1 = (double)field[r0 + x + 1], b1 = (double)field[r1 + x + 1], c1 = (double)field[r2 + x + 1],
-                   d1 = (double)field[r3 + x + 1];
-      // corner order 0 (0,0,0) 1 (0,1,0) 2 (1,1,0) 3 (1,0,0) 4 (0,0,1) 5 (0,1,1) 6 (1,1,1) 7 (1,0,1)
-      const unsigned ci = (unsigned)(a < iso) | (unsigned)(b < iso) << 1 | (unsigned)(b1 < iso) << 2 |
-                          (unsigned)(a1 < iso) << 3 | (unsigned)(c < iso) << 4 | (unsigned)(d < iso) << 5 |
-                          (unsigned)(d1 < iso) << 6 | (unsigned)(c1 < iso) << 7;
-      cube[base + j] = (uint8_t)ci;
-      cnt += cMcCase[ci] & 15ull;
-      a = a1;
-      b = b1;
-      c = c1;
-      d = d1;
-      have = true;
-      if (++x == R) {  // next row
-        x = 0;
-        have = false;
-        if (++y == R) {
-          y = 0;
-          ++z;
+    }
+  }
+  sCount[threadIdx.x] = (unsigned char)(cMcCase[threadIdx.x] & 15ull);
+  __syncthreads();
+  unsigned sums[kTiles];
+#pragma unroll
+  for (int t = 0; t < kTiles; ++t) {
+    const int64_t base = ((tile0 + t) * 32 + lane) * ITEMS;
+    unsigned cnt = 0;
+    if (whole[t]) {
+      uint32_t out[ITEMS / 4];
+      const uint32_t some = c[t][0] | c[t][1] | c[t][2] | c[t][3] | n[t][0] | n[t][1] | n[t][2] | n[t][3];
+      const uint32_t all = c[t][0] & c[t][1] & c[t][2] & c[t][3] & n[t][0] & n[t][1] & n[t][2] & n[t][3];
+      if (some == 0u || all == kMask) {
+#pragma unroll
+        for (int j = 0; j < ITEMS / 4; ++j) out[j] = some ? 0xffffffffu : 0u;
+      } else {
+        // corner order 0 (0,0,0) 1 (0,1,0) 2 (1,1,0) 3 (1,0,0) 4 (0,0,1) 5 (0,1,1) 6 (1,1,1) 7 (1,0,1)
+#pragma unroll
+        for (int j = 0; j < ITEMS / 4; ++j) {
+          const uint32_t v = spread4(c[t][0] >> (4 * j)) | spread4(c[t][1] >> (4 * j)) << 1 |
+                             spread4(n[t][1] >> (4 * j)) << 2 | spread4(n[t][0] >> (4 * j)) << 3 |
+                             spread4(c[t][2] >> (4 * j)) << 4 | spread4(c[t][3] >> (4 * j)) << 5 |
+                             spread4(n[t][3] >> (4 * j)) << 6 | spread4(n[t][2] >> (4 * j)) << 7;
+          out[j] = v;
+          cnt += sCount[v & 255u] + sCount[(v >> 8) & 255u] + sCount[(v >> 16) & 255u] + sCount[v >> 24];
+        }
+      }
+      uint8_t* dst = cube + base;
+      if (!((uintptr_t)dst & (ITEMS - 1))) {  // base is a multiple of ITEMS: the caller's buffer decides
+        if constexpr (ITEMS == 16) *(uint4*)dst = make_uint4(out[0], out[1], out[2], out[3]);
+        else if constexpr (ITEMS == 8) *(uint2*)dst = make_uint2(out[0], out[1]);
+        else *(uint32_t*)dst = out[0];
+      } else {
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) dst[j] = (uint8_t)(out[j >> 2] >> (8 * (j & 3)));
+      }
+    } else if (base < nvox) {
+      int64_t x, y, z;
+      voxelXYZ(base, R, x, y, z);
+      for (int j = 0; j < ITEMS && base + j < nvox; ++j) {
+        const int64_t q = (z * M + y) * M + x;
+        const unsigned ci = signBit(signs, q) | signBit(signs, q + M) << 1 | signBit(signs, q + M + 1) << 2 |
+                            signBit(signs, q + 1) << 3 | signBit(signs, q + M * M) << 4 |
+                            signBit(signs, q + M * M + M) << 5 | signBit(signs, q + M * M + M + 1) << 6 |
+                            signBit(signs, q + M * M + 1) << 7;
+        cube[base + j] = (uint8_t)ci;
+        cnt += sCount[ci];
+        if (++x == R) {  // next row
+          x = 0;
+          if (++y == R) {
+            y = 0;
+            ++z;
+          }
         }
       }
     }
+    sums[t] = __reduce_add_sync(0xffffffffu, cnt);
   }
-  unsigned long long total;
-  blockExclusiveScan<unsigned long long>(cnt, total);
-  if (threadIdx.x == 0) blockSums[blockIdx.x] = total;
-}
-
-// kMcClassify for R a multiple of 256 (tiles of 8 voxels per thread): the same case bytes and
-// block sums with coalesced loads. A warp takes 256 consecutive voxels of one row, lane l the
-// voxels x0 + l + 32 j; each of the 4 corner rows is read 32 values per load, compared with
-// the iso level, and the comparison of the x+1 corner comes from the next lane's bit of the
-// row's ballot (lane 31: the next round's bit 0, or one extra value).
-template <typename T>
-__global__ void __launch_bounds__(kScanThreads) kMcClassifyRows(const T* __restrict__ field, int R, double iso,
-                                                               uint8_t* __restrict__ cube,
-                                                               unsigned long long* __restrict__ blockSums) {
-  const int64_t M = (int64_t)R + 1;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t s = (int64_t)blockIdx.x * (kScanThreads * 8) + (int64_t)warp * 256;  // the warp's first voxel
-  int64_t x0, y, z;
-  voxelXYZ(s, R, x0, y, z);
-  const int64_t r[4] = {(z * M + y) * M + x0, (z * M + y + 1) * M + x0, ((z + 1) * M + y) * M + x0,
-                        ((z + 1) * M + y + 1) * M + x0};
-  double v[4][9];  // corner rows: v[k][j] at x0 + lane + 32 j; v[k][8] at x0 + 256 (all lanes)
+  if (lane == 0) {
+    unsigned any = 0;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[k][j] = (double)field[r[k] + lane + 32 * j];
-    v[k][8] = (double)field[r[k] + 256];
-  }
-  // each corner row's comparisons as warp ballots: the x+1 corner of lane l is bit l+1 (lane
-  // 31: bit 0 of the next round, or the extra value)
-  unsigned bal[4][8];
-  unsigned ext = 0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) bal[k][j] = __ballot_sync(0xffffffffu, v[k][j] < iso);
-    ext |= (unsigned)(v[k][8] < iso) << k;
-  }
-  unsigned long long cnt = 0;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    unsigned c[4], n[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      c[k] = (bal[k][j] >> lane) & 1u;
-      n[k] = lane < 31 ? (bal[k][j] >> (lane + 1)) & 1u : (j < 7 ? bal[k][j < 7 ? j + 1 : 0] & 1u : (ext >> k) & 1u);
+    for (int t = 0; t < kTiles; ++t) {
+      if (tile0 + t < numTiles) tileSums[tile0 + t] = sums[t];
+      any += sums[t] ? 1u : 0u;
     }
-    // corner order 0 (0,0,0) 1 (0,1,0) 2 (1,1,0) 3 (1,0,0) 4 (0,0,1) 5 (0,1,1) 6 (1,1,1) 7 (1,0,1)
-    const unsigned ci = c[0] | c[1] << 1 | n[1] << 2 | n[0] << 3 | c[2] << 4 | c[3] << 5 | n[3] << 6 | n[2] << 7;
-    cube[s + lane + 32 * j] = (uint8_t)ci;
-    cnt += cMcCase[ci] & 15ull;
+    if (any && listed) {  // in any order: every tile has its own place in the soup
+      unsigned at = atomicAdd(numListed, any);
+#pragma unroll
+      for (int t = 0; t < kTiles; ++t)
+        if (sums[t]) listed[at++] = (uint32_t)(tile0 + t);
+    }
   }
-  unsigned long long total;
-  blockExclusiveScan<unsigned long long>(cnt, total);
-  if (threadIdx.x == 0) blockSums[blockIdx.x] = total;
 }
 
+// The listed tiles' triangles, a warp per tile. The tile's voxels with vertices are listed in voxel
+// order (one scan of voxel and vertex counts packed in 32 bits), then its vertices are written, a
+// lane each: a lane finds its voxel in the list, reads the two field values at its edge's ends
+// and writes its point, so neighbouring lanes write neighbouring vertices.
 template <typename T, int ITEMS>
-__global__ void __launch_bounds__(kScanThreads) kMcEmit(McCaseT<T> mc, double3 o, double3 vs,
-                                                         const uint8_t* __restrict__ cube,
-                                                         const unsigned long long* __restrict__ blockOffsets,
-                                                         const unsigned long long* __restrict__ grandTotal,
-                                                         double* __restrict__ tri, unsigned long long capacity) {
-  // a block whose voxels emit nothing (most of them: the surface crosses few tiles) leaves at once
-  const unsigned long long next = blockIdx.x + 1 < gridDim.x ? blockOffsets[blockIdx.x + 1] : *grandTotal;
-  if (next == blockOffsets[blockIdx.x]) return;
-  const int64_t nvox = (int64_t)mc.R * mc.R * mc.R;
-  const int64_t base = (int64_t)blockIdx.x * (kScanThreads * ITEMS) + (int64_t)threadIdx.x * ITEMS;
-  unsigned char ci[ITEMS];
-  unsigned long long cnt = 0;
-#pragma unroll
-  for (int j = 0; j < ITEMS; ++j) {
-    ci[j] = base + j < nvox ? cube[base + j] : 0;
-    cnt += cMcCase[ci[j]] & 15ull;
-  }
-  unsigned long long total;
-  const unsigned long long tileBase = blockOffsets[blockIdx.x];
-  unsigned long long run = blockExclusiveScan<unsigned long long>(cnt, total);  // within the tile
-  if (!total || !tri) return;
-  // The tile's voxels with vertices are listed (place in the tile | offset within the tile's
-  // output << 12: at most 15 vertices per voxel, so the offset stays below 2^16) and the block
-  // emits the list round-robin, instead of each thread its own ITEMS voxels one after another.
-  // Every voxel writes at its own offset: the order of the list does not matter.
-  static_assert(kScanThreads * ITEMS <= 4096 && 15 * kScanThreads * ITEMS < 65536, "list entry packing");
-  __shared__ uint32_t sList[kScanThreads * ITEMS];
-  __shared__ unsigned sCount;
-  if (threadIdx.x == 0) sCount = 0;
+__global__ void __launch_bounds__(kScanThreads) kMcEmit(McCaseT<T> mc, FastDiv byR, double3 o, double3 vs,
+                                                        const uint8_t* __restrict__ cube,
+                                                        const unsigned long long* __restrict__ tileOffsets,
+                                                        const uint32_t* __restrict__ listed,
+                                                        const unsigned* __restrict__ numListed,
+                                                        double* __restrict__ tri, unsigned long long capacity) {
+  constexpr int kTile = 32 * ITEMS;
+  static_assert(15 * kTile < 65536, "voxel and vertex counts share 32 bits");
+  __shared__ uint32_t sLists[kScanThreads / 32][kTile];  // place in the tile | first vertex << 16
+  __shared__ uint8_t sCases[kScanThreads / 32][kTile];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, R = mc.R;
+  uint32_t* sList = sLists[warp];
+  uint8_t* sCase = sCases[warp];
+  __shared__ uint32_t sWords[kScanThreads / 32][kTile / 4];
+  __shared__ uint8_t sPlaces[kScanThreads / 32][kTile / 4];
+  uint32_t* sWord = sWords[warp];
+  uint8_t* sPlace = sPlaces[warp];
+  __shared__ uint64_t sTable[256];  // per-lane indices: shared memory, not the constant cache
+  sTable[threadIdx.x] = cMcCase[threadIdx.x];
   __syncthreads();
+  const int64_t nvox = (int64_t)R * R * R, M = (int64_t)R + 1;
+  const unsigned n = *numListed, step = gridDim.x * (kScanThreads / 32);
+  for (unsigned t = blockIdx.x * (kScanThreads / 32) + warp; t < n; t += step) {
+    const uint32_t tile = listed[t];
+    const int64_t tile0 = (int64_t)tile * kTile, base = tile0 + (int64_t)lane * ITEMS;
+    const unsigned long long tileBase = tileOffsets[tile];
+    // the words of four case bytes that are not all 0 or all 255, in voxel order
+    uint32_t word[ITEMS / 4];
+    if (base + ITEMS <= nvox && !((uintptr_t)(cube + base) & 3u)) {
 #pragma unroll
-  for (int j = 0; j < ITEMS; ++j) {
-    const unsigned c = cMcCase[ci[j]] & 15u;
-    if (c) sList[atomicAdd(&sCount, 1u)] = (uint32_t)(threadIdx.x * ITEMS + j) | (uint32_t)run << 12;
-    run += c;
-  }
-  __syncthreads();
-  const int64_t tile0 = (int64_t)blockIdx.x * (kScanThreads * ITEMS);
-  for (unsigned e = threadIdx.x; e < sCount; e += kScanThreads) {
-    const uint32_t item = sList[e];
-    const int64_t v = tile0 + (item & 4095u);
-    const unsigned char c8 = cube[v];
-    mcEmitVoxel(mc, o, vs, tri, capacity, v, c8, tileBase + (item >> 12), cMcCase[c8] & 15ull);
+      for (int j = 0; j < ITEMS / 4; ++j) word[j] = *(const uint32_t*)(cube + base + 4 * j);
+    } else {
+#pragma unroll
+      for (int j = 0; j < ITEMS / 4; ++j) {
+        word[j] = 0;
+        for (int k = 0; k < 4; ++k)
+          if (base + 4 * j + k < nvox) word[j] |= (uint32_t)cube[base + 4 * j + k] << (8 * k);
+      }
+    }
+    uint32_t mixed = 0;
+#pragma unroll
+    for (int j = 0; j < ITEMS / 4; ++j) mixed += word[j] != 0u && word[j] != 0xffffffffu;
+    uint32_t incl = mixed;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t up = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += up;
+    }
+    const uint32_t words = __shfl_sync(0xffffffffu, incl, 31);
+    uint32_t at = incl - mixed;
+    __syncwarp();  // the previous tile's lists have been read
+#pragma unroll
+    for (int j = 0; j < ITEMS / 4; ++j)
+      if (word[j] != 0u && word[j] != 0xffffffffu) {
+        sWord[at] = word[j];
+        sPlace[at++] = (uint8_t)(lane * (ITEMS / 4) + j);
+      }
+    __syncwarp();
+    // their voxels with vertices, a lane per byte
+    uint32_t total = 0;  // vertices | voxels << 16
+    for (uint32_t b0 = 0; b0 < 4 * words; b0 += 32) {
+      const uint32_t b = b0 + lane;
+      const uint32_t c = b < 4 * words ? (sWord[b >> 2] >> (8 * (b & 3))) & 255u : 0u;
+      const uint32_t cnt = c != 0u && c != 255u ? ((unsigned)sTable[c] & 15u) + 65536u : 0u;
+      uint32_t run = cnt;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, run, d);
+        if (lane >= d) run += up;
+      }
+      const uint32_t first = total + run - cnt;
+      if (cnt) {
+        sList[first >> 16] = (4u * sPlace[b >> 2] + (b & 3u)) | first << 16;
+        sCase[first >> 16] = (uint8_t)c;
+      }
+      total += __shfl_sync(0xffffffffu, run, 31);
+    }
+    __syncwarp();
+    const unsigned nv = total & 65535u, nl = total >> 16;
+    for (unsigned e = lane; e < nv; e += 32) {
+      if (tileBase + e >= capacity) break;
+      unsigned lo = 0, hi = nl;  // the last listed voxel whose first vertex is at or before e
+      while (hi - lo > 1) {
+        const unsigned mid = (lo + hi) / 2;
+        if ((sList[mid] >> 16) <= e) lo = mid;
+        else hi = mid;
+      }
+      const uint32_t item = sList[lo];
+      const int64_t v = tile0 + (item & 65535u), row = byR(v), z = byR(row), x = v - row * R, y = row - z * R;
+      const int edge = (int)((sTable[sCase[lo]] >> (4 * (e - (item >> 16) + 1))) & 15u);
+      // the edge's corners (cMcEdge as nibbles) and their offsets (cMcCorner's columns as bits)
+      const int a = (int)(0x321076543210ull >> (4 * edge)) & 15, b = (int)(0x765447650321ull >> (4 * edge)) & 15;
+      const int oa[3] = {0xCC >> a & 1, 0x66 >> a & 1, 0xF0 >> a & 1},
+                ob[3] = {0xCC >> b & 1, 0x66 >> b & 1, 0xF0 >> b & 1};
+      const double vp[3] = {(double)x * vs.x + o.x, (double)y * vs.y + o.y, (double)z * vs.z + o.z};
+      const double vsz[3] = {vs.x, vs.y, vs.z};
+      double pa[3], pb[3], q[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        pa[k] = oa[k] ? vp[k] + vsz[k] : vp[k];
+        pb[k] = ob[k] ? vp[k] + vsz[k] : vp[k];
+      }
+      const int64_t corner = (z * M + y) * M + x;
+      const double sa = (double)mc.field[corner + (oa[2] * M + oa[1]) * M + oa[0]];
+      const double sb = (double)mc.field[corner + (ob[2] * M + ob[1]) * M + ob[0]];
+      vertexLerp(pa, pb, sa, sb, mc.iso, q);
+      double* dst = tri + 3 * (tileBase + e);
+      dst[0] = q[0];
+      dst[1] = q[1];
+      dst[2] = q[2];
+    }
   }
 }
 
@@ -1316,42 +1426,57 @@ its_status marchingCubesT(its_ctx* ctx, const FT* field, int res, const double o
     if ((st = cubeTmp.alloc(ctx, nvox)) != ITS_OK) return st;
     cubeD = cubeTmp.p;
   }
-  // tile of 256 threads x ITEMS voxels; the autotuner picks ITEMS (same bits for every choice)
+  // tiles of 32 lanes x ITEMS voxels; the autotuner picks ITEMS (same bits for every choice)
   const int itemsOf[3] = {8, 16, 4};
-  const int64_t nbMax = (nvox + kScanThreads * 4 - 1) / (kScanThreads * 4);
+  const int64_t points = M * M * M, signBlocks = (points + 32 * kSignWords * (kScanThreads / 32) - 1) /
+                                                 (32 * kSignWords * (kScanThreads / 32));
   DevBuf<unsigned long long> sums, tot;
-  if ((st = sums.alloc(ctx, nbMax + spineTops(nbMax))) != ITS_OK || (st = tot.alloc(ctx, 1)) != ITS_OK) return st;
+  DevBuf<uint32_t> signs, listed;  // a window reads the word after its own
+  DevBuf<unsigned> numListed;
+  if ((st = tot.alloc(ctx, 1)) != ITS_OK || (st = numListed.alloc(ctx, 1)) != ITS_OK ||
+      (st = signs.alloc(ctx, signBlocks * (kScanThreads / 32) * kSignWords + 1)) != ITS_OK)
+    return st;
   const double3 o3 = make_double3(origin[0], origin[1], origin[2]);
   const double3 v3 = make_double3(width[0] / res, width[1] / res, width[2] / res);
-  auto run = [&](int i) -> its_status {
-    const int items = itemsOf[i];
-    const int64_t nb = (nvox + kScanThreads * items - 1) / (kScanThreads * items);
-    if (items == 16)
-      kMcClassify<FT, 16><<<(unsigned)nb, kScanThreads, 0, ctx->stream>>>(F.d, res, iso, cubeD, sums.p);
-    else if (items == 4)
-      kMcClassify<FT, 4><<<(unsigned)nb, kScanThreads, 0, ctx->stream>>>(F.d, res, iso, cubeD, sums.p);
-    else if (res % 256 == 0)
-      kMcClassifyRows<FT><<<(unsigned)nb, kScanThreads, 0, ctx->stream>>>(F.d, res, iso, cubeD, sums.p);
+  auto runTiles = [&](auto itemsTag) -> its_status {
+    constexpr int kItems = decltype(itemsTag)::value;
+    const int64_t nt = (nvox + 32 * kItems - 1) / (32 * kItems);
+    if ((int64_t)sums.n != nt + spineTops(nt) &&
+        ((st = sums.alloc(ctx, nt + spineTops(nt))) != ITS_OK || (T.d && (st = listed.alloc(ctx, nt)) != ITS_OK)))
+      return st;
+    // four tiles per warp once that many keep every SM full of warps
+    constexpr int kWarps = kScanThreads / 32;
+    if (nt >= 4ll * 64 * ctx->numSMs)
+      kMcCases<kItems, 4><<<(unsigned)((nt + 4 * kWarps - 1) / (4 * kWarps)), kScanThreads, 0, ctx->stream>>>(
+          signs.p, res, fastDiv(res), cubeD, nt, sums.p, listed.p, numListed.p);
     else
-      kMcClassify<FT, 8><<<(unsigned)nb, kScanThreads, 0, ctx->stream>>>(F.d, res, iso, cubeD, sums.p);
+      kMcCases<kItems, 1><<<(unsigned)((nt + kWarps - 1) / kWarps), kScanThreads, 0, ctx->stream>>>(
+          signs.p, res, fastDiv(res), cubeD, nt, sums.p, listed.p, numListed.p);
     ITS_LAUNCHED(ctx);
-    if ((st = scanSpine<unsigned long long>(ctx, sums.p, nb, tot.p, sums.p + nbMax)) != ITS_OK) return st;
+    if ((st = scanSpine<unsigned long long>(ctx, sums.p, nt, tot.p, sums.p + nt)) != ITS_OK) return st;
     if (T.d) {
-      const unsigned long long cap = (unsigned long long)capacity;
-      if (items == 16)
-        kMcEmit<FT, 16><<<(unsigned)nb, kScanThreads, 0, ctx->stream>>>(mc, o3, v3, cubeD, sums.p, tot.p, T.d, cap);
-      else if (items == 4)
-        kMcEmit<FT, 4><<<(unsigned)nb, kScanThreads, 0, ctx->stream>>>(mc, o3, v3, cubeD, sums.p, tot.p, T.d, cap);
-      else
-        kMcEmit<FT, 8><<<(unsigned)nb, kScanThreads, 0, ctx->stream>>>(mc, o3, v3, cubeD, sums.p, tot.p, T.d, cap);
+      kMcEmit<FT, kItems><<<(unsigned)std::min<int64_t>((nt + kWarps - 1) / kWarps, 8ll * ctx->numSMs), kScanThreads, 0,
+                            ctx->stream>>>(mc, fastDiv(res), o3, v3, cubeD, sums.p, listed.p, numListed.p, T.d,
+                                           (unsigned long long)capacity);
       ITS_LAUNCHED(ctx);
     }
     return ITS_OK;
   };
+  auto run = [&](int i) -> its_status {
+    kMcSigns<FT><<<(unsigned)signBlocks, kScanThreads, 0, ctx->stream>>>(F.d, points, iso, signs.p, numListed.p);
+    ITS_LAUNCHED(ctx);
+    if (itemsOf[i] == 16) return runTiles(std::integral_constant<int, 16>());
+    if (itemsOf[i] == 4) return runTiles(std::integral_constant<int, 4>());
+    return runTiles(std::integral_constant<int, 8>());
+  };
   const std::string key = std::string("marching_cubes/") + (sizeof(FT) == 8 ? "f64" : "f32") + "/res=" +
                           std::to_string(res) + (T.d ? "/soup" : "/cases");
   int choice = 0;
-  if ((st = tuneChoice(ctx, key, 3, 0, run, &choice)) != ITS_OK) return st;
+  // By default the shortest runs on small grids, so that every SM has warps, and longer ones as the
+  // grid grows (us with 4, 8, 16 voxels per lane: 67^3 62, 70, 85; 128^3 79, 84, 96; 330^3 219, 190,
+  // 200; 512^3 477, 376, 328).
+  const int def = nvox < (1ll << 22) ? 2 : (nvox < (1ll << 26) ? 0 : 1);
+  if ((st = tuneChoice(ctx, key, 3, def, run, &choice)) != ITS_OK) return st;
   if ((st = run(choice)) != ITS_OK) return st;
   unsigned long long total = 0;
   if ((st = readScalar(ctx, tot.p, &total)) != ITS_OK) return st;
