@@ -24,7 +24,9 @@
 #include <vector>
 
 #include "its_op.cuh"
+#include "its_rows.cuh"
 #include "its_scan.cuh"
+#include "its_segs.cuh"
 #include "its_umma.cuh"
 
 namespace its {
@@ -147,7 +149,8 @@ __device__ __forceinline__ bool coincidentVertex(const FeatParams& P, int64_t v,
   return (((lin / (M * M)) | ((lin / M) % M) | (lin % M)) & 1u) == 0u;
 }
 // Vertex index of lattice point (X,Y,Z) at depth d, or -1.
-__device__ __forceinline__ int64_t latticeVertex(const FeatParams& P, int d, int64_t X, int64_t Y, int64_t Z) {
+template <class Params>
+__device__ __forceinline__ int64_t latticeVertex(const Params& P, int d, int64_t X, int64_t Y, int64_t Z) {
   if (d < 0 || d >= P.depth) return -1;
   const LatticeIndex& L = P.lat[d];
   if (X < 0 || Y < 0 || Z < 0 || X >= L.M || Y >= L.M || Z >= L.M) return -1;
@@ -157,7 +160,8 @@ __device__ __forceinline__ int64_t latticeVertex(const FeatParams& P, int d, int
 
 // latticeVertex with both words (presence bits and rank) loaded up front, so that independent
 // lookups issued together overlap their memory latency; -1 where no vertex is.
-__device__ __forceinline__ int64_t latticeVertexIlp(const FeatParams& P, int d, int64_t X, int64_t Y, int64_t Z) {
+template <class Params>
+__device__ __forceinline__ int64_t latticeVertexIlp(const Params& P, int d, int64_t X, int64_t Y, int64_t Z) {
   if (d < 0 || d >= P.depth) return -1;
   const LatticeIndex& L = P.lat[d];
   if (X < 0 || Y < 0 || Z < 0 || X >= L.M || Y >= L.M || Z >= L.M) return -1;
@@ -180,31 +184,37 @@ struct FeatNorm {
   int on;
 };
 
-constexpr int kFeatLanes = 4;                       // lanes per vertex
-constexpr int kFeatThreads = 128;
-constexpr int kFeatRows = kFeatThreads / kFeatLanes;  // vertices per block
+static FeatNorm featNorm(const float* host) {  // no normalisation where null
+  FeatNorm norm;
+  norm.on = host != nullptr;
+  for (int k = 0; k < 2 * kFeat; ++k) norm.v[k] = host ? host[k] : 0.0f;
+  return norm;
+}
 
-// Four lanes per vertex: lane 0 the coincident copies above and the scalar features, lane 1
-// the copies below, the face neighbours split over the lanes, lane 3 also the sample features
-// of the owner's 27-neighbourhood (computed with the octree, kCoincGeom). The block's rows go
-// through shared memory so that the normalised features leave in coalesced stores.
-__global__ void __launch_bounds__(kFeatThreads) kShareFeatures(const __grid_constant__ FeatParams P,
-                                                               const int64_t* __restrict__ ids, int64_t count,
-                                                               const double* __restrict__ b,
-                                                               const double* __restrict__ lam0,
-                                                               const float* __restrict__ geom,
-                                                               const __grid_constant__ FeatNorm norm,
-                                                               float* __restrict__ out, __nv_bfloat16* __restrict__ tiles,
-                                                               int64_t tileRow0) {
-  gridDependencyWait();
-  gridDependents();
-  __shared__ __align__(16) float sf[kFeatRows][kFeat];
-  const int sub = threadIdx.x & (kFeatLanes - 1), slot = threadIdx.x / kFeatLanes;
-  const int64_t i0 = (int64_t)blockIdx.x * kFeatRows, i = i0 + slot;
+constexpr int kFeatRoles = 4;                         // warps per 32 vertices
+constexpr int kFeatRows = 32;                         // vertices per block
+constexpr int kFeatThreads = kFeatRows * kFeatRoles;
+
+// A block takes 32 vertices, a lane each, and splits a vertex's features over its four warps: warp 0
+// the coincident copies above and the scalar features, warp 1 the copies below, the face
+// neighbours split over the warps, warp 3 also the sample features of the owner's
+// 27-neighbourhood (computed with the octree, kCoincGeom). (With the parts on four lanes of one
+// warp each warp ran every part in turn: 17.1 us against 12.6 for 33,505 vertices of one octree, 386
+// against 303 for 1.2 million of 24.) The rows go through shared memory, a
+// bank apart, so that the normalised features leave in coalesced stores.
+template <class Params>  // FeatParams by value with the launch, or an octree's RowParams on the device
+__device__ __forceinline__ void featureRows(const Params& P, const int64_t* __restrict__ ids, int64_t count,
+                                            const double* __restrict__ b, const double* __restrict__ lam0,
+                                            const float* __restrict__ geom, const FeatNorm& norm,
+                                            float* __restrict__ out, __nv_bfloat16* __restrict__ tiles,
+                                            int64_t tileRow0, int64_t block) {
+  __shared__ float sf[kFeatRows][kFeat + 1];
+  const int sub = threadIdx.x / kFeatRows, slot = threadIdx.x % kFeatRows;
+  const int64_t i0 = block * kFeatRows, i = i0 + slot;
   float* f = sf[slot];
 #pragma unroll
-  for (int k = 0; k < kFeat / kFeatLanes; ++k) f[sub * (kFeat / kFeatLanes) + k] = 0.0f;
-  __syncwarp();
+  for (int k = 0; k < kFeat / kFeatRoles; ++k) f[sub * (kFeat / kFeatRoles) + k] = 0.0f;
+  __syncthreads();
   const bool valid = i < count;
   int64_t v = 0;
   int d = 0;
@@ -253,18 +263,18 @@ __global__ void __launch_bounds__(kFeatThreads) kShareFeatures(const __grid_cons
         if (down == s - 1 && has[s]) down = s;
       f[5] = (float)down / (float)P.depth;
     }
-    // face neighbours: lanes 0, 1 one each, lanes 2, 3 two each
-    const int ex[6] = {1, -1, 0, 0, 0, 0}, ey[6] = {0, 0, 1, -1, 0, 0}, ez[6] = {0, 0, 0, 0, 1, -1};
+    // face neighbours: warps 0, 1 one each, warps 2, 3 two each
     const int k0 = sub < 2 ? sub : 2 * sub - 2, k1 = sub < 2 ? sub + 1 : 2 * sub;
-    for (int k = k0; k < k1; ++k) {
-      const int64_t u = latticeVertex(P, d, X + ex[k], Y + ey[k], Z + ez[k]);
+    for (int k = k0; k < k1; ++k) {  // +x, -x, +y, -y, +z, -z
+      const int sign = k & 1 ? -1 : 1, ex = k < 2 ? sign : 0, ey = (k >> 1) == 1 ? sign : 0, ez = k > 3 ? sign : 0;
+      const int64_t u = latticeVertex(P, d, X + ex, Y + ey, Z + ez);
       if (u >= 0) {
         f[6 + k] = 1.0f;
         f[12 + k] = (float)(b[u] - bv);
         f[18 + k] = (float)lam0[u];
       }
       if (d > 0) {
-        const int64_t qv = latticeVertex(P, d - 1, 2 * X + ex[k], 2 * Y + ey[k], 2 * Z + ez[k]);
+        const int64_t qv = latticeVertex(P, d - 1, 2 * X + ex, 2 * Y + ey, 2 * Z + ez);
         if (qv >= 0) {
           f[24 + k] = 1.0f;
           f[30 + k] = (float)lam0[qv];
@@ -300,7 +310,7 @@ __global__ void __launch_bounds__(kFeatThreads) kShareFeatures(const __grid_cons
   // the block's rows are consecutive in out: float4 stores over all of them
   for (int e = threadIdx.x; e < rows * (kFeat / 4); e += kFeatThreads) {
     const int r = e / (kFeat / 4), k = 4 * (e % (kFeat / 4));
-    float4 x = *(const float4*)&sf[r][k];
+    float4 x = make_float4(sf[r][k], sf[r][k + 1], sf[r][k + 2], sf[r][k + 3]);
     if (norm.on) {
       x.x = (x.x - norm.v[k]) * norm.v[kFeat + k];
       x.y = (x.y - norm.v[k + 1]) * norm.v[kFeat + k + 1];
@@ -319,14 +329,52 @@ __global__ void __launch_bounds__(kFeatThreads) kShareFeatures(const __grid_cons
   }
 }
 
-// Learned shares of the coincident vertices: share[ids[i]] = pred[i] * scale + mean.
-__global__ void kScatterShares(const int64_t* __restrict__ ids, int64_t count, const float* __restrict__ pred,
-                               float scale, float mean, double* __restrict__ shares) {
+__global__ void __launch_bounds__(kFeatThreads) kShareFeatures(const __grid_constant__ FeatParams P,
+                                                               const int64_t* __restrict__ ids, int64_t count,
+                                                               const double* __restrict__ b,
+                                                               const double* __restrict__ lam0,
+                                                               const float* __restrict__ geom,
+                                                               const __grid_constant__ FeatNorm norm,
+                                                               float* __restrict__ out, __nv_bfloat16* __restrict__ tiles,
+                                                               int64_t tileRow0) {
   gridDependencyWait();
   gridDependents();
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  shares[ids[i]] = (double)pred[i] * (double)scale + (double)mean;
+  featureRows(P, ids, count, b, lam0, geom, norm, out, tiles, tileRow0, blockIdx.x);
+}
+
+// Many octrees in one launch (a block's rows are one octree's): one launch per octree left most of
+// the GPU idle, 24 launches of 22 us for 24 octrees.
+struct FeatSeg {
+  const RowParams* P;
+  const int64_t* ids;
+  int64_t count;
+  const double* b;
+  const double* lam0;
+  const float* geom;
+  int64_t row0;  // the octree's first row in the tiles
+  double* shares;
+};
+__global__ void __launch_bounds__(kFeatThreads) kShareFeaturesBatch(const __grid_constant__ SegArgs<FeatSeg> A,
+                                                                    const __grid_constant__ FeatNorm norm,
+                                                                    __nv_bfloat16* __restrict__ tiles) {
+  gridDependencyWait();
+  gridDependents();
+  const int k = A.find(blockIdx.x);
+  const FeatSeg& s = A.seg(k);
+  featureRows(*s.P, s.ids, s.count, s.b, s.lam0, s.geom, norm, (float*)nullptr, tiles, s.row0, blockIdx.x - A.pre(k));
+}
+
+// Learned shares of the coincident vertices: share[ids[i]] = pred[i] * scale + mean; the blocks are
+// kShareFeaturesBatch's.
+__global__ void __launch_bounds__(kFeatRows) kScatterShares(const __grid_constant__ SegArgs<FeatSeg> A,
+                                                               const float* __restrict__ pred, float scale,
+                                                               float mean) {
+  gridDependencyWait();
+  gridDependents();
+  const int k = A.find(blockIdx.x);
+  const FeatSeg& s = A.seg(k);
+  const int64_t i = (blockIdx.x - A.pre(k)) * kFeatRows + threadIdx.x;
+  if (i < s.count) s.shares[s.ids[i]] = (double)pred[s.row0 + i] * (double)scale + (double)mean;
 }
 
 static FeatParams featParams(const SvoDevice& d) {
@@ -459,23 +507,10 @@ its_status shareFeatures(its_ctx* ctx, const SvoDevice& d, const double* b, cons
                          int64_t count, const float* hostNorm, float* out, bool afterKernel, __nv_bfloat16* tiles,
                          int64_t tileRow0) {
   const FeatParams P = featParams(d);
-  FeatNorm norm;
-  norm.on = hostNorm != nullptr;
-  for (int k = 0; k < 2 * kFeat; ++k) norm.v[k] = hostNorm ? hostNorm[k] : 0.0f;
+  const FeatNorm norm = featNorm(hostNorm);
   if (count > 0) {
     its_status st = launchDependent(ctx, afterKernel, kShareFeatures, gridFor(count, kFeatRows), kFeatThreads, 0, ctx->stream, P, ids,
                                     count, b, lam0, (const float*)d.coincGeom, norm, out, tiles, tileRow0);
-    if (st != ITS_OK) return st;
-  }
-  return ITS_OK;
-}
-
-// Learned shares of the coincident vertices (the exact start reads shares nowhere else).
-its_status scatterShares(its_ctx* ctx, const int64_t* ids, int64_t count, const float* pred, float scale, float mean,
-                         double* shares) {
-  if (count > 0) {
-    its_status st = launchDependent(ctx, true, kScatterShares, gridFor(count, 256), 256, 0, ctx->stream, ids, count, pred, scale,
-                                    mean, shares);
     if (st != ITS_OK) return st;
   }
   return ITS_OK;
@@ -520,19 +555,21 @@ its_status hostNorm(its_ctx* ctx, const float* norm, float* hn) {
 its_status learnedStart(its_ctx* ctx, its_svo* const* svos, int64_t count, its_mlp* mlp, const double* const* b,
                         const float* hn, double* const* lam, unsigned long long* stamp) {
   its_status st;
-  std::vector<DevBuf<double>> lam0(count), shares(count);
   std::vector<const double*> sp(count);
   std::vector<double*> l0(count);
-  std::vector<int64_t> cnt(count);
   int64_t total = 0, verts = 0;
   for (int64_t m = 0; m < count; ++m) {
-    const int64_t n = svos[m]->d.numVerts;
-    if ((st = lam0[m].alloc(ctx, n)) != ITS_OK || (st = shares[m].alloc(ctx, n)) != ITS_OK) return st;
-    l0[m] = lam0[m].p;
-    sp[m] = shares[m].p;
-    cnt[m] = svos[m]->d.numCoinc;
-    total += cnt[m];
-    verts += n;
+    total += svos[m]->d.numCoinc;
+    verts += svos[m]->d.numVerts;
+  }
+  DevBuf<double> lam0, shares;
+  if ((st = lam0.alloc(ctx, std::max<int64_t>(verts, 1))) != ITS_OK ||
+      (st = shares.alloc(ctx, std::max<int64_t>(verts, 1))) != ITS_OK)
+    return st;
+  for (int64_t m = 0, at = 0; m < count; ++m) {
+    l0[m] = lam0.p + at;
+    sp[m] = shares.p + at;
+    at += svos[m]->d.numVerts;
   }
   // every buffer up front: from the first kernel on, each launch follows a kernel (dependent
   // launches, gridDependencyWait at the top of each kernel)
@@ -544,29 +581,37 @@ its_status learnedStart(its_ctx* ctx, its_svo* const* svos, int64_t count, its_m
       (st = pred.alloc(ctx, std::max<int64_t>(total, 1))) != ITS_OK ||
       (st = G.alloc(ctx, std::max<int64_t>(verts, 1))) != ITS_OK)
     return st;
-  if ((st = exactStart(ctx, svos, count, b, nullptr, l0.data(), false, nullptr, stamp)) != ITS_OK) return st;
-  int64_t off = 0;
-  for (int64_t m = 0; m < count; ++m) {
-    if ((st = shareFeatures(ctx, svos[m]->d, b[m], l0[m], svos[m]->d.coincIds, cnt[m], hn, nullptr, true, feat.p,
-                            off)) != ITS_OK)
-      return st;
-    off += cnt[m];
-  }
-  if (count == 1) {  // one octree: the network writes the shares itself
-    if (total > 0 && (st = mlpInferTiles(mlp, feat.p, total, nullptr, svos[0]->d.coincIds, hn[2 * kFeat + 1],
-                                         hn[2 * kFeat], shares[0].p, true)) != ITS_OK)
-      return st;
-  } else {
-    if (total > 0 &&
-        (st = mlpInferTiles(mlp, feat.p, total, pred.p, nullptr, 0.0f, 0.0f, nullptr, true)) != ITS_OK)
-      return st;
-    off = 0;
-    for (int64_t m = 0; m < count; ++m) {
-      if ((st = scatterShares(ctx, svos[m]->d.coincIds, cnt[m], pred.p + off, hn[2 * kFeat + 1], hn[2 * kFeat],
-                              shares[m].p)) != ITS_OK)
-        return st;
-      off += cnt[m];
+  // many octrees: their feature and share tables (more than kInlineSegs are copied, before the kernels)
+  std::vector<FeatSeg> segs;
+  std::vector<int64_t> prefix(1, 0);
+  SegArgs<FeatSeg> A;
+  DevBuf<uint8_t> keep;
+  if (count > 1) {
+    for (int64_t m = 0, row = 0; m < count; ++m) {
+      const SvoDevice& d = svos[m]->d;
+      if (!d.numCoinc) continue;
+      segs.push_back(FeatSeg{(const RowParams*)d.rowParams, d.coincIds, d.numCoinc, b[m], l0[m], d.coincGeom, row,
+                             l0[m] - lam0.p + shares.p});
+      prefix.push_back(prefix.back() + (d.numCoinc + kFeatRows - 1) / kFeatRows);
+      row += d.numCoinc;
     }
+    if (!segs.empty() && (st = makeSegArgs(ctx, segs, prefix, A, keep)) != ITS_OK) return st;
+  }
+  if ((st = exactStart(ctx, svos, count, b, nullptr, l0.data(), false, nullptr, stamp)) != ITS_OK) return st;
+  if (count == 1) {  // one octree: its parameters travel with the launch, and the network writes the shares
+    const SvoDevice& d = svos[0]->d;
+    if ((st = shareFeatures(ctx, d, b[0], l0[0], d.coincIds, total, hn, nullptr, true, feat.p, 0)) != ITS_OK) return st;
+    if (total > 0 && (st = mlpInferTiles(mlp, feat.p, total, nullptr, d.coincIds, hn[2 * kFeat + 1], hn[2 * kFeat],
+                                         shares.p, true)) != ITS_OK)
+      return st;
+  } else if (total > 0) {
+    const unsigned blocks = (unsigned)prefix.back();
+    if ((st = launchDependent(ctx, true, kShareFeaturesBatch, blocks, kFeatThreads, 0, ctx->stream, A, featNorm(hn),
+                              feat.p)) != ITS_OK ||
+        (st = mlpInferTiles(mlp, feat.p, total, pred.p, nullptr, 0.0f, 0.0f, nullptr, true)) != ITS_OK ||
+        (st = launchDependent(ctx, true, kScatterShares, blocks, kFeatRows, 0, ctx->stream, A, (const float*)pred.p,
+                              hn[2 * kFeat + 1], hn[2 * kFeat])) != ITS_OK)
+      return st;
   }
   return exactStart(ctx, svos, count, b, sp.data(), lam, total > 0, G.p, nullptr);
 }

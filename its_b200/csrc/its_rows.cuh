@@ -94,40 +94,83 @@ __device__ __forceinline__ void hatPair(double x, double b, double w, double wi,
   h[1] = (fabs(x - e1) < 1e-9 || x < e1) ? 0.0 : (x <= b1 ? 1 + divRn(x - b1, w, wi) : 1 - divRn(x - b1, w, wi));
 }
 
-// visit(col, val) for the non-zero hats at (qx, qy, qz) of the 8 corners of the depth-dd
-// ancestor of the depth-d vertex c's owner, corners in x-major order. (Corner positions are
-// the cell's origin (+ w), as the reference forms them, so the cell must be the owner's
-// ancestor itself: a neighbouring cell sharing the corner would place it an ulp away.)
+// The depth-dd ancestor of the depth-d vertex c's owner: the axis factors of its 8 corners at
+// (qx, qy, qz), and the lattice index of its lowest corner. (Corner positions are the cell's origin
+// (+ w), as the reference forms them, so the cell must be the owner's ancestor itself: a
+// neighbouring cell sharing the corner would place it an ulp away.)
+struct AncestorHats {
+  double hx[2], hy[2], hz[2];
+  uint32_t lin;
+};
+__device__ __forceinline__ AncestorHats ancestorHats(const RowParams& P, const VertCoord& c, int dd, double qx,
+                                                     double qy, double qz) {
+  AncestorHats A;
+  const int up = dd - c.d;
+  const uint32_t Xa = c.Xo >> up, Ya = c.Yo >> up, Za = c.Zo >> up, M = P.lat[dd].M;
+  const double w = P.w0 * (double)(1u << dd), wi = P.winv[dd];
+  hatPair(qx, latticePos(P.g.x, w, Xa), w, wi, A.hx);
+  hatPair(qy, latticePos(P.g.y, w, Ya), w, wi, A.hy);
+  hatPair(qz, latticePos(P.g.z, w, Za), w, wi, A.hz);
+  A.lin = (Xa * M + Ya) * M + Za;
+  return A;
+}
+
+// visit(col, val) for the non-zero hats at (qx, qy, qz) of that ancestor's corners, in x-major order.
 template <class Visit>
 __device__ __forceinline__ void walkAncestor(const RowParams& P, const VertCoord& c, int dd, double qx, double qy,
                                              double qz, Visit&& visit) {
-  const int up = dd - c.d;
   const LatticeIndex& L = P.lat[dd];
-  const uint32_t Xa = c.Xo >> up, Ya = c.Yo >> up, Za = c.Zo >> up;
-  const double w = P.w0 * (double)(1u << dd), wi = P.winv[dd];
-  const double bx = latticePos(P.g.x, w, Xa), by = latticePos(P.g.y, w, Ya), bz = latticePos(P.g.z, w, Za);
-  // the six axis factors once (the corners share them)
-  double hxs[2], hys[2], hzs[2];
-  hatPair(qx, bx, w, wi, hxs);
-  hatPair(qy, by, w, wi, hys);
-  hatPair(qz, bz, w, wi, hzs);
+  const AncestorHats A = ancestorHats(P, c, dd, qx, qy, qz);
 #pragma unroll
   for (int ox = 0; ox < 2; ++ox) {
-    const double hx = hxs[ox];
+    const double hx = A.hx[ox];
     if (hx <= 0.0) continue;
 #pragma unroll
     for (int oy = 0; oy < 2; ++oy) {
-      const double hy = hys[oy];
+      const double hy = A.hy[oy];
       if (hy <= 0.0) continue;
 #pragma unroll
       for (int oz = 0; oz < 2; ++oz) {
-        const double hz = hzs[oz];
+        const double hz = A.hz[oz];
         if (hz <= 0.0) continue;
         const double v = hx * hy * hz;
         if (v == 0.0) continue;
-        visit((int32_t)latticeRank(L, ((Xa + ox) * L.M + (Ya + oy)) * L.M + (Za + oz)), v);
+        visit((int32_t)latticeRank(L, A.lin + (ox * L.M + oy) * L.M + oz), v);
       }
     }
+  }
+}
+
+// acc + src[col] * val over walkAncestor's entries, in its order and with its values, with the loads
+// ahead of the sums: the counting columns' lattice words and ranks together, then the values. All
+// 8 corners of a node are vertices, so the upper one of a z pair is the column after the lower
+// one's: one word and rank per pair. (7.3 million rows: 198 us an interpolation with walkAncestor's
+// one corner after another, 178 so.)
+__device__ __forceinline__ void addAncestor(const RowParams& P, const VertCoord& c, int dd, double qx, double qy,
+                                            double qz, const double* __restrict__ src, double& acc) {
+  const LatticeIndex& L = P.lat[dd];
+  const AncestorHats A = ancestorHats(P, c, dd, qx, qy, qz);
+  unsigned long long bits[4];
+  uint32_t rank[4];
+  bool on[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint32_t lin = A.lin + ((k >> 1) * L.M + (k & 1)) * L.M;
+    on[k] = A.hx[k >> 1] > 0.0 && A.hy[k & 1] > 0.0;
+    bits[k] = on[k] ? __ldg(L.bits + (lin >> 6)) & ((1ull << (lin & 63)) - 1ull) : 0ull;
+    rank[k] = on[k] ? __ldg(L.rank + (lin >> 6)) : 0u;
+  }
+  double s[8];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double* at = src + L.base + rank[k] + (uint32_t)__popcll(bits[k]);
+    s[2 * k] = on[k] && A.hz[0] > 0.0 ? at[0] : 0.0;
+    s[2 * k + 1] = on[k] && A.hz[1] > 0.0 ? at[1] : 0.0;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const double v = A.hx[k >> 2] * A.hy[(k >> 1) & 1] * A.hz[k & 1];
+    if (on[k >> 1] && A.hz[k & 1] > 0.0 && v != 0.0) acc += v * s[k];
   }
 }
 

@@ -40,6 +40,7 @@
 
 #include "its_op.cuh"
 #include "its_rows.cuh"
+#include "its_segs.cuh"
 #include "its_tune.cuh"
 
 namespace its {
@@ -47,73 +48,21 @@ namespace its {
 // One octree of an exact start.
 struct RowSeg {
   const RowParams* P;    // the octree's row parameters (device)
-  int64_t rowBegin, rows;
+  int64_t rows;
   const double* b;
   const double* shares;  // may be null (all shares 0)
   double* g;             // values less the finer shares (b itself when there are no shares)
   double* lam;
 };
 
-// A segment table and its prefix. Up to kInlineSegs segments travel with the launch as a
-// kernel parameter (no copy, nothing to wait for); a larger table is copied to the device once
-// (from pageable memory, staged at the call) into keep, which the caller holds until the
-// launches are queued.
-constexpr int kInlineSegs = 16;
-template <class Seg>
-struct SegArgs {
-  int nseg = 0;
-  const Seg* dsegs = nullptr;
-  const int64_t* dprefix = nullptr;
-  unsigned long long* stamp = nullptr;  // when set: the device clock (ns) at the kernel's start
-  Seg segs[kInlineSegs];
-  int64_t prefix[kInlineSegs + 1];
-  __device__ __forceinline__ const Seg& seg(int k) const { return dsegs ? dsegs[k] : segs[k]; }
-  __device__ __forceinline__ int64_t pre(int k) const { return dsegs ? dprefix[k] : prefix[k]; }
-  // last segment whose first item is <= i
-  __device__ __forceinline__ int find(int64_t i) const {
-    int lo = 0, hi = nseg - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (pre(mid) <= i) lo = mid;
-      else hi = mid - 1;
-    }
-    return lo;
-  }
-};
-
-template <class Seg>
-static its_status makeSegArgs(its_ctx* ctx, const std::vector<Seg>& segs, const std::vector<int64_t>& prefix,
-                              SegArgs<Seg>& A, DevBuf<uint8_t>& keep) {
-  A.nseg = (int)segs.size();
-  if (A.nseg <= kInlineSegs) {
-    for (int k = 0; k < A.nseg; ++k) {
-      A.segs[k] = segs[k];
-      A.prefix[k] = prefix[k];
-    }
-    A.prefix[A.nseg] = prefix[A.nseg];
-    return ITS_OK;
-  }
-  const size_t a = segs.size() * sizeof(Seg), b = (segs.size() + 1) * sizeof(int64_t);
-  std::vector<uint8_t> h(a + b);
-  std::memcpy(h.data(), segs.data(), a);
-  std::memcpy(h.data() + a, prefix.data(), b);
-  its_status st;
-  if ((st = keep.alloc(ctx, a + b)) != ITS_OK) return st;
-  ITS_CU(ctx, cudaMemcpyAsync(keep.p, h.data(), a + b, cudaMemcpyHostToDevice, ctx->stream));
-  A.dsegs = (const Seg*)keep.p;
-  A.dprefix = (const int64_t*)(keep.p + a);
-  return ITS_OK;
-}
-
 // G_r = b_r - the shares of the finer coincident vertices at r's point (finest first).
-__global__ void __launch_bounds__(256) kStartValues(const __grid_constant__ SegArgs<RowSeg> A, int64_t total) {
+__global__ void __launch_bounds__(256) kStartValues(const __grid_constant__ SegArgs<RowSeg> A) {
   gridDependencyWait();
   gridDependents();
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const int k = A.find(i);
+  const int k = A.find(blockIdx.x);
   const RowSeg& s = A.seg(k);
-  const int64_t r = s.rowBegin + (i - A.pre(k));
+  const int64_t r = (blockIdx.x - A.pre(k)) * blockDim.x + threadIdx.x;
+  if (r >= s.rows) return;
   const RowParams& P = *s.P;
   double acc = 0.0;
   if (s.shares) {
@@ -125,15 +74,14 @@ __global__ void __launch_bounds__(256) kStartValues(const __grid_constant__ SegA
 
 // lambda_r: the share of a coincident vertex; otherwise G_r less the interpolant of G over
 // the corners of the owner's parent cell (the row's hats of that depth, in column order).
-__global__ void __launch_bounds__(256) kStartInterp(const __grid_constant__ SegArgs<RowSeg> A, int64_t total) {
+__global__ void __launch_bounds__(256) kStartInterp(const __grid_constant__ SegArgs<RowSeg> A) {
   gridDependencyWait();
   gridDependents();
   if (A.stamp && blockIdx.x == 0 && threadIdx.x == 0) *A.stamp = globalTimer();
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const int k = A.find(i);
+  const int k = A.find(blockIdx.x);
   const RowSeg& s = A.seg(k);
-  const int64_t r = s.rowBegin + (i - A.pre(k));
+  const int64_t r = (blockIdx.x - A.pre(k)) * blockDim.x + threadIdx.x;
+  if (r >= s.rows) return;
   const RowParams& P = *s.P;
   const VertCoord v = vertCoord(P, r);
   if (coordCoincident(P, v)) {
@@ -143,8 +91,7 @@ __global__ void __launch_bounds__(256) kStartInterp(const __grid_constant__ SegA
   const double* __restrict__ g = s.g;
   double acc = 0.0;
   if (v.d + 1 < P.depth)
-    walkAncestor(P, v, v.d + 1, P.vertPos[3 * r], P.vertPos[3 * r + 1], P.vertPos[3 * r + 2],
-                 [&](int32_t c, double h) { acc += h * g[c]; });
+    addAncestor(P, v, v.d + 1, P.vertPos[3 * r], P.vertPos[3 * r + 1], P.vertPos[3 * r + 2], g, acc);
   s.lam[r] = g[r] - acc;
 }
 
@@ -153,12 +100,13 @@ __global__ void __launch_bounds__(256) kStartInterp(const __grid_constant__ SegA
 // F_{>d}(v) is the field of v's own and the coarser depths at v. F_{>d} is trilinear on the
 // owner's parent cell (the argument of the exact start), so
 //   H_v = lambda_v + sum_{corners c of the parent cell} hat_c(v) H_c:
-// the same operator with 8 hats per row instead of 8 per ancestor. Two bands, each one launch
-// for all octrees: the vertices above the finest depth sum H_v as row v has it (the hats of
-// every ancestor's corners); then the finest depth -- most of the rows, with the most
-// ancestors -- interpolates H from the band above. Every chunk of rows (32 in the coarse band,
-// 256 at the finest depth) leaves its sums of e^2 and b^2 in a slot of its own, a mesh's slots
-// contiguous, and kResidualFinish adds a mesh's slots in a fixed order.
+// the same operator with 8 hats per row instead of 8 per ancestor. Few rows above the finest depth:
+// two bands, each one launch for all octrees, the vertices above the finest depth summing H_v as
+// row v has it (the hats of every ancestor's corners), then the finest depth -- most of the rows,
+// with the most ancestors -- interpolating H from the band above. Many (a batch of octrees): a
+// launch per depth, coarsest first, each interpolating H from the depth before. Every chunk of
+// rows (32 in the coarse band, else 256) leaves its sums of e^2 and b^2 in a slot of its own, a
+// mesh's slots contiguous, and kResidualFinish adds a mesh's slots in a fixed order.
 constexpr int kResThreads = 256;
 
 struct ResSeg {
@@ -170,7 +118,8 @@ struct ResSeg {
   int64_t slot;            // slot of the segment's first chunk
 };
 
-// The finest depth: one row per thread, H interpolated from the parent cell's corners.
+// One depth: one row per thread, H interpolated from the parent cell's corners, and kept where a
+// finer depth will read it.
 __global__ void __launch_bounds__(kResThreads) kResidualFine(const __grid_constant__ SegArgs<ResSeg> A,
                                                             double* __restrict__ part) {
   gridDependencyWait();
@@ -185,12 +134,12 @@ __global__ void __launch_bounds__(kResThreads) kResidualFine(const __grid_consta
     const int64_t r = s.rowBegin + i;
     const VertCoord v = vertCoord(P, r);
     const double* __restrict__ lam = s.lam;
-    const double* __restrict__ H = s.H;
+    const double* H = s.H;
     double acc = 0.0;
     if (v.d + 1 < P.depth)
-      walkAncestor(P, v, v.d + 1, P.vertPos[3 * r], P.vertPos[3 * r + 1], P.vertPos[3 * r + 2],
-                   [&](int32_t c, double h) { acc += h * H[c]; });
+      addAncestor(P, v, v.d + 1, P.vertPos[3 * r], P.vertPos[3 * r + 1], P.vertPos[3 * r + 2], H, acc);
     const double h = lam[r] + acc;
+    if (v.d > 0) s.H[r] = h;
     double chain = 0.0;
     walkChain(P, v.d, v.X, v.Y, v.Z, [&](int32_t c) { chain += lam[c]; });
     const double e = s.b[r] - (chain + h);
@@ -344,36 +293,33 @@ its_status exactStart(its_ctx* ctx, its_svo* const* svos, int64_t count, const d
     if (!n) continue;
     RowSeg s;
     s.P = rowParamsOf(svos[m]);
-    s.rowBegin = 0;
     s.rows = n;
     s.b = b[m];
     s.shares = shares ? shares[m] : nullptr;
     s.g = anyShares ? g + acc : const_cast<double*>(b[m]);  // no shares anywhere: G = b
     s.lam = lam[m];
     segs.push_back(s);
-    prefix.push_back(acc);
     acc += n;
   }
   if (segs.empty()) return ITS_OK;
-  prefix.push_back(acc);
-  SegArgs<RowSeg> A;
-  DevBuf<uint8_t> keep;
-  if ((st = makeSegArgs(ctx, segs, prefix, A, keep)) != ITS_OK) return st;
-  A.stamp = stamp;
   // dependent launches only straight after a kernel (no segment table copied in between; not
   // while the autotuner times candidates, which records events between them)
   bool timing = true;
-  const bool dep = afterKernel && !A.dsegs;
-  // a thread per row, no block-level sums: the block size is result-neutral and tuned
+  // a thread per row, no block-level sums: the block size is result-neutral and tuned. A block's
+  // rows are one octree's, so that its table entry and parameters are the same for every thread.
   static const int kStartBlocks[3] = {256, 128, 64};
+  DevBuf<uint8_t> keep;
   auto run = [&](int c) -> its_status {
     const int bs = kStartBlocks[c];
-    if (anyShares &&
-        (st = launchDependent(ctx, dep && !timing, kStartValues, gridFor(total, bs), bs, 0, ctx->stream, A, total)) !=
-            ITS_OK)
-      return st;
-    return launchDependent(ctx, anyShares || (dep && !timing), kStartInterp, gridFor(total, bs), bs, 0, ctx->stream, A,
-                           total);
+    prefix.assign(1, 0);
+    for (const RowSeg& s : segs) prefix.push_back(prefix.back() + (s.rows + bs - 1) / bs);
+    SegArgs<RowSeg> A;
+    if ((st = makeSegArgs(ctx, segs, prefix, A, keep)) != ITS_OK) return st;
+    A.stamp = stamp;
+    const bool dep = afterKernel && !A.dsegs && !timing;
+    const unsigned blocks = (unsigned)prefix.back();
+    if (anyShares && (st = launchDependent(ctx, dep, kStartValues, blocks, bs, 0, ctx->stream, A)) != ITS_OK) return st;
+    return launchDependent(ctx, anyShares || dep, kStartInterp, blocks, bs, 0, ctx->stream, A);
   };
   const std::string key = std::string("exact_start/rows=") + std::to_string(total) + "/octrees=" +
                           std::to_string(count) + (anyShares ? "/shares" : "/zero");
@@ -399,28 +345,37 @@ its_status fitResidualEnqueue(its_ctx* ctx, its_svo* const* svos, int64_t count,
   for (int64_t m = 0; m < count; ++m) total += svos[m]->d.numVerts;
   DevBuf<double> H;
   if ((st = H.alloc(ctx, std::max<int64_t>(total, 1))) != ITS_OK) return st;
-  // band 0: depths >= 1; band 1: the finest depth. Mesh m owns slots [mFirst[m], mFirst[m+1]):
-  // its band 0 chunks, then band 1's.
-  constexpr int kBands = 2;
-  std::vector<ResSeg> segs[kBands];
-  std::vector<int64_t> cf[kBands];
-  int64_t chunks[kBands] = {0, 0};
+  // The bands: above the finest depth in one, or a depth each where those rows are many enough to
+  // outweigh the launches (24 octrees, 1.8 million rows above the finest depth: the residual 779 us
+  // in two bands, 354 a depth at a time; the benchmark tube's 54,000 take 20 us in one band, about
+  // the time of 8 launches that wait for one another). Mesh m owns slots [mFirst[m], mFirst[m+1]): its chunks, coarsest band first.
+  int64_t above = 0;
+  int maxDepth = 1;
+  for (int64_t m = 0; m < count; ++m) {
+    above += svos[m]->d.numVerts - svos[m]->d.vertCount[0];
+    maxDepth = std::max(maxDepth, svos[m]->d.depth);
+  }
+  const bool sweep = above >= 200000;
+  const int bands = sweep ? maxDepth : 2;
+  std::vector<std::vector<ResSeg>> segs(bands);
+  std::vector<std::vector<int64_t>> cf(bands);
+  std::vector<int64_t> chunks(bands, 0);
   std::vector<int64_t> mFirst(count + 1, 0);
   for (int64_t m = 0, h = 0; m < count; ++m) {
     const SvoDevice& d = svos[m]->d;
     auto vs = [&](int k) { return d.vertStart[k < d.depth ? k : d.depth]; };
-    const int64_t lo[kBands] = {vs(1), 0}, hi[kBands] = {d.numVerts, vs(1)};
     int64_t slot = mFirst[m];
-    for (int band = 0; band < kBands; ++band) {
+    for (int band = 0; band < bands; ++band) {
+      const int dd = bands - 1 - band;  // the band's depth (the first of two: depths >= 1)
       ResSeg s;
       s.P = rowParamsOf(svos[m]);
-      s.rowBegin = lo[band];
-      s.rows = hi[band] - lo[band];
+      s.rowBegin = vs(dd);
+      s.rows = (sweep || dd == 0 ? vs(dd + 1) : d.numVerts) - vs(dd);
       s.b = b[m];
       s.lam = lam[m];
       s.H = H.p + h;
       s.slot = slot;
-      const int64_t per = band == 0 ? kResCoarseRows : kResThreads;  // rows per chunk
+      const int64_t per = sweep || dd == 0 ? kResThreads : kResCoarseRows;  // rows per chunk
       const int64_t c = (s.rows + per - 1) / per;
       if (!c) continue;
       segs[band].push_back(s);
@@ -432,9 +387,9 @@ its_status fitResidualEnqueue(its_ctx* ctx, its_svo* const* svos, int64_t count,
     h += d.numVerts;
   }
   const int64_t slots = mFirst[count];
-  SegArgs<ResSeg> A[kBands];
-  DevBuf<uint8_t> keep[kBands + 1];
-  for (int band = 0; band < kBands; ++band) {
+  std::vector<SegArgs<ResSeg>> A(bands);
+  std::vector<DevBuf<uint8_t>> keep(bands + 1);
+  for (int band = 0; band < bands; ++band) {
     cf[band].push_back(chunks[band]);
     if ((st = makeSegArgs(ctx, segs[band], cf[band], A[band], keep[band])) != ITS_OK) return st;
   }
@@ -445,25 +400,24 @@ its_status fitResidualEnqueue(its_ctx* ctx, its_svo* const* svos, int64_t count,
   if (count <= kInlineSegs) {
     for (int64_t m = 0; m <= count; ++m) F.first[m] = mFirst[m];
   } else {
-    if ((st = keep[kBands].alloc(ctx, (count + 1) * 8)) != ITS_OK) return st;
-    ITS_CU(ctx, cudaMemcpyAsync(keep[kBands].p, mFirst.data(), (count + 1) * 8, cudaMemcpyHostToDevice, ctx->stream));
-    F.dfirst = (const int64_t*)keep[kBands].p;
+    if ((st = keep[bands].alloc(ctx, (count + 1) * 8)) != ITS_OK) return st;
+    ITS_CU(ctx, cudaMemcpyAsync(keep[bands].p, mFirst.data(), (count + 1) * 8, cudaMemcpyHostToDevice, ctx->stream));
+    F.dfirst = (const int64_t*)keep[bands].p;
   }
   DevBuf<double> part;
   if ((st = part.alloc(ctx, 2 * std::max<int64_t>(slots, 1))) != ITS_OK) return st;
-  // the coarse band first: the finest rows interpolate the H values it writes
-  if (chunks[0]) {
-    // dependent only straight after the caller's kernel (no table copied in between)
-    const bool dep = afterKernel && !A[0].dsegs && !F.dfirst;
-    if ((st = launchDependent(ctx, dep, kResidualCoarse, (unsigned)chunks[0], kResThreads, 0, ctx->stream, A[0],
-                              part.p)) != ITS_OK)
-      return st;
-  }
-  for (int band = 1; band < kBands; ++band) {
+  // coarsest band first: the next interpolates the H values it writes. Dependent on the caller's
+  // kernel only straight after it (no table copied in between).
+  bool tables = F.dfirst != nullptr;
+  for (int band = 0; band < bands; ++band) tables = tables || A[band].dsegs;
+  bool dep = afterKernel && !tables;
+  for (int band = 0; band < bands; ++band) {
     if (!chunks[band]) continue;
-    if ((st = launchDependent(ctx, chunks[0] > 0, kResidualFine, (unsigned)chunks[band], kResThreads, 0, ctx->stream,
-                              A[band], part.p)) != ITS_OK)
+    const bool fine = sweep || band == 1;
+    if ((st = launchDependent(ctx, dep, fine ? kResidualFine : kResidualCoarse, (unsigned)chunks[band], kResThreads, 0,
+                              ctx->stream, A[band], part.p)) != ITS_OK)
       return st;
+    dep = true;
   }
   if (!slots) ITS_CU(ctx, cudaMemsetAsync(part.p, 0, 16, ctx->stream));
   if ((st = launchDependent(ctx, slots > 0, kResidualFinish, (unsigned)count, kResThreads, 0, ctx->stream, (const double*)part.p,
