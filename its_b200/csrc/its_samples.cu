@@ -86,8 +86,46 @@ struct SampleParams {
 __device__ inline bool inRange(double l, double r, double q) { return l <= q && q <= r; }
 __device__ inline bool isLargeDouble(double l, double r) { return !(fabs(l - r) < 1e-9) && l > r; }
 
-// Edge-step hits of mesh edge (p1,p2); emit == nullptr only counts.
-__device__ int edgeHits(const SampleParams& S, const double* p1, const double* p2, double* emit) {
+// Edge-step hits of mesh edge (p1,p2): the reference tests the min faces of every fine node in the
+// edge's voxel box grown by one. The point where the edge meets lattice plane i of an axis is the same
+// for every node there, so each plane of the box is met once (a quotient per plane instead of three
+// per node), and only the nodes whose face can hold the point are looked up: the cell of each lateral
+// coordinate and its neighbours (3.1 million edge slots: 441 us a count with every node of the box
+// tested, 105 so). Same values, same tests. emit == nullptr only counts; else the points
+// go out in the reference's order, cell by cell (x fastest), planes x, y, z within a cell.
+constexpr int kEdgeList = 8;  // hits sorted in registers' reach; longer edges write by the full sweep
+template <class Hit>
+__device__ __forceinline__ void edgePlaneHits(const SampleParams& S, const double* p1, const double* dir, const int* lo,
+                                              const int* hi, Hit hit) {
+  const double org[3] = {S.g.x, S.g.y, S.g.z};
+  const double w = S.w0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    if (dir[a] == 0) continue;
+    const int b = a == 0 ? 1 : 0, c = a == 2 ? 1 : 2;
+    for (int i = lo[a]; i <= hi[a]; ++i) {
+      const double tt = (latticePos(org[a], w, (uint32_t)i) - p1[a]) / dir[a];
+      if (!inRange(0.0, 1.0, tt)) continue;
+      double q[3];
+#pragma unroll
+      for (int e = 0; e < 3; ++e) q[e] = p1[e] + tt * dir[e];
+      // (a cell quotient's rounding moves a floor by at most one)
+      const int jb = (int)floor((q[b] - org[b]) / w), jc = (int)floor((q[c] - org[c]) / w);
+      for (int u = max(jb - 1, lo[b]); u <= min(jb + 1, hi[b]); ++u) {
+        const double lb = latticePos(org[b], w, (uint32_t)u);
+        if (!inRange(lb, lb + w, q[b])) continue;
+        for (int v = max(jc - 1, lo[c]); v <= min(jc + 1, hi[c]); ++v) {
+          const double lc = latticePos(org[c], w, (uint32_t)v);
+          if (!inRange(lc, lc + w, q[c])) continue;
+          const int x = a == 0 ? i : u, y = a == 1 ? i : (a == 0 ? u : v), z = a == 2 ? i : v;
+          const uint32_t m = mortonEncode(x, y, z);
+          if ((S.fineOcc[m >> 6] >> (m & 63)) & 1ull) hit(x, y, z, a, q);
+        }
+      }
+    }
+  }
+}
+__device__ int edgeHits(const SampleParams& S, const double* p1, const double* p2, int count, double* emit) {
   const double dir[3] = {p2[0] - p1[0], p2[1] - p1[1], p2[2] - p1[2]};
   const double org[3] = {S.g.x, S.g.y, S.g.z};
   int lo[3], hi[3];
@@ -97,6 +135,31 @@ __device__ int edgeHits(const SampleParams& S, const double* p1, const double* p
     hi[a] = clampi((d1 > d2 ? d1 : d2) + 1, 0, S.res - 1);
   }
   int n = 0;
+  if (!emit) {
+    edgePlaneHits(S, p1, dir, lo, hi, [&](int, int, int, int, const double*) { ++n; });
+    return n;
+  }
+  if (count <= kEdgeList) {
+    // a hit's place is the number of hits before it in (z, y, x, plane) order
+    uint64_t key[kEdgeList];
+    edgePlaneHits(S, p1, dir, lo, hi, [&](int x, int y, int z, int a, const double*) {
+      const uint64_t k = (((uint64_t)z << 20 | (uint64_t)y << 10 | (uint64_t)x) << 2) | (uint64_t)a;
+#pragma unroll
+      for (int e = 0; e < kEdgeList; ++e)
+        if (e == n) key[e] = k;
+      ++n;
+    });
+    edgePlaneHits(S, p1, dir, lo, hi, [&](int x, int y, int z, int a, const double* q) {
+      const uint64_t k = (((uint64_t)z << 20 | (uint64_t)y << 10 | (uint64_t)x) << 2) | (uint64_t)a;
+      int at = 0;
+#pragma unroll
+      for (int e = 0; e < kEdgeList; ++e) at += e < n && key[e] < k;
+      emit[3 * at] = q[0];
+      emit[3 * at + 1] = q[1];
+      emit[3 * at + 2] = q[2];
+    });
+    return n;
+  }
   for (int z = lo[2]; z <= hi[2]; ++z)
     for (int y = lo[1]; y <= hi[1]; ++y)
       for (int x = lo[0]; x <= hi[0]; ++x) {
@@ -112,7 +175,9 @@ __device__ int edgeHits(const SampleParams& S, const double* p1, const double* p
           for (int c = 0; c < 3; ++c) q[c] = p1[c] + tt[a] * dir[c];
           const int b = a == 0 ? 1 : 0, c = a == 2 ? 1 : 2;
           if (inRange(lbb[b], lbb[b] + w, q[b]) && inRange(lbb[c], lbb[c] + w, q[c])) {
-            if (emit) { emit[3 * n] = q[0]; emit[3 * n + 1] = q[1]; emit[3 * n + 2] = q[2]; }
+            emit[3 * n] = q[0];
+            emit[3 * n + 1] = q[1];
+            emit[3 * n + 2] = q[2];
             ++n;
           }
         }
@@ -132,7 +197,7 @@ struct EdgeStep {
     if (!isUnique(slot)) return 0;
     const unsigned long long key = edgeKeyOf(F, slot);
     const uint32_t a = (uint32_t)(key >> 32), b = (uint32_t)(key & 0xffffffffu);
-    return (uint32_t)edgeHits(S, V + 3 * a, V + 3 * b, nullptr);
+    return (uint32_t)edgeHits(S, V + 3 * a, V + 3 * b, 0, nullptr);
   }
 };
 struct EdgeEmit {
@@ -142,7 +207,7 @@ struct EdgeEmit {
     if (!count) return;
     const unsigned long long key = edgeKeyOf(es.F, slot);
     const uint32_t a = (uint32_t)(key >> 32), b = (uint32_t)(key & 0xffffffffu);
-    edgeHits(es.S, es.V + 3 * a, es.V + 3 * b, out + 3 * (int64_t)prefix);
+    edgeHits(es.S, es.V + 3 * a, es.V + 3 * b, (int)count, out + 3 * (int64_t)prefix);
   }
 };
 
@@ -235,8 +300,19 @@ __device__ int faceHits(const SampleParams& S, const double* V, const int32_t* F
     const double c[3] = {te[1] * d[2] - te[2] * d[1], te[2] * d[0] - te[0] * d[2], te[0] * d[1] - te[1] * d[0]};
     return dot3(c, tn) >= 0;
   };
+  // The candidates are narrowed by the lattice positions themselves, which the edges' own (formed from
+  // their owner nodes) match to a few ulps (a million triangles of about a cell: 711 us a pass with every
+  // edge of the box looked up, 136 so): margins of a millionth of a cell and 1e-12 of the terms'
+  // sizes cover that and every rounding, as long as the coordinates are not huge against a cell.
+  const double w = S.w0;
+  double size = 0.0;
+  for (int a = 0; a < 3; ++a) size = dmax(size, dmax(fabs(org[a]) + w * S.res, dmax(fabs(lo[a]), fabs(hi[a]))));
+  const bool narrow = size <= 1e6 * w;
+  const double near = 1e-6 * w, terms = 1e-12 * (fabs(tdir) + (fabs(tn[0]) + fabs(tn[1]) + fabs(tn[2])) * size);
   int n = 0;
   for (int axis = 0; axis < 3; ++axis) {
+    // an edge along the axis: nd below is tn[axis] times its length
+    if (narrow && fabs(tn[axis]) * w < 0.9999e-9) continue;
     const uint32_t ord = axis == 2 ? 0u : (axis == 1 ? 1u : 2u);
     // Candidate fine edges along the axis. Along it: those whose span can meet the sweep window
     // [lo - 1e-9, hi + 1e-9] (start cells floor(lo) - 1 .. floor(hi) + 1). Across it: a hit is
@@ -250,9 +326,25 @@ __device__ int faceHits(const SampleParams& S, const double* V, const int32_t* F
       l1[a] = c1 > S.res ? S.res : c1;
     }
     if (l1[axis] > S.res - 1) l1[axis] = S.res - 1;  // edge start along its axis
+    if (narrow)
+      for (int a = 0; a < 3; ++a)
+        if (a != axis) {  // the lattice lines in [lo, hi] themselves
+          l0[a] = max(l0[a], (int)ceil((lo[a] - near - org[a]) / w));
+          l1[a] = min(l1[a], (int)floor((hi[a] + near - org[a]) / w));
+        }
+    const double inv = 1.0 / tn[axis], off = near + terms * fabs(inv);
     for (int X = l0[0]; X <= l1[0]; ++X)
       for (int Y = l0[1]; Y <= l1[1]; ++Y)
         for (int Z = l0[2]; Z <= l1[2]; ++Z) {
+          if (narrow) {  // where the line meets the triangle's plane: within this edge?
+            const double at[3] = {latticePos(org[0], w, (uint32_t)X), latticePos(org[1], w, (uint32_t)Y),
+                                  latticePos(org[2], w, (uint32_t)Z)};
+            double sum = tdir;
+            for (int a = 0; a < 3; ++a)
+              if (a != axis) sum = sum + tn[a] * at[a];
+            const double meet = -sum * inv - at[axis];
+            if (meet < -off || meet > w + off) continue;
+          }
           const uint32_t key = (((uint32_t)X * M + (uint32_t)Y) * M + (uint32_t)Z) * 3u + ord;
           const unsigned long long wbits = S.ebits[key >> 6];
           if (!((wbits >> (key & 63)) & 1ull)) continue;
