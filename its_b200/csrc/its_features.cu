@@ -102,10 +102,7 @@ __global__ void kFineSums(const uint32_t* __restrict__ sortedNode, const uint32_
 }
 
 // Nodes of one depth sum their 8 children (children 0..7 in order).
-__global__ void kParentSums(int64_t begin, int64_t count, const uint32_t* __restrict__ child0, NodeStats S) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const int64_t t = begin + i;
+__device__ __forceinline__ void parentSum(int64_t t, const uint32_t* __restrict__ child0, const NodeStats& S) {
   const uint32_t c0 = child0[t];
   float c = 0.0f;
   double p[3] = {0, 0, 0}, q[3] = {0, 0, 0};
@@ -125,29 +122,37 @@ __global__ void kParentSums(int64_t begin, int64_t count, const uint32_t* __rest
     S.sn[3 * t + a] = q[a];
   }
 }
+__global__ void kParentSums(int64_t begin, int64_t count, const uint32_t* __restrict__ child0, NodeStats S) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < count) parentSum(begin + i, child0, S);
+}
+// The levels first .. depth - 1, one after another, by one block: a launch per level of a few
+// hundred nodes costs more than its sums (up to 2,048 nodes in the one block: 35 us, its loads).
+constexpr int64_t kTopNodes = 256;
+constexpr int kTopThreads = 512;
+struct LevelRuns {
+  int first, depth;
+  int64_t start[kMaxDepth + 1];
+};
+__global__ void __launch_bounds__(kTopThreads) kParentSumsTop(LevelRuns R, const uint32_t* __restrict__ child0,
+                                                              NodeStats S) {
+  for (int L = R.first; L < R.depth; ++L) {
+    for (int64_t t = R.start[L] + threadIdx.x; t < R.start[L + 1]; t += kTopThreads) parentSum(t, child0, S);
+    __threadfence_block();
+    __syncthreads();
+  }
+}
 
 struct FeatParams {
   int depth, res;
   double w0;
   LatticeIndex lat[kMaxDepth];
-  int64_t vertStart[kMaxDepth + 1];
-  const uint32_t* vertLin;
   const uint64_t* vertKey;
   const uint32_t* vertOwner;
   const double* vertPos;
   const uint32_t* nodeNb;
 };
 
-__device__ __forceinline__ int vertDepth(const FeatParams& P, int64_t v) {
-  int d = 0;
-  while (d + 1 < P.depth && P.vertStart[d + 1] <= v) ++d;
-  return d;
-}
-__device__ __forceinline__ bool coincidentVertex(const FeatParams& P, int64_t v, int d) {
-  if (d + 1 >= P.depth) return false;
-  const uint32_t M = P.lat[d].M, lin = P.vertLin[v];
-  return (((lin / (M * M)) | ((lin / M) % M) | (lin % M)) & 1u) == 0u;
-}
 // Vertex index of lattice point (X,Y,Z) at depth d, or -1.
 template <class Params>
 __device__ __forceinline__ int64_t latticeVertex(const Params& P, int d, int64_t X, int64_t Y, int64_t Z) {
@@ -170,12 +175,6 @@ __device__ __forceinline__ int64_t latticeVertexIlp(const Params& P, int d, int6
   const uint32_t rank = L.rank[lin >> 6];
   if (!((word >> (lin & 63)) & 1ull)) return -1;
   return (int64_t)(L.base + rank + (uint32_t)__popcll(word & ((1ull << (lin & 63)) - 1ull)));
-}
-
-__global__ void kMarkCoincident(const __grid_constant__ FeatParams P, int64_t n, uint32_t* __restrict__ flag) {
-  const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (v >= n) return;
-  flag[v] = coincidentVertex(P, v, vertDepth(P, v)) ? 1u : 0u;
 }
 
 // Feature normalisation (mean[64], scale[64]) passed by value with the launch.
@@ -383,8 +382,6 @@ static FeatParams featParams(const SvoDevice& d) {
   P.res = d.res;
   P.w0 = d.unit[0];
   for (int L = 0; L < kMaxDepth; ++L) P.lat[L] = L < d.depth ? d.lattice(L) : LatticeIndex{};
-  for (int L = 0; L <= kMaxDepth; ++L) P.vertStart[L] = L <= d.depth ? d.vertStart[L] : d.numVerts;
-  P.vertLin = d.vertLin;
   P.vertKey = d.vertKey;
   P.vertOwner = d.vertOwner;
   P.vertPos = d.vertPos;
@@ -396,19 +393,23 @@ static FeatParams featParams(const SvoDevice& d) {
 its_status coincidentIds(its_ctx* ctx, const SvoDevice& d, int64_t* ids, int64_t* count) {
   const int64_t n = d.numVerts;
   its_status st;
-  DevBuf<uint32_t> flag;
-  DevBuf<int64_t> tot;
-  if ((st = flag.alloc(ctx, n)) != ITS_OK || (st = tot.alloc(ctx, 1)) != ITS_OK) return st;
-  const FeatParams P = featParams(d);
-  kMarkCoincident<<<gridFor(n, 256), 256, 0, ctx->stream>>>(P, n, flag.p);
-  ITS_LAUNCHED(ctx);
-  const uint32_t* fl = flag.p;
-  auto fv = [fl] __device__(int64_t i) -> int64_t { return (int64_t)fl[i]; };
-  auto wr = [fl, ids] __device__(int64_t i, int64_t prefix, int64_t) {
-    if (fl[i]) ids[prefix] = i;
+  DevBuf<uint32_t> tot;
+  if ((st = tot.alloc(ctx, 1)) != ITS_OK) return st;
+  // below the root depth with all-even lattice coordinates (bits 0, 11 and 22 of the key)
+  const uint64_t* key = d.vertKey;
+  const int depth = d.depth;
+  auto is = [key, depth] __device__(int64_t i) -> uint32_t {
+    const uint64_t k = key[i];
+    return (int)((k >> 33) & 15u) + 1 < depth && !((k | (k >> 11) | (k >> 22)) & 1u) ? 1u : 0u;
   };
-  if ((st = scanExclusiveAlloc<int64_t>(ctx, fv, n, wr, tot.p)) != ITS_OK) return st;
-  return readScalar(ctx, tot.p, count);
+  auto wr = [ids] __device__(int64_t i, uint32_t prefix, uint32_t v) {
+    if (v) ids[prefix] = i;
+  };
+  if ((st = scanExclusiveAlloc<uint32_t>(ctx, is, n, wr, tot.p)) != ITS_OK) return st;
+  uint32_t c = 0;
+  if ((st = readScalar(ctx, tot.p, &c)) != ITS_OK) return st;
+  *count = c;
+  return ITS_OK;
 }
 
 // Features 38-45 of coincident vertex i (one thread each): the samples of the 27 nodes around
@@ -490,13 +491,19 @@ its_status nodeSampleStats(its_ctx* ctx, SvoDevice& d, const double* V, const in
   NodeStats S{d.nodeSampleCnt, d.nodeSamplePos, d.nodeSampleNrm};
   kFineSums<<<gridFor(nf, 256), 256, 0, ctx->stream>>>(sNode.p, sId.p, nf, fineCount, cent.p, nrm.p, S);
   ITS_LAUNCHED(ctx);
-  for (int L = 1; L < d.depth; ++L) {
-    if (!d.levelCount[L]) continue;
+  // large levels in a launch each, the rest, up to the root, in one block
+  int L = 1;
+  for (; L < d.depth && d.levelCount[L] > kTopNodes; ++L) {
     kParentSums<<<gridFor(d.levelCount[L], 256), 256, 0, ctx->stream>>>(d.levelStart[L], d.levelCount[L],
                                                                         d.nodeChild0, S);
     ITS_LAUNCHED(ctx);
   }
-  ITS_CU(ctx, cudaStreamSynchronize(ctx->stream));  // the sample scratch is freed on return
+  if (L < d.depth) {
+    LevelRuns R{L, d.depth, {}};
+    for (int k = L; k <= d.depth; ++k) R.start[k] = d.levelStart[k];
+    kParentSumsTop<<<1, kTopThreads, 0, ctx->stream>>>(R, d.nodeChild0, S);
+    ITS_LAUNCHED(ctx);
+  }
   return ITS_OK;
 }
 

@@ -102,7 +102,7 @@ struct LatticeIndex {
   const unsigned long long* bits;  // M^3 bits
   const uint32_t* rank;            // exclusive popcount prefix per 64-bit word
   uint32_t M;
-  uint32_t base;                   // global index of the depth's first vertex
+  uint32_t base;                   // added to the ranks (0 where they are global vertex indices)
 };
 __device__ __forceinline__ bool latticeHas(const LatticeIndex& L, uint32_t lin) {
   return (L.bits[lin >> 6] >> (lin & 63)) & 1ull;
@@ -144,12 +144,14 @@ struct SvoDevice {
   int64_t numVoxels = 0, numNodes = 0, numVerts = 0, numEdges = 0;
   int64_t levelCount[kMaxDepth] = {0}, levelStart[kMaxDepth + 1] = {0};
   int64_t vertCount[kMaxDepth] = {0}, vertStart[kMaxDepth + 1] = {0};
-  uint32_t* voxels = nullptr;      // surface voxels, ascending Morton
+  uint32_t* voxels = nullptr;      // surface voxels, ascending Morton; the coarser levels' cells follow
   uint32_t* nodeMorton = nullptr;
   uint32_t* nodeParent = nullptr;
   uint32_t* nodeChild0 = nullptr;  // first of 8 consecutive children, kNone for leaves
   uint8_t* nodeLeaf = nullptr;
   uint32_t* nodeNb = nullptr;      // 27 per node, slot (dx+1)+3(dy+1)+9(dz+1)
+  // corner lattices, every depth's words one after another (vbits[0] and vrank[0] own the memory);
+  // the ranks run on over the depths, so they are global vertex indices
   unsigned long long* vbits[kMaxDepth] = {nullptr};
   uint32_t* vrank[kMaxDepth] = {nullptr};
   uint32_t* vertLin = nullptr;     // lattice index within its depth
@@ -179,7 +181,7 @@ struct SvoDevice {
     L.bits = vbits[d];
     L.rank = vrank[d];
     L.M = (uint32_t)(res >> d) + 1u;
-    L.base = (uint32_t)vertStart[d];
+    L.base = 0;
     return L;
   }
 };

@@ -172,6 +172,33 @@ its_status scanSpine(its_ctx* ctx, T* sums, int64_t nb, T* total, T* tops) {
   return ITS_OK;
 }
 
+// Short scans in one launch: one block takes the tiles in turn.
+constexpr int64_t kScanOneBlock = 4 * kScanTile;
+template <typename T, typename F, typename W>
+__global__ void __launch_bounds__(kScanThreads) kScanSmall(F f, int64_t n, W write, T* total) {
+  T carry = 0;
+  for (int64_t i0 = 0; i0 < n; i0 += kScanTile) {
+    const int64_t base = i0 + (int64_t)threadIdx.x * kScanItems;
+    T v[kScanItems];
+    T s = 0;
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j) {
+      v[j] = (base + j < n) ? f(base + j) : T(0);
+      s += v[j];
+    }
+    T tot;
+    T run = carry + blockExclusiveScan<T>(s, tot);
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j)
+      if (base + j < n) {
+        write(base + j, run, v[j]);
+        run += v[j];
+      }
+    carry += tot;
+  }
+  if (threadIdx.x == 0 && total) *total = carry;
+}
+
 // Exclusive scan of f(0..n-1); write(i, prefix, value) receives each element's prefix.
 // The total lands in *dTotal (device memory, may be NULL). scratch must hold
 // scanScratchSize(n) elements of T (the block sums, then the spine's tile totals).
@@ -184,6 +211,11 @@ template <typename T, typename F, typename W>
 its_status scanExclusive(its_ctx* ctx, F f, int64_t n, W write, T* dTotal, T* scratch) {
   if (n <= 0) {
     if (dTotal) ITS_CU(ctx, cudaMemsetAsync(dTotal, 0, sizeof(T), ctx->stream));
+    return ITS_OK;
+  }
+  if (n <= kScanOneBlock) {
+    kScanSmall<T, F, W><<<1, kScanThreads, 0, ctx->stream>>>(f, n, write, dTotal);
+    ITS_LAUNCHED(ctx);
     return ITS_OK;
   }
   const int64_t nb = scanBlocks(n);

@@ -5,8 +5,8 @@
 // reference's svoNodeArray):
 //   * occupancy of the res^3 voxel grid is a Morton-indexed bitset (res^3/8 bytes) instead
 //     of a dense uint32 array; surface voxels are compacted from it in Morton order;
-//   * each level's occupied codes O_L are sorted, so the next level is unique(O_L >> 3):
-//     no dense per-level arrays and no sort;
+//   * so is every coarser level's, and one scan ranks all levels' cells: no dense per-level arrays,
+//     no sort, and parent, children and neighbours by bit tests and ranks;
 //   * nodes: morton / parent / first-child / leaf flag / 27 neighbours;
 //   * per-depth corner vertices are a bitmap over the (res_d+1)^3 corner lattice with a
 //     popcount rank per 64-bit word, which gives the reference's sorted (x,y,z) vertex order
@@ -96,121 +96,205 @@ __global__ void kVoxelize(const double* __restrict__ V, const int32_t* __restric
   }
 }
 
-// ---- level build ---------------------------------------------------------------------------
-__global__ void kFillGroups(int64_t G, const uint32_t* __restrict__ next, uint32_t* morton, uint32_t* parent,
-                            uint32_t* child0, uint8_t* leaf, int64_t start) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;  // node within the level
-  if (i >= 8 * G) return;
-  const int64_t g = i >> 3;
-  morton[start + i] = (next[g] << 3) | (uint32_t)(i & 7);
-  parent[start + i] = kNone;
-  child0[start + i] = kNone;
-  leaf[start + i] = 1;
-}
-// Occupied nodes of level L >= 1 (createNode_2, SVO.cu:596-638): not leaves, children are the
-// i-th sibling group of level L-1, which point back at them.
-__global__ void kFillOccupied(int64_t c, const uint32_t* __restrict__ O, const uint32_t* __restrict__ grp,
-                              int64_t start, int64_t childStart, uint32_t* parent, uint32_t* child0,
-                              uint8_t* leaf) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= c) return;
-  const uint32_t node = (uint32_t)(start + 8 * (int64_t)grp[i] + (O[i] & 7u));
-  leaf[node] = 0;
-  child0[node] = (uint32_t)(childStart + 8 * i);
+// Which of n consecutive runs i lies in.
+__device__ __forceinline__ int levelOf(const int64_t* start, int n, int64_t i) {
+  int L = 0;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) parent[childStart + 8 * i + k] = node;
-}
-__global__ void kFillRoot(uint32_t O0, int64_t start, int64_t childStart, int hasChildren, uint32_t* morton,
-                          uint32_t* parent, uint32_t* child0, uint8_t* leaf, uint32_t* nb) {
-  const int k = threadIdx.x;
-  if (k == 0) {
-    morton[start] = O0;
-    parent[start] = kNone;
-    child0[start] = hasChildren ? (uint32_t)childStart : kNone;
-    leaf[start] = hasChildren ? 0 : 1;
-  }
-  if (k < 27) nb[start * 27 + k] = (k == 13) ? (uint32_t)start : kNone;
-  if (hasChildren && k < 8) parent[childStart + k] = (uint32_t)start;
+  for (int k = 1; k < kMaxDepth; ++k) L += k < n && i >= start[k] ? 1 : 0;
+  return L;
 }
 
-// 27-neighbours top-down (findNeighbors, SVO.cu:861-890): the neighbour at offset d of the
-// child with key k is child ((k+d) mod 2) of the parent's neighbour floor((k+d)/2).
-__global__ void kNeighbors(int64_t count, int64_t start, const uint32_t* __restrict__ morton,
-                           const uint32_t* __restrict__ parent, const uint32_t* __restrict__ child0,
-                           uint32_t* nb) {
-  const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (idx >= count * 27) return;
-  const int64_t t = start + idx / 27;
-  const int s = (int)(idx % 27);
-  const uint32_t key = morton[t] & 7u;
-  const int d[3] = {s % 3 - 1, (s / 3) % 3 - 1, s / 9 - 1};
-  int P[3], C = 0;
+// ---- level build ---------------------------------------------------------------------------
+// The occupancy of every level as Morton bitsets, the voxels' words first and each coarser level's
+// after them (a cell is occupied when one of its eight children is). One scan over all the words
+// ranks every level's cells at once, so that a node's parent, children and neighbours are a bit
+// test and a rank away, for all levels in one launch each; only the levels' counts go to the host.
+// (Level by level -- a scan, a read of its count and three fills each, then the neighbours from
+// the top down -- an octree of 6 levels took 110 launches and 13 waits.)
+struct Pyramid {
+  int levels;  // log2(res) + 1
+  int64_t word[kMaxDepth + 1];  // first word of each level
+  const unsigned long long* bits;
+  const uint32_t* rank;  // over all words
+  __device__ __forceinline__ bool has(int L, uint32_t code) const {
+    return (bits[word[L] + (code >> 6)] >> (code & 63)) & 1ull;
+  }
+  __device__ __forceinline__ uint32_t rankOf(int L, uint32_t code) const {  // cells of finer levels included
+    const int64_t w = word[L] + (code >> 6);
+    return rank[w] + (uint32_t)__popcll(bits[w] & ((1ull << (code & 63)) - 1ull));
+  }
+};
+// Bit i of the result: byte i of the word is not 0.
+__device__ __forceinline__ uint32_t bytesSet(unsigned long long w) {
+  w |= w >> 4;
+  w |= w >> 2;
+  w |= w >> 1;
+  w &= 0x0101010101010101ull;
+  return (uint32_t)((w * 0x0102040810204080ull) >> 56);
+}
+// Levels first + 1 .. first + 3 from level first (as many as there are): a block takes 512 of its
+// words, 64 of the next level's, 8, 1. A block alone with its level goes on to the top.
+constexpr int kPyrThreads = 64;
+__global__ void __launch_bounds__(kPyrThreads) kPyramid(unsigned long long* __restrict__ bits,
+                                                        const __grid_constant__ Pyramid P, int first) {
+  __shared__ unsigned long long s[2][kPyrThreads];
+  int64_t from = (int64_t)blockIdx.x * 512;  // the block's first word of the current level
+  const int t = threadIdx.x;
+  for (int L = first; L + 1 < P.levels && (L < first + 3 || gridDim.x == 1); ++L) {
+    const int64_t words = P.word[L + 1] - P.word[L], next = P.word[L + 2] - P.word[L + 1], to = from / 8;
+    const unsigned long long* prev = s[(L - first + 1) & 1];
+    const int outs = L == first ? 64 : (L == first + 1 ? 8 : 1);  // the block's words of level L + 1
+    unsigned long long w = 0;
+    if (t < outs) {
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    const int tt = (int)((key >> a) & 1u) + d[a];
-    P[a] = tt < 0 ? -1 : (tt > 1 ? 1 : 0);
-    C |= (tt & 1) << a;
+      for (int k = 0; k < 8; ++k) {
+        const int64_t i = from + 8 * t + k;
+        const unsigned long long v = i >= words ? 0ull : (L == first ? bits[P.word[L] + i] : prev[8 * t + k]);
+        w |= (unsigned long long)bytesSet(v) << (8 * k);
+      }
+    }
+    s[(L - first) & 1][t] = w;
+    if (t < outs && to + t < next) bits[P.word[L + 1] + to + t] = w;
+    __syncthreads();
+    from = to;
   }
-  const uint32_t p = parent[t];
-  const uint32_t pn = nb[(int64_t)p * 27 + (P[0] + 1) + 3 * (P[1] + 1) + 9 * (P[2] + 1)];
+}
+// Every level's cells in Morton order, the voxels first.
+__global__ void kEmitCells(const __grid_constant__ Pyramid P, int64_t words, uint32_t* __restrict__ cells) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= words) return;
+  unsigned long long w = P.bits[i];
+  if (!w) return;
+  const uint32_t first = (uint32_t)((i - P.word[levelOf(P.word, P.levels, i)]) * 64);
+  uint32_t r = P.rank[i];
+  while (w) {
+    cells[r++] = first + (uint32_t)(__ffsll((long long)w) - 1);
+    w &= w - 1;
+  }
+}
+// out[k] = the rank at word at[k]
+struct Bounds {
+  int n;
+  int64_t at[2 * kMaxDepth];
+};
+__global__ void kRanksAt(const uint32_t* __restrict__ rank, Bounds B, uint32_t* __restrict__ out) {
+  if ((int)threadIdx.x < B.n) out[threadIdx.x] = rank[B.at[threadIdx.x]];
+}
+
+// The octree's levels as the kernels below see them.
+struct Levels {
+  int depth, res;
+  int64_t node[kMaxDepth + 1];  // first node of each depth
+  int64_t cell[kMaxDepth + 1];  // first of the level's cells among all levels' cells
+  int64_t vert[kMaxDepth + 1];  // first vertex of each depth
+  int64_t vword[kMaxDepth + 1]; // first word of each depth's corner lattice
+};
+// Nodes (createNode_1/2, SVO.cu:560-638): the eight children of every cell of the level above.
+__global__ void kNodes(const __grid_constant__ Pyramid P, const __grid_constant__ Levels V,
+                       const uint32_t* __restrict__ cells, uint32_t* __restrict__ morton, uint32_t* __restrict__ parent,
+                       uint32_t* __restrict__ child0, uint8_t* __restrict__ leaf) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= V.node[V.depth]) return;
+  const int top = V.depth - 1, L = levelOf(V.node, V.depth, t);
+  if (L == top) {  // the root
+    morton[t] = cells[V.cell[top]];
+    parent[t] = kNone;
+    child0[t] = top > 0 ? (uint32_t)V.node[top - 1] : kNone;
+    leaf[t] = top > 0 ? 0 : 1;
+    return;
+  }
+  const int64_t i = t - V.node[L];
+  const uint32_t up = cells[V.cell[L + 1] + (i >> 3)], code = (up << 3) | (uint32_t)(i & 7);
+  morton[t] = code;
+  parent[t] = L + 1 == top ? (uint32_t)V.node[top]
+                           : (uint32_t)(V.node[L + 1] + 8 * (int64_t)(P.rankOf(L + 2, up >> 3) - V.cell[L + 2]) +
+                                        (up & 7u));
+  const bool inner = L > 0 && P.has(L, code);
+  child0[t] = inner ? (uint32_t)(V.node[L - 1] + 8 * (int64_t)(P.rankOf(L, code) - V.cell[L])) : kNone;
+  leaf[t] = inner ? 0 : 1;
+}
+
+// 27-neighbours (findNeighbors, SVO.cu:861-890): the node at offset d of the same depth, which exists
+// when its parent cell is occupied.
+__global__ void kNeighbors(const __grid_constant__ Pyramid P, const __grid_constant__ Levels V,
+                           const uint32_t* __restrict__ morton, uint32_t* __restrict__ nb) {
+  const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (idx >= V.node[V.depth] * 27) return;
+  const int64_t t = idx / 27;
+  const int s = (int)(idx - 27 * t), L = levelOf(V.node, V.depth, t);
   uint32_t r = kNone;
-  if (pn != kNone) {
-    const uint32_t c0 = child0[pn];
-    if (c0 != kNone) r = c0 + (uint32_t)C;
+  if (L == V.depth - 1) {
+    if (s == 13) r = (uint32_t)t;
+  } else {
+    uint32_t X, Y, Z;
+    mortonDecode(morton[t], X, Y, Z);
+    const int x = (int)X + s % 3 - 1, y = (int)Y + (s / 3) % 3 - 1, z = (int)Z + s / 9 - 1, side = V.res >> L;
+    if (x >= 0 && y >= 0 && z >= 0 && x < side && y < side && z < side) {
+      const uint32_t m = mortonEncode((uint32_t)x, (uint32_t)y, (uint32_t)z);
+      if (P.has(L + 1, m >> 3))
+        r = (uint32_t)(V.node[L] + 8 * (int64_t)(P.rankOf(L + 1, m >> 3) - V.cell[L + 1]) + (m & 7u));
+    }
   }
-  nb[t * 27 + s] = r;
+  nb[idx] = r;
 }
 
 // ---- corner vertices (determineNodeVertex + sort + unique, SVO.cu:913-963, 1064-1096) -------
-__global__ void kMarkCorners(int64_t count, int64_t start, const uint32_t* __restrict__ morton, uint32_t M,
-                             unsigned long long* bits) {
-  const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (idx >= count * 8) return;
-  const int64_t t = start + (idx >> 3);
-  const int k = (int)(idx & 7);
+// All depths in one launch each.
+__device__ __forceinline__ int64_t cornerBit(const Levels& V, int64_t idx, const uint32_t* __restrict__ morton) {
+  const int64_t t = idx >> 3;
+  const int k = (int)(idx & 7), L = levelOf(V.node, V.depth, t);
+  const uint32_t M = (uint32_t)(V.res >> L) + 1u;
   uint32_t X, Y, Z;
   mortonDecode(morton[t], X, Y, Z);
-  const uint32_t lin = ((X + (k & 1)) * M + (Y + ((k >> 1) & 1))) * M + (Z + ((k >> 2) & 1));
-  atomicOr(bits + (lin >> 6), 1ull << (lin & 63));
+  return V.vword[L] * 64 + ((X + (k & 1)) * M + (Y + ((k >> 1) & 1))) * M + (Z + ((k >> 2) & 1));
 }
+__global__ void kMarkCorners(const __grid_constant__ Levels V, const uint32_t* __restrict__ morton,
+                             unsigned long long* bits) {
+  const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (idx >= V.node[V.depth] * 8) return;
+  const int64_t b = cornerBit(V, idx, morton);
+  atomicOr(bits + (b >> 6), 1ull << (b & 63));
+}
+// The set bits' indices (of vertices within their depth's lattice) in order, their owners to come.
 __global__ void kEmitBits(int64_t words, const unsigned long long* __restrict__ bits,
-                          const uint32_t* __restrict__ rank, uint32_t* __restrict__ out) {
+                          const uint32_t* __restrict__ rank, uint32_t* __restrict__ out, uint32_t* __restrict__ owner) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= words) return;
   unsigned long long w = bits[i];
+  if (!w) return;
   uint32_t r = rank[i];
   while (w) {
     const int b = __ffsll((long long)w) - 1;
+    if (owner) owner[r] = kNone;
     out[r++] = (uint32_t)(i * 64 + b);
     w &= w - 1;
   }
 }
-__global__ void kOwnerCorners(int64_t count, int64_t start, const uint32_t* __restrict__ morton, LatticeIndex L,
+__global__ void kOwnerCorners(const __grid_constant__ Levels V, const uint32_t* __restrict__ morton,
+                              const unsigned long long* __restrict__ bits, const uint32_t* __restrict__ rank,
                               uint32_t* owner) {
   const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (idx >= count * 8) return;
-  const int64_t t = start + (idx >> 3);
-  const int k = (int)(idx & 7);
-  uint32_t X, Y, Z;
-  mortonDecode(morton[t], X, Y, Z);
-  const uint32_t lin = ((X + (k & 1)) * L.M + (Y + ((k >> 1) & 1))) * L.M + (Z + ((k >> 2) & 1));
-  atomicMin(owner + latticeRank(L, lin), (uint32_t)t);
+  if (idx >= V.node[V.depth] * 8) return;
+  const int64_t b = cornerBit(V, idx, morton);
+  const uint32_t v = rank[b >> 6] + (uint32_t)__popcll(bits[b >> 6] & ((1ull << (b & 63)) - 1ull));
+  atomicMin(owner + v, (uint32_t)(idx >> 3));
 }
 // Representative position of a corner: taken from its owner node, corner = origin (+ w),
 // origin = g + w*X (the surviving entry of the reference's stable sort + unique).
 // Also the vertex's packed key (lattice coordinates, depth, corner of the owner).
-__global__ void kVertexPositions(int64_t count, int64_t vstart, uint32_t M, int depth, double3 g, double w,
-                                 const uint32_t* __restrict__ lin, const uint32_t* __restrict__ owner,
-                                 const uint32_t* __restrict__ morton, double* __restrict__ pos,
-                                 uint64_t* __restrict__ key) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const int64_t v = vstart + i;
-  const uint32_t l = lin[v];
+__global__ void kVertexPositions(const __grid_constant__ Levels V, double3 g, double w0, uint32_t* __restrict__ lin,
+                                 const uint32_t* __restrict__ owner, const uint32_t* __restrict__ morton,
+                                 double* __restrict__ pos, uint64_t* __restrict__ key) {
+  const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (v >= V.vert[V.depth]) return;
+  const int L = levelOf(V.vert, V.depth, v);
+  const uint32_t M = (uint32_t)(V.res >> L) + 1u, l = lin[v] - (uint32_t)(V.vword[L] * 64);
+  const double w = w0 * (double)(1u << L);
+  lin[v] = l;
   const uint32_t X = l / (M * M), Y = (l / M) % M, Z = l % M;
   uint32_t Xo, Yo, Zo;
   mortonDecode(morton[owner[v]], Xo, Yo, Zo);
-  key[v] = encodeVertKey(X, Y, Z, depth, Xo, Yo, Zo);
+  key[v] = encodeVertKey(X, Y, Z, L, Xo, Yo, Zo);
   const double bx = latticePos(g.x, w, Xo), by = latticePos(g.y, w, Yo), bz = latticePos(g.z, w, Zo);
   pos[3 * v] = (X != Xo) ? bx + w : bx;
   pos[3 * v + 1] = (Y != Yo) ? by + w : by;
@@ -254,11 +338,25 @@ __global__ void kOwnerEdges(int64_t count, const uint32_t* __restrict__ morton, 
   const uint32_t r = rank[key >> 6] + (uint32_t)__popcll(w & ((1ull << (key & 63)) - 1ull));
   atomicMin(owner + r, (uint32_t)t);
 }
-__global__ void kMarkFine(int64_t count, const uint32_t* __restrict__ morton, unsigned long long* occ) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= count) return;
-  const uint32_t m = morton[t];
-  atomicOr(occ + (m >> 6), 1ull << (m & 63));
+// The depth-0 nodes as a Morton bitset with its ranks: the eight children of every cell of level 1 (of
+// a lone root: itself).
+__global__ void kFineNodes(const __grid_constant__ Pyramid P, const __grid_constant__ Levels V, int64_t words,
+                           unsigned long long* __restrict__ occ, uint32_t* __restrict__ rank) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= words) return;
+  if (V.depth == 1) {
+    occ[i] = P.bits[i];
+    rank[i] = P.rank[i];
+    return;
+  }
+  const int64_t at = P.word[1] + (i >> 3);
+  const int shift = 8 * (int)(i & 7);
+  const unsigned long long up = P.bits[at];
+  unsigned long long b = (up >> shift) & 0xffull;  // bit j: the j-th byte of the word is full
+  b = (b * 0x0101010101010101ull) & 0x8040201008040201ull;
+  b = ((b + 0x7f7f7f7f7f7f7f7full) | b) & 0x8080808080808080ull;  // byte j's top bit
+  occ[i] = (b >> 7) * 0xffull;
+  rank[i] = 8u * (P.rank[at] + (uint32_t)__popcll(up & ((1ull << shift) - 1ull)) - (uint32_t)V.cell[1]);
 }
 
 // ---- getters -------------------------------------------------------------------------------------
@@ -317,7 +415,8 @@ static void svoRelease(its_svo* s) {
                   d.vertOwner, d.vertPos, d.ebits, d.erank, d.edgeKey, d.edgeOwner, d.fineOcc, d.fineRank,
                   d.nodeSampleCnt, d.nodeSamplePos, d.nodeSampleNrm, d.coincIds, d.rowParams, d.coincGeom};
   for (void* p : ptrs) devFree(c, p);
-  for (int i = 0; i < kMaxDepth; ++i) { devFree(c, d.vbits[i]); devFree(c, d.vrank[i]); }
+  devFree(c, d.vbits[0]);
+  devFree(c, d.vrank[0]);
   d = SvoDevice();
 }
 
@@ -331,8 +430,6 @@ its_status svoBuild(its_ctx* ctx, const double* dV, int64_t nv, const int32_t* d
   for (int a = 0; a < 3; ++a) { d.origin[a] = origin[a]; d.unit[a] = width[a] / res; }
   const double3 g = make_double3(origin[0], origin[1], origin[2]);
   const double3 u = make_double3(d.unit[0], d.unit[1], d.unit[2]);
-  const int64_t gridBits = (int64_t)res * res * res;
-  const int64_t gridWords = (gridBits + 63) / 64;
   its_status st;
   // device time of the build and of the learned fit's tables (reported by its_svo_get_info)
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
@@ -343,193 +440,151 @@ its_status svoBuild(its_ctx* ctx, const double* dV, int64_t nv, const int32_t* d
   } evFree{ev};
   ITS_CU(ctx, cudaEventRecord(ev[0], ctx->stream));
 
-  // 1. voxelise into the Morton bitset
-  DevBuf<unsigned long long> occ;
-  if ((st = occ.zeros(ctx, gridWords)) != ITS_OK) return st;
+  // 1. voxelise into the finest level of the occupancy pyramid, then the coarser levels
+  Pyramid P{};
+  P.levels = 1;
+  while ((res >> P.levels) > 0) ++P.levels;
+  for (int L = 0; L < P.levels; ++L) {
+    const int64_t side = res >> L;
+    P.word[L + 1] = P.word[L] + (side * side * side + 63) / 64;
+  }
+  const int64_t pyrWords = P.word[P.levels];
+  DevBuf<unsigned long long> pyr;
+  DevBuf<uint32_t> pyrRank, counts;
+  if ((st = pyr.zeros(ctx, pyrWords)) != ITS_OK || (st = pyrRank.alloc(ctx, pyrWords)) != ITS_OK ||
+      (st = counts.alloc(ctx, 2 * kMaxDepth)) != ITS_OK)
+    return st;
+  P.bits = pyr.p;
+  P.rank = pyrRank.p;
   if (nf > 0) {
     const int block = 128;
     const unsigned grid = (unsigned)std::min<int64_t>(gridFor(nf, block), (int64_t)ctx->numSMs * 64);
-    kVoxelize<<<grid, block, 0, ctx->stream>>>(dV, dF, nf, res, g, u, occ.p);
+    kVoxelize<<<grid, block, 0, ctx->stream>>>(dV, dF, nf, res, g, u, pyr.p);
     ITS_LAUNCHED(ctx);
   }
-  // 2. compact to the sorted list of surface voxels
-  DevBuf<uint32_t> dCount;
-  if ((st = dCount.alloc(ctx, 1)) != ITS_OK) return st;
+  for (int L = 0; L + 1 < P.levels; L += 3) {
+    const unsigned blocks = (unsigned)((P.word[L + 1] - P.word[L] + 511) / 512);
+    kPyramid<<<blocks, kPyrThreads, 0, ctx->stream>>>(pyr.p, P, L);
+    ITS_LAUNCHED(ctx);
+    if (blocks == 1) break;
+  }
+  // 2. ranks and counts of every level's cells; the root's level is the first with one cell
+  uint32_t host[2 * kMaxDepth];
+  auto popc = [](const unsigned long long* bits) {
+    return [bits] __device__(int64_t i) -> uint32_t { return (uint32_t)__popcll(bits[i]); };
+  };
   {
-    const unsigned long long* bits = occ.p;
-    auto f = [bits] __device__(int64_t i) -> uint32_t { return (uint32_t)__popcll(bits[i]); };
-    DevBuf<uint32_t> wordRank;
-    if ((st = wordRank.alloc(ctx, gridWords)) != ITS_OK) return st;
-    uint32_t* wr = wordRank.p;
-    if ((st = scanExclusiveAlloc<uint32_t>(ctx, f, gridWords, StorePrefix<uint32_t>{wr}, dCount.p)) != ITS_OK) return st;
-    uint32_t nvox = 0;
-    if ((st = readScalar(ctx, dCount.p, &nvox)) != ITS_OK) return st;
-    d.numVoxels = nvox;
-    if (nvox == 0) return setError(ctx, ITS_ERR_INVALID, "no surface voxel: the mesh does not meet the grid");
-    if ((st = devAlloc(ctx, (void**)&d.voxels, nvox * sizeof(uint32_t))) != ITS_OK) return st;
-    kEmitBits<<<gridFor(gridWords, 256), 256, 0, ctx->stream>>>(gridWords, occ.p, wr, d.voxels);
+    if ((st = scanExclusiveAlloc<uint32_t>(ctx, popc(pyr.p), pyrWords, StorePrefix<uint32_t>{pyrRank.p},
+                                           counts.p + P.levels - 1)) != ITS_OK)
+      return st;
+    Bounds B{P.levels - 1, {}};
+    for (int L = 0; L + 1 < P.levels; ++L) B.at[L] = P.word[L + 1];
+    kRanksAt<<<1, 32, 0, ctx->stream>>>(pyrRank.p, B, counts.p);
     ITS_LAUNCHED(ctx);
+    ITS_CU(ctx, cudaMemcpyAsync(host, counts.p, P.levels * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    ITS_CU(ctx, cudaStreamSynchronize(ctx->stream));
   }
-  occ.reset();
-
-  // 3. levels: O_{L+1} = unique(O_L >> 3); group index of every element
-  std::vector<DevBuf<uint32_t>> O, grp;  // levels >= 1 and per-level group indices
-  std::vector<int64_t> cnt;
-  const uint32_t* cur = d.voxels;
-  int64_t c = d.numVoxels;
-  std::vector<const uint32_t*> Optr;
-  Optr.push_back(cur);
-  cnt.push_back(c);
-  while (c > 1) {
-    if ((int)cnt.size() >= kMaxDepth) return setError(ctx, ITS_ERR_INVALID, "octree deeper than supported");
-    DevBuf<uint32_t> g1(ctx), nx(ctx);
-    if ((st = g1.alloc(ctx, c)) != ITS_OK) return st;
-    if ((st = nx.alloc(ctx, c)) != ITS_OK) return st;
-    const uint32_t* Oc = cur;
-    uint32_t* gp = g1.p;
-    uint32_t* np = nx.p;
-    auto head = [Oc] __device__(int64_t i) -> uint32_t { return (i == 0 || (Oc[i] >> 3) != (Oc[i - 1] >> 3)) ? 1u : 0u; };
-    auto wr = [Oc, gp, np] __device__(int64_t i, uint32_t prefix, uint32_t v) {
-      gp[i] = prefix + v - 1u;
-      if (v) np[prefix] = Oc[i] >> 3;
-    };
-    if ((st = scanExclusiveAlloc<uint32_t>(ctx, head, c, wr, dCount.p)) != ITS_OK) return st;
-    uint32_t G = 0;
-    if ((st = readScalar(ctx, dCount.p, &G)) != ITS_OK) return st;
-    grp.push_back(std::move(g1));
-    O.push_back(std::move(nx));
-    cur = O.back().p;
-    Optr.push_back(cur);
-    c = G;
-    cnt.push_back(c);
-  }
-  const int top = (int)cnt.size() - 1;  // root level
-  d.depth = top + 1;
+  d.numVoxels = host[0];
+  if (d.numVoxels == 0) return setError(ctx, ITS_ERR_INVALID, "no surface voxel: the mesh does not meet the grid");
+  Levels V{};
+  V.res = res;
+  for (int L = 0; L < P.levels; ++L) V.cell[L + 1] = host[L];
+  int top = 0;  // root level
+  while (V.cell[top + 1] - V.cell[top] > 1) ++top;
+  d.depth = V.depth = top + 1;
   int64_t total = 0;
   for (int L = 0; L <= top; ++L) {
     d.levelStart[L] = total;
-    d.levelCount[L] = (L < top) ? 8 * cnt[L + 1] : 1;
+    d.levelCount[L] = (L < top) ? 8 * (V.cell[L + 2] - V.cell[L + 1]) : 1;
     total += d.levelCount[L];
   }
   d.levelStart[top + 1] = total;
   d.numNodes = total;
+  for (int L = 0; L <= d.depth; ++L) V.node[L] = d.levelStart[L];
+  // every level's cells in Morton order, the surface voxels first
+  const int64_t cells = V.cell[P.levels];
+  if ((st = devAlloc(ctx, (void**)&d.voxels, cells * sizeof(uint32_t))) != ITS_OK) return st;
+  kEmitCells<<<gridFor(pyrWords, 256), 256, 0, ctx->stream>>>(P, pyrWords, d.voxels);
+  ITS_LAUNCHED(ctx);
+  // 3. nodes and their 27 neighbours
   if ((st = devAlloc(ctx, (void**)&d.nodeMorton, total * 4)) != ITS_OK) return st;
   if ((st = devAlloc(ctx, (void**)&d.nodeParent, total * 4)) != ITS_OK) return st;
   if ((st = devAlloc(ctx, (void**)&d.nodeChild0, total * 4)) != ITS_OK) return st;
   if ((st = devAlloc(ctx, (void**)&d.nodeLeaf, total)) != ITS_OK) return st;
   if ((st = devAlloc(ctx, (void**)&d.nodeNb, total * 27 * 4)) != ITS_OK) return st;
-  for (int L = 0; L < top; ++L) {
-    const int64_t G = cnt[L + 1];
-    kFillGroups<<<gridFor(8 * G, 256), 256, 0, ctx->stream>>>(G, Optr[L + 1], d.nodeMorton, d.nodeParent,
-                                                              d.nodeChild0, d.nodeLeaf, d.levelStart[L]);
-    ITS_LAUNCHED(ctx);
-  }
-  for (int L = 1; L < top; ++L) {
-    kFillOccupied<<<gridFor(cnt[L], 256), 256, 0, ctx->stream>>>(cnt[L], Optr[L], grp[L].p, d.levelStart[L],
-                                                                  d.levelStart[L - 1], d.nodeParent,
-                                                                  d.nodeChild0, d.nodeLeaf);
-    ITS_LAUNCHED(ctx);
-  }
-  {
-    uint32_t O0 = 0;
-    ITS_CU(ctx, cudaMemcpyAsync(&O0, Optr[top], 4, cudaMemcpyDeviceToHost, ctx->stream));
-    ITS_CU(ctx, cudaStreamSynchronize(ctx->stream));
-    kFillRoot<<<1, 32, 0, ctx->stream>>>(O0, d.levelStart[top], top >= 1 ? d.levelStart[top - 1] : 0, top >= 1 ? 1 : 0,
-                                         d.nodeMorton, d.nodeParent, d.nodeChild0, d.nodeLeaf, d.nodeNb);
-    ITS_LAUNCHED(ctx);
-  }
-  O.clear();
-  grp.clear();
+  kNodes<<<gridFor(total, 256), 256, 0, ctx->stream>>>(P, V, d.voxels, d.nodeMorton, d.nodeParent, d.nodeChild0,
+                                                      d.nodeLeaf);
+  ITS_LAUNCHED(ctx);
+  kNeighbors<<<gridFor(total * 27, 256), 256, 0, ctx->stream>>>(P, V, d.nodeMorton, d.nodeNb);
+  ITS_LAUNCHED(ctx);
 
-  // 4. neighbours, top-down
-  for (int L = top - 1; L >= 0; --L) {
-    const int64_t n27 = d.levelCount[L] * 27;
-    kNeighbors<<<gridFor(n27, 256), 256, 0, ctx->stream>>>(d.levelCount[L], d.levelStart[L], d.nodeMorton,
-                                                           d.nodeParent, d.nodeChild0, d.nodeNb);
-    ITS_LAUNCHED(ctx);
-  }
-
-  // 5. corner vertices per depth
-  DevBuf<uint32_t> vcnt;
-  if ((st = vcnt.zeros(ctx, d.depth)) != ITS_OK) return st;
+  // 4. corner vertices per depth and fine-node edges: marked, ranked, counted
   for (int L = 0; L < d.depth; ++L) {
-    const uint32_t M = (uint32_t)(res >> L) + 1u;
-    const int64_t words = ((int64_t)M * M * M + 63) / 64;
-    if ((st = devAlloc(ctx, (void**)&d.vbits[L], words * 8)) != ITS_OK) return st;
-    if ((st = devAlloc(ctx, (void**)&d.vrank[L], words * 4)) != ITS_OK) return st;
-    ITS_CU(ctx, cudaMemsetAsync(d.vbits[L], 0, words * 8, ctx->stream));
-    kMarkCorners<<<gridFor(d.levelCount[L] * 8, 256), 256, 0, ctx->stream>>>(d.levelCount[L], d.levelStart[L],
-                                                                              d.nodeMorton, M, d.vbits[L]);
-    ITS_LAUNCHED(ctx);
-    const unsigned long long* bits = d.vbits[L];
-    auto f = [bits] __device__(int64_t i) -> uint32_t { return (uint32_t)__popcll(bits[i]); };
-    if ((st = scanExclusiveAlloc<uint32_t>(ctx, f, words, StorePrefix<uint32_t>{d.vrank[L]}, vcnt.p + L)) != ITS_OK)
-      return st;
+    const int64_t M = (int64_t)(res >> L) + 1;
+    V.vword[L + 1] = V.vword[L] + (M * M * M + 63) / 64;
   }
+  const int64_t vwords = V.vword[d.depth], nf0 = d.levelCount[0];
+  const uint32_t M0 = (uint32_t)res + 1u;
+  const int64_t ewords = (3ll * M0 * M0 * M0 + 63) / 64;
+  if ((st = devAlloc(ctx, (void**)&d.vbits[0], vwords * 8)) != ITS_OK) return st;
+  if ((st = devAlloc(ctx, (void**)&d.vrank[0], vwords * 4)) != ITS_OK) return st;
+  if ((st = devAlloc(ctx, (void**)&d.ebits, ewords * 8)) != ITS_OK) return st;
+  if ((st = devAlloc(ctx, (void**)&d.erank, ewords * 4)) != ITS_OK) return st;
+  for (int L = 1; L < d.depth; ++L) {
+    d.vbits[L] = d.vbits[0] + V.vword[L];
+    d.vrank[L] = d.vrank[0] + V.vword[L];
+  }
+  ITS_CU(ctx, cudaMemsetAsync(d.vbits[0], 0, vwords * 8, ctx->stream));
+  ITS_CU(ctx, cudaMemsetAsync(d.ebits, 0, ewords * 8, ctx->stream));
+  kMarkCorners<<<gridFor(total * 8, 256), 256, 0, ctx->stream>>>(V, d.nodeMorton, d.vbits[0]);
+  ITS_LAUNCHED(ctx);
+  kMarkEdges<<<gridFor(nf0 * 12, 256), 256, 0, ctx->stream>>>(nf0, d.nodeMorton, M0, d.ebits);
+  ITS_LAUNCHED(ctx);
   {
-    std::vector<uint32_t> hv(d.depth);
-    ITS_CU(ctx, cudaMemcpyAsync(hv.data(), vcnt.p, 4 * d.depth, cudaMemcpyDeviceToHost, ctx->stream));
+    if ((st = scanExclusiveAlloc<uint32_t>(ctx, popc(d.vbits[0]), vwords, StorePrefix<uint32_t>{d.vrank[0]},
+                                           counts.p + d.depth - 1)) != ITS_OK ||
+        (st = scanExclusiveAlloc<uint32_t>(ctx, popc(d.ebits), ewords, StorePrefix<uint32_t>{d.erank},
+                                           counts.p + d.depth)) != ITS_OK)
+      return st;
+    Bounds B{d.depth - 1, {}};
+    for (int L = 0; L + 1 < d.depth; ++L) B.at[L] = V.vword[L + 1];
+    kRanksAt<<<1, 32, 0, ctx->stream>>>(d.vrank[0], B, counts.p);
+    ITS_LAUNCHED(ctx);
+    ITS_CU(ctx, cudaMemcpyAsync(host, counts.p, (d.depth + 1) * 4, cudaMemcpyDeviceToHost, ctx->stream));
     ITS_CU(ctx, cudaStreamSynchronize(ctx->stream));
-    int64_t t = 0;
-    for (int L = 0; L < d.depth; ++L) { d.vertStart[L] = t; d.vertCount[L] = hv[L]; t += hv[L]; }
-    d.vertStart[d.depth] = t;
-    d.numVerts = t;
   }
+  for (int L = 0; L < d.depth; ++L) V.vert[L + 1] = host[L];
+  for (int L = 0; L < d.depth; ++L) {
+    d.vertStart[L] = V.vert[L];
+    d.vertCount[L] = V.vert[L + 1] - V.vert[L];
+  }
+  d.vertStart[d.depth] = d.numVerts = V.vert[d.depth];
+  d.numEdges = host[d.depth];
   if ((st = devAlloc(ctx, (void**)&d.vertLin, d.numVerts * 4)) != ITS_OK) return st;
   if ((st = devAlloc(ctx, (void**)&d.vertOwner, d.numVerts * 4)) != ITS_OK) return st;
   if ((st = devAlloc(ctx, (void**)&d.vertPos, d.numVerts * 24)) != ITS_OK) return st;
   if ((st = devAlloc(ctx, (void**)&d.vertKey, d.numVerts * 8)) != ITS_OK) return st;
-  ITS_CU(ctx, cudaMemsetAsync(d.vertOwner, 0xFF, d.numVerts * 4, ctx->stream));
-  for (int L = 0; L < d.depth; ++L) {
-    const uint32_t M = (uint32_t)(res >> L) + 1u;
-    const int64_t words = ((int64_t)M * M * M + 63) / 64;
-    kEmitBits<<<gridFor(words, 256), 256, 0, ctx->stream>>>(words, d.vbits[L], d.vrank[L], d.vertLin + d.vertStart[L]);
-    ITS_LAUNCHED(ctx);
-    kOwnerCorners<<<gridFor(d.levelCount[L] * 8, 256), 256, 0, ctx->stream>>>(d.levelCount[L], d.levelStart[L],
-                                                                               d.nodeMorton, d.lattice(L), d.vertOwner);
-    ITS_LAUNCHED(ctx);
-    const double w = d.unit[0] * (double)(1u << L);
-    kVertexPositions<<<gridFor(d.vertCount[L], 256), 256, 0, ctx->stream>>>(d.vertCount[L], d.vertStart[L], M, L, g,
-                                                                             w, d.vertLin, d.vertOwner, d.nodeMorton,
-                                                                             d.vertPos, d.vertKey);
-    ITS_LAUNCHED(ctx);
-  }
+  kEmitBits<<<gridFor(vwords, 256), 256, 0, ctx->stream>>>(vwords, d.vbits[0], d.vrank[0], d.vertLin, d.vertOwner);
+  ITS_LAUNCHED(ctx);
+  kOwnerCorners<<<gridFor(total * 8, 256), 256, 0, ctx->stream>>>(V, d.nodeMorton, d.vbits[0], d.vrank[0], d.vertOwner);
+  ITS_LAUNCHED(ctx);
+  kVertexPositions<<<gridFor(d.numVerts, 256), 256, 0, ctx->stream>>>(V, g, d.unit[0], d.vertLin, d.vertOwner,
+                                                                     d.nodeMorton, d.vertPos, d.vertKey);
+  ITS_LAUNCHED(ctx);
 
-  // 6. fine-node edges and the fine-node occupancy bitset
-  {
-    const uint32_t M = (uint32_t)res + 1u;
-    const int64_t ebitsN = 3ll * M * M * M;
-    const int64_t words = (ebitsN + 63) / 64;
-    if ((st = devAlloc(ctx, (void**)&d.ebits, words * 8)) != ITS_OK) return st;
-    if ((st = devAlloc(ctx, (void**)&d.erank, words * 4)) != ITS_OK) return st;
-    ITS_CU(ctx, cudaMemsetAsync(d.ebits, 0, words * 8, ctx->stream));
-    const int64_t nf0 = d.levelCount[0];
-    kMarkEdges<<<gridFor(nf0 * 12, 256), 256, 0, ctx->stream>>>(nf0, d.nodeMorton, M, d.ebits);
-    ITS_LAUNCHED(ctx);
-    const unsigned long long* bits = d.ebits;
-    auto f = [bits] __device__(int64_t i) -> uint32_t { return (uint32_t)__popcll(bits[i]); };
-    if ((st = scanExclusiveAlloc<uint32_t>(ctx, f, words, StorePrefix<uint32_t>{d.erank}, dCount.p)) != ITS_OK) return st;
-    uint32_t ne = 0;
-    if ((st = readScalar(ctx, dCount.p, &ne)) != ITS_OK) return st;
-    d.numEdges = ne;
-    if ((st = devAlloc(ctx, (void**)&d.edgeKey, (size_t)ne * 4)) != ITS_OK) return st;
-    if ((st = devAlloc(ctx, (void**)&d.edgeOwner, (size_t)ne * 4)) != ITS_OK) return st;
-    ITS_CU(ctx, cudaMemsetAsync(d.edgeOwner, 0xFF, (size_t)ne * 4, ctx->stream));
-    kEmitBits<<<gridFor(words, 256), 256, 0, ctx->stream>>>(words, d.ebits, d.erank, d.edgeKey);
-    ITS_LAUNCHED(ctx);
-    kOwnerEdges<<<gridFor(nf0 * 12, 256), 256, 0, ctx->stream>>>(nf0, d.nodeMorton, M, d.ebits, d.erank, d.edgeOwner);
-    ITS_LAUNCHED(ctx);
-    if ((st = devAlloc(ctx, (void**)&d.fineOcc, gridWords * 8)) != ITS_OK) return st;
-    ITS_CU(ctx, cudaMemsetAsync(d.fineOcc, 0, gridWords * 8, ctx->stream));
-    kMarkFine<<<gridFor(nf0, 256), 256, 0, ctx->stream>>>(nf0, d.nodeMorton, (unsigned long long*)d.fineOcc);
-    ITS_LAUNCHED(ctx);
-    if ((st = devAlloc(ctx, (void**)&d.fineRank, gridWords * 4)) != ITS_OK) return st;
-    const unsigned long long* occBits = (const unsigned long long*)d.fineOcc;
-    auto pc = [occBits] __device__(int64_t i) -> uint32_t { return (uint32_t)__popcll(occBits[i]); };
-    if ((st = scanExclusiveAlloc<uint32_t>(ctx, pc, gridWords, StorePrefix<uint32_t>{d.fineRank}, (uint32_t*)nullptr)) !=
-        ITS_OK)
-      return st;
-  }
+  // 5. fine-node edges and the fine-node occupancy bitset
+  if ((st = devAlloc(ctx, (void**)&d.edgeKey, (size_t)d.numEdges * 4)) != ITS_OK) return st;
+  if ((st = devAlloc(ctx, (void**)&d.edgeOwner, (size_t)d.numEdges * 4)) != ITS_OK) return st;
+  kEmitBits<<<gridFor(ewords, 256), 256, 0, ctx->stream>>>(ewords, d.ebits, d.erank, d.edgeKey, d.edgeOwner);
+  ITS_LAUNCHED(ctx);
+  kOwnerEdges<<<gridFor(nf0 * 12, 256), 256, 0, ctx->stream>>>(nf0, d.nodeMorton, M0, d.ebits, d.erank, d.edgeOwner);
+  ITS_LAUNCHED(ctx);
+  const int64_t gridWords = P.word[1];
+  if ((st = devAlloc(ctx, (void**)&d.fineOcc, gridWords * 8)) != ITS_OK) return st;
+  if ((st = devAlloc(ctx, (void**)&d.fineRank, gridWords * 4)) != ITS_OK) return st;
+  kFineNodes<<<gridFor(gridWords, 256), 256, 0, ctx->stream>>>(P, V, gridWords, (unsigned long long*)d.fineOcc,
+                                                              d.fineRank);
+  ITS_LAUNCHED(ctx);
   // per-node sums of the face samples (features of the share network)
   ITS_CU(ctx, cudaEventRecord(ev[1], ctx->stream));
   if ((st = nodeSampleStats(ctx, d, dV, dF, nf)) != ITS_OK) return st;
