@@ -26,8 +26,10 @@ namespace its {
 
 
 template <class Op>
-__global__ void __launch_bounds__(kRedThreads) kReduce(Op op, int64_t n, double* __restrict__ partials,
-                                                       CgScalars* __restrict__ S, int honorDone) {
+__global__ void __launch_bounds__(kRedThreads) kReduce(Op op, int64_t n, double* partials, CgScalars* S,
+                                                       int honorDone) {
+  gridDependencyWait();
+  gridDependents();
   if (honorDone && S->done) return;
   double a = 0.0, b = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)kRedThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kRedThreads)
@@ -57,8 +59,10 @@ __global__ void __launch_bounds__(kRedThreads) kReduce(Op op, int64_t n, double*
 }
 
 // ---- initial state ------------------------------------------------------------------------
-__global__ void kUpdateP(int64_t n, const double* __restrict__ nr, const double* __restrict__ invdiag,
-                         double* __restrict__ p, float* __restrict__ pf, const CgScalars* __restrict__ S) {
+__global__ void kUpdateP(int64_t n, const double* nr, const double* __restrict__ invdiag, double* p, float* pf,
+                         const CgScalars* S) {
+  gridDependencyWait();
+  gridDependents();
   if (S->done) return;
   const double beta = S->beta;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -131,10 +135,9 @@ struct SolveCtx {
 };
 
 template <class Op>
-static its_status reduce(its_ctx* ctx, const SolveCtx& sc, const Op& o, int honorDone) {
-  kReduce<Op><<<sc.redBlocks, kRedThreads, 0, ctx->stream>>>(o, sc.op->n, sc.part[o.slot], sc.S, honorDone);
-  ITS_LAUNCHED(ctx);
-  return ITS_OK;
+static its_status reduce(its_ctx* ctx, const SolveCtx& sc, const Op& o, int honorDone, bool dependent = false) {
+  return launchDependent(ctx, dependent, kReduce<Op>, sc.redBlocks, kRedThreads, 0, ctx->stream, o, sc.op->n,
+                         sc.part[o.slot], sc.S, honorDone);
 }
 
 // CGLS on A x = rhs (FP64 values, or FP32 copies when f32), starting from x (in w.x).
@@ -159,23 +162,23 @@ static its_status cglsInit(its_ctx* ctx, const SolveCtx& sc, const double* rhs, 
   return ITS_OK;
 }
 
-static its_status cglsIteration(its_ctx* ctx, const SolveCtx& sc, bool f32) {
+// One iteration, each kernel launched while the one before drains.
+static its_status cglsIteration(its_ctx* ctx, const SolveCtx& sc, bool f32, bool dependent) {
   its_op* op = sc.op;
   const Work& w = sc.w;
   its_status st;
   const int* skip = &sc.S->done;
-  if (f32) st = spmv(ctx, op->A32(), op->planA, (const float*)w.pf, w.t, skip);
-  else st = spmv(ctx, op->A64(), op->planA, (const double*)w.p, w.t, skip);
+  if (f32) st = spmv(ctx, op->A32(), op->planA, (const float*)w.pf, w.t, skip, dependent);
+  else st = spmv(ctx, op->A64(), op->planA, (const double*)w.p, w.t, skip, dependent);
   if (st != ITS_OK) return st;
-  if ((st = reduce(ctx, sc, OpTmpNorm{w.t}, 1)) != ITS_OK) return st;
-  if ((st = reduce(ctx, sc, OpUpdateXR{sc.S, w.x, w.r, f32 ? w.rf : nullptr, w.p, w.t}, 1)) != ITS_OK) return st;
-  if (f32) st = spmv(ctx, op->T32(), op->planT, (const float*)w.rf, w.nr, skip);
-  else st = spmv(ctx, op->T64(), op->planT, (const double*)w.r, w.nr, skip);
+  if ((st = reduce(ctx, sc, OpTmpNorm{w.t}, 1, true)) != ITS_OK) return st;
+  if ((st = reduce(ctx, sc, OpUpdateXR{sc.S, w.x, w.r, f32 ? w.rf : nullptr, w.p, w.t}, 1, true)) != ITS_OK) return st;
+  if (f32) st = spmv(ctx, op->T32(), op->planT, (const float*)w.rf, w.nr, skip, true);
+  else st = spmv(ctx, op->T64(), op->planT, (const double*)w.r, w.nr, skip, true);
   if (st != ITS_OK) return st;
-  if ((st = reduce(ctx, sc, OpNormal{w.nr, op->invdiag}, 1)) != ITS_OK) return st;
-  kUpdateP<<<sc.redBlocks, 256, 0, ctx->stream>>>(op->n, w.nr, op->invdiag, w.p, f32 ? w.pf : nullptr, sc.S);
-  ITS_LAUNCHED(ctx);
-  return ITS_OK;
+  if ((st = reduce(ctx, sc, OpNormal{w.nr, op->invdiag}, 1, true)) != ITS_OK) return st;
+  return launchDependent(ctx, true, kUpdateP, sc.redBlocks, 256, 0, ctx->stream, op->n, (const double*)w.nr,
+                         (const double*)op->invdiag, w.p, f32 ? w.pf : (float*)nullptr, (const CgScalars*)sc.S);
 }
 
 // Runs iterations until the device sets done: graphs of `every` iterations.
@@ -191,7 +194,7 @@ static its_status cglsRun(its_ctx* ctx, const SolveCtx& sc, bool f32, int every)
     ITS_CU(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     its_status st = ITS_OK;
     const int64_t before = ctx->launches;
-    for (int k = 0; k < every && st == ITS_OK; ++k) st = cglsIteration(ctx, sc, f32);
+    for (int k = 0; k < every && st == ITS_OK; ++k) st = cglsIteration(ctx, sc, f32, k > 0);
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
     if (st != ITS_OK) return st;
     if (e != cudaSuccess) return cudaFail(ctx, e, "cudaStreamEndCapture");

@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kRsThreads, 6) kRadixDownsweep(const uint32_t*
     if (mine + 32 * j < n) {
       const uint32_t digit = (key[j] >> shift) & 255u, at = sFirst[digit] + warpCnt[warp][digit] + rank[j];
       sKey[at] = key[j];
-      sVal[at] = vals[mine + 32 * j];
+      sVal[at] = vals ? vals[mine + 32 * j] : (uint32_t)(mine + 32 * j);
     }
   __syncthreads();
 #pragma unroll
