@@ -27,7 +27,6 @@ constexpr int kIn = 64, kHid = 128;
 constexpr int64_t kOffW1 = 0, kOffB1 = kOffW1 + kHid * kIn, kOffW2 = kOffB1 + kHid, kOffB2 = kOffW2 + kHid * kHid,
                   kOffW3 = kOffB2 + kHid, kOffB3 = kOffW3 + kHid * kHid, kOffW4 = kOffB3 + kHid,
                   kOffB4 = kOffW4 + kHid, kNumParams = kOffB4 + 1;
-constexpr int kSplitK = 128;  // weight-gradient partial sums per layer
 
 using bf16 = __nv_bfloat16;
 
@@ -199,31 +198,9 @@ __device__ __forceinline__ uint4 packBf16x8(const float* v) {
   for (int e = 0; e < 4; ++e) q[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
   return r;
 }
-// The transposed copy of a 128-row tile goes through shared memory (sT[column][row], BF16):
-// each thread stages its row's values, then the block writes whole rows of the transposed
-// matrix (128 consecutive m) in 16-byte pieces.
-__device__ __forceinline__ void stageT(bf16* sT, int row, int j, const uint4& vals) {
-  const bf16* v = (const bf16*)&vals;
-#pragma unroll
-  for (int e = 0; e < 8; ++e) sT[(j + e) * 128 + row] = v[e];
-}
-__device__ __forceinline__ void storeT(const bf16* sT, bf16* dstT, int64_t ldt, int64_t m0, int64_t M) {
-  for (int p = threadIdx.x; p < kHid * 16; p += blockDim.x) {
-    const int j = p >> 4, r8 = (p & 15) * 8;
-    const int64_t m = m0 + r8;
-    bf16* dst = dstT + (int64_t)j * ldt + m;
-    const bf16* src = sT + j * 128 + r8;
-    if (m + 8 <= M) {
-      *(uint4*)dst = *(const uint4*)src;
-    } else {
-      for (int e = 0; e < 8 && m + e < M; ++e) dst[e] = src[e];
-    }
-  }
-}
-
-// A row-major 128-row tile goes through shared memory too: each thread stages its row's 16-byte
+// A row-major 128-row tile goes out through shared memory: each thread stages its row's 16-byte
 // pieces (piece c of row r at slot c ^ (r mod pieces per row): no bank conflicts either way),
-// then consecutive threads write consecutive pieces of whole rows, or, for loadRows, read them.
+// then consecutive threads write consecutive pieces of whole rows.
 template <int RowBytes>
 __device__ __forceinline__ void stageRow(uint8_t* sR, int row, int byteCol, const uint4& v) {
   constexpr int kPieces = RowBytes / 16;
@@ -243,41 +220,13 @@ __device__ __forceinline__ void storeRows(const uint8_t* sR, void* dst, int64_t 
       *(uint4*)((uint8_t*)dst + (m0 + row) * RowBytes + c * 16) = rowPiece<RowBytes>(sR, row, c * 16);
   }
 }
-template <int RowBytes, int kThreads>  // a thread's loads go out four at a time before their shared stores
-__device__ __forceinline__ void loadRows(uint8_t* sR, const void* src, int64_t m0, int64_t M) {
-  constexpr int kPieces = RowBytes / 16, kPer = 128 * kPieces / kThreads, kBatch = 4;
-  static_assert(kPer * kThreads == 128 * kPieces && kPer % kBatch == 0, "whole batches of pieces per thread");
-#pragma unroll
-  for (int i0 = 0; i0 < kPer; i0 += kBatch) {
-    uint4 q[kBatch];
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const int p = threadIdx.x + (i0 + i) * kThreads, row = p / kPieces, c = p % kPieces;
-      q[i] = m0 + row < M ? *(const uint4*)((const uint8_t*)src + (m0 + row) * RowBytes + c * 16)
-                          : make_uint4(0, 0, 0, 0);
-    }
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const int p = threadIdx.x + (i0 + i) * kThreads;
-      stageRow<RowBytes>(sR, p / kPieces, (p % kPieces) * 16, q[i]);
-    }
-  }
-}
-
-// Hidden layer: z = acc + b, h = gelu(z); Z (FP32, for the backward pass), H row-major and
-// its transpose (the operands of the next layer and of the weight gradient). Ht and H go out
-// through the two halves of the stage area, then Z through all of it.
+// Hidden layer: h = gelu(acc + b), out through the first half of the stage area.
 struct EpiHidden {
   const float* bias;
-  float* Z;
   bf16* H;
-  bf16* Ht;
-  int64_t ldt;
   template <int C>
   __device__ void operator()(int64_t m, bool valid, int j0, float (&v)[C], float*, float*, int, uint8_t* stage,
                              int64_t m0, int64_t M) const {
-    bf16* sT = (bf16*)stage;
-    uint8_t* sH = stage + kHid * 128 * 2;  // the second half: H row-major
     const int row = threadIdx.x & 127;
     if (valid) {
 #pragma unroll
@@ -285,170 +234,44 @@ struct EpiHidden {
         const int j = j0 + jb;
         float h[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          v[jb + e] += bias[j + e];  // z, kept for Z
-          h[e] = geluF(v[jb + e]);
-        }
-        const uint4 hb = packBf16x8(h);
-        stageRow<kHid * 2>(sH, row, j * 2, hb);
-        if (Ht) stageT(sT, row, j, hb);
+        for (int e = 0; e < 8; ++e) h[e] = geluF(v[jb + e] + bias[j + e]);
+        stageRow<kHid * 2>(stage, row, j * 2, packBf16x8(h));
       }
     }
     __syncthreads();
-    storeRows<kHid * 2>(sH, H, m0, M);
-    if (Ht) storeT(sT, Ht, ldt, m0, M);
-    if (!Z) return;
-    __syncthreads();
-    if (valid) {
-#pragma unroll
-      for (int jb = 0; jb < C; jb += 4)
-        stageRow<kHid * 4>(stage, row, (j0 + jb) * 4,
-                           make_uint4(__float_as_uint(v[jb]), __float_as_uint(v[jb + 1]), __float_as_uint(v[jb + 2]),
-                                      __float_as_uint(v[jb + 3])));
-    }
-    __syncthreads();
-    storeRows<kHid * 4>(stage, Z, m0, M);
+    storeRows<kHid * 2>(stage, H, m0, M);
   }
 };
 
 constexpr int kOutParts = 4;  // partial sums of the output unit (one per quarter of the columns)
 static_assert(kOutParts == kGemmGroups, "the output unit's partial sums follow the warp groups");
 
-// Last hidden layer plus the output unit. Inference: out = sum_j h_j w4_j + b4. Training also
-// forms the loss gradient d = scale (out - y) and dZ3 = d w4 gelu'(z3), H3 transposed (for
-// the w4 gradient) and the per-row squared error. The output unit sums each quarter of the
-// columns in order (one per warp group), then the four partial sums in order -- the fused
-// inference kernel's split, so both give the same bits.
+// Last hidden layer plus the output unit: out = sum_j h_j w4_j + b4. The output unit sums each quarter
+// of the columns in order (one per warp group), then the four partial sums in order -- the fused
+// kernels' split, so all give the same bits.
 struct EpiOutput {
   const float* bias;
   const float* w4;  // BF16-rounded values
   const float* b4;
   float* out;
-  // training only
-  const float* y;
-  float scale;
-  bf16* H3t;  // H3 transposed (for the w4 gradient)
-  bf16* dZ;
-  bf16* dZt;
-  int64_t ldt;
-  float* dOut;
-  float* sqErr;
   template <int C>
-  __device__ void operator()(int64_t m, bool valid, int j0, float (&v)[C], float* sPart, float* sRow, int grp,
-                             uint8_t* stage, int64_t m0, int64_t M) const {
+  __device__ void operator()(int64_t m, bool valid, int j0, float (&v)[C], float* sPart, float*, int grp, uint8_t*,
+                             int64_t, int64_t) const {
     const int row = threadIdx.x & 127;
-    bf16* sT3 = (bf16*)stage + kHid * 128;  // H3's transposed tile (the stage area's second half)
     float o = 0.0f;
     if (valid) {
 #pragma unroll
-      for (int jb = 0; jb < C; jb += 8) {
-        float h[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int j = j0 + jb + e;
-          v[jb + e] += bias[j];
-          h[e] = __bfloat162float(__float2bfloat16_rn(geluF(v[jb + e])));
-          o += h[e] * w4[j];
-        }
-        if (H3t) stageT(sT3, row, j0 + jb, packBf16x8(h));
-      }
+      for (int e = 0; e < C; ++e)
+        o += __bfloat162float(__float2bfloat16_rn(geluF(v[e] + bias[j0 + e]))) * w4[j0 + e];
     }
     sPart[grp * 128 + row] = o;
     __syncthreads();
-    if (H3t) storeT(sT3, H3t, ldt, m0, M);
-    if (grp == 0) {
-      float d = 0.0f;
-      if (valid) {
-        float oo = sPart[row];
+    if (grp == 0 && valid) {
+      float oo = sPart[row];
 #pragma unroll
-        for (int g = 1; g < kOutParts; ++g) oo += sPart[g * 128 + row];
-        oo += b4[0];
-        if (out) out[m] = oo;
-        if (y) {
-          const float e = oo - y[m];
-          d = scale * e;
-          dOut[m] = d;
-          sqErr[m] = e * e;
-        }
-      }
-      sRow[row] = d;
+      for (int g = 1; g < kOutParts; ++g) oo += sPart[g * 128 + row];
+      out[m] = oo + b4[0];
     }
-    __syncthreads();
-    if (!y) return;
-    bf16* sT = (bf16*)stage;  // dZt; dZ row-major in the second half (H3t's copy is out)
-    if (valid) {
-      const float d = sRow[row];
-#pragma unroll
-      for (int jb = 0; jb < C; jb += 8) {
-        const int j = j0 + jb;
-        float g[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) g[k] = d * w4[j + k] * geluGrad(v[jb + k]);
-        const uint4 gb = packBf16x8(g);
-        stageRow<kHid * 2>((uint8_t*)sT3, row, j * 2, gb);
-        stageT(sT, row, j, gb);
-      }
-    }
-    __syncthreads();
-    storeRows<kHid * 2>((const uint8_t*)sT3, dZ, m0, M);
-    storeT(sT, dZt, ldt, m0, M);
-  }
-};
-
-// Backward through a hidden layer: dZ = acc * gelu'(Z) (acc = dH of that layer).
-struct EpiBack {
-  const float* Z;
-  bf16* dZ;
-  bf16* dZt;
-  int64_t ldt;
-  template <int C>
-  __device__ void operator()(int64_t m, bool valid, int j0, float (&v)[C], float*, float*, int, uint8_t* stage,
-                             int64_t m0, int64_t M) const {
-    // Z's tile comes in through all of the stage area (whole rows per warp), then dZt and dZ go
-    // out through its two halves
-    bf16* sT = (bf16*)stage;
-    uint8_t* sD = stage + kHid * 128 * 2;
-    const int row = threadIdx.x & 127;
-    loadRows<kHid * 4, kGemmThreads>(stage, Z, m0, M);
-    __syncthreads();
-    if (valid) {  // dZ in place of the accumulators
-#pragma unroll
-      for (int jb = 0; jb < C; jb += 4) {
-        const uint4 zq = rowPiece<kHid * 4>(stage, row, (j0 + jb) * 4);
-        v[jb] *= geluGrad(__uint_as_float(zq.x));
-        v[jb + 1] *= geluGrad(__uint_as_float(zq.y));
-        v[jb + 2] *= geluGrad(__uint_as_float(zq.z));
-        v[jb + 3] *= geluGrad(__uint_as_float(zq.w));
-      }
-    }
-    __syncthreads();
-    if (valid) {
-#pragma unroll
-      for (int jb = 0; jb < C; jb += 8) {
-        const int j = j0 + jb;
-        const uint4 gb = packBf16x8(v + jb);
-        if (dZ) stageRow<kHid * 2>(sD, row, j * 2, gb);
-        stageT(sT, row, j, gb);
-      }
-    }
-    __syncthreads();
-    if (dZ) storeRows<kHid * 2>(sD, dZ, m0, M);
-    storeT(sT, dZt, ldt, m0, M);
-  }
-};
-
-// Split-K partial of a weight gradient: partial[split][m][n].
-template <int N>
-struct EpiPartial {
-  float* partial;
-  int64_t rows;
-  template <int C>
-  __device__ void operator()(int64_t m, bool valid, int j0, float (&v)[C], float*, float*, int, uint8_t*, int64_t,
-                             int64_t) const {
-    if (!valid) return;
-    float* p = partial + ((int64_t)blockIdx.z * rows + m) * N + j0;
-#pragma unroll
-    for (int j = 0; j < C; j += 4) *(float4*)(p + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
   }
 };
 
@@ -674,107 +497,363 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 }
 
 // ---- small kernels ----------------------------------------------------------------------
-// Features (FP32, n x 64, already normalised) to BF16 rows (and columns for training).
-__global__ void kFeaturesBf16(const float* __restrict__ X, int64_t n, bf16* __restrict__ Xb, bf16* __restrict__ Xt,
-                              int64_t ldt) {
+// Features (FP32, n x 64, already normalised) to BF16 rows.
+__global__ void kFeaturesBf16(const float* __restrict__ X, int64_t n, bf16* __restrict__ Xb) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n * kIn) return;
-  const int64_t m = i / kIn;
-  const int k = (int)(i % kIn);
-  const bf16 v = __float2bfloat16_rn(X[i]);
-  Xb[i] = v;
-  if (Xt) Xt[(int64_t)k * ldt + m] = v;
+  if (i < n * kIn) Xb[i] = __float2bfloat16_rn(X[i]);
 }
 
-// BF16 weight copies (row-major and transposed) and the BF16-rounded output weights.
-__global__ void kCastWeights(const float* __restrict__ P, bf16* __restrict__ W1, bf16* __restrict__ W1t,
-                             bf16* __restrict__ W2, bf16* __restrict__ W2t, bf16* __restrict__ W3,
-                             bf16* __restrict__ W3t, float* __restrict__ w4r) {
+// BF16 weight copies and the BF16-rounded output weights.
+__global__ void kCastWeights(const float* __restrict__ P, bf16* __restrict__ W1, bf16* __restrict__ W2,
+                             bf16* __restrict__ W3, float* __restrict__ w4r) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < kHid * kIn) {
-    const int o = i / kIn, k = i % kIn;
-    const bf16 v = __float2bfloat16_rn(P[kOffW1 + i]);
-    W1[i] = v;
-    W1t[k * kHid + o] = v;
-  }
+  if (i < kHid * kIn) W1[i] = __float2bfloat16_rn(P[kOffW1 + i]);
   if (i < kHid * kHid) {
-    const int o = i / kHid, k = i % kHid;
-    const bf16 v2 = __float2bfloat16_rn(P[kOffW2 + i]);
-    W2[i] = v2;
-    W2t[k * kHid + o] = v2;
-    const bf16 v3 = __float2bfloat16_rn(P[kOffW3 + i]);
-    W3[i] = v3;
-    W3t[k * kHid + o] = v3;
+    W2[i] = __float2bfloat16_rn(P[kOffW2 + i]);
+    W3[i] = __float2bfloat16_rn(P[kOffW3 + i]);
   }
   if (i < kHid) w4r[i] = __bfloat162float(__float2bfloat16_rn(P[kOffW4 + i]));
 }
 
-// Fixed-order block sum over a row of length n (one block per output).
-__device__ __forceinline__ float blockSum256(float v) {
-  __shared__ float sh[8];
+// ---- fused training step ------------------------------------------------------------------
+// Loss and gradient of a batch in one persistent kernel, a CTA per SM: a 128-row tile goes forward
+// and back without leaving the SM. Shared memory holds the weights (80 KB) and the tile's features,
+// H1, H2 and dZ (112 KB), each once, row by row: the transposed products (dH = dZ W, dW = dZ^T H)
+// read the same blocks MN-major. TMEM holds one 128-column accumulator for the layers and, across
+// the CTA's tiles, the three weight gradients (320 columns). gelu' needs the pre-activations in
+// FP32: they are formed again by the same products just before they are used, instead of being
+// kept. Bias and output-weight gradients are summed over a warp's rows by exchanges, a column per
+// lane. Every CTA leaves its sums in a slot of its own, which kSumPartials adds in CTA order, so a
+// step is deterministic. The forward values, the loss gradient and every dZ are those of a pass
+// layer by layer, bit for bit; the weight gradients are grouped by CTA. (Layer by layer, with the
+// activations, their transposes and FP32 pre-activations through memory, 75-84 MB a layer: 253 us in
+// 11 launches at 65,536 rows; now TRAINUS.)
+constexpr int kTrainThreads = 512;
+constexpr int64_t kPartStride = (kNumParams + 1 + 3) / 4 * 4;  // the parameters' order, then the squared errors
+constexpr int kTrainSmem = 16384 + 32768 + 32768 /*W1 W2 W3*/ + 16384 /*X*/ + 3 * 32768 /*H1 H2 dZ*/ +
+                           4 * 128 * 4 /*b1 b2 b3 w4*/ + kOutParts * 128 * 4 /*partial sums*/ + 128 * 4 /*d*/ + 64 + 1024;
+
+// Where a batch's row m lies in the dataset: itself, or a random row (splitmix64 of seed, step and m).
+struct BatchRows {
+  int64_t n;  // rows of the dataset to draw from; 0: row m itself
+  uint64_t seed, first;
+  __device__ __forceinline__ int64_t operator()(int64_t m) const {
+    if (n == 0) return m;
+    uint64_t z = seed + 0x9E3779B97F4A7C15ull * (first + (uint64_t)m + 1);
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    z ^= z >> 31;
+    return (int64_t)(z % (uint64_t)n);
+  }
+};
+
+// Column l of the warp's 32 x 32 block (v: a lane's row) summed over its rows, in lane l.
+__device__ __forceinline__ float columnSum(float (&v)[32], int lane) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float t = 0.0f;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < 8; ++w) t += sh[w];
-  return t;
-}
-
-// Gradients not produced by a GEMM: biases of the hidden layers (row sums of dZ^T), the output
-// weights (H3^T dOut), the output bias (sum dOut) and the loss (mean squared error).
-// Block b: 0..383 hidden biases, 384..511 w4, 512 b4, 513 loss.
-__global__ void __launch_bounds__(256) kSmallGrads(const bf16* __restrict__ dZ1t, const bf16* __restrict__ dZ2t,
-                                                  const bf16* __restrict__ dZ3t, const bf16* __restrict__ H3t,
-                                                  const float* __restrict__ dOut, const float* __restrict__ sqErr,
-                                                  int64_t n, int64_t ldt, float* __restrict__ grad,
-                                                  float* __restrict__ loss) {
-  const int b = blockIdx.x;
-  float s = 0.0f;
-  if (b < 3 * kHid) {
-    const bf16* row = (b < kHid ? dZ1t : b < 2 * kHid ? dZ2t : dZ3t) + (int64_t)(b % kHid) * ldt;
-    for (int64_t m = threadIdx.x; m < n; m += 256) s += __bfloat162float(row[m]);
-  } else if (b < 4 * kHid) {
-    const int j = b - 3 * kHid;
-    for (int64_t m = threadIdx.x; m < n; m += 256) s += dOut[m] * __bfloat162float(H3t[(int64_t)j * ldt + m]);
-  } else if (b == 4 * kHid) {
-    for (int64_t m = threadIdx.x; m < n; m += 256) s += dOut[m];
-  } else {
-    for (int64_t m = threadIdx.x; m < n; m += 256) s += sqErr[m];
-  }
-  const float t = blockSum256(s);
-  if (threadIdx.x != 0) return;
-  if (b < 3 * kHid) {
-    const int64_t off = b < kHid ? kOffB1 : b < 2 * kHid ? kOffB2 : kOffB3;
-    grad[off + b % kHid] = t;
-  } else if (b < 4 * kHid) {
-    grad[kOffW4 + (b - 3 * kHid)] = t;
-  } else if (b == 4 * kHid) {
-    grad[kOffB4] = t;
-  } else {
-    loss[0] = t / (float)n;
-  }
-}
-
-// Weight gradients from the split-K partials (summed in split order).
-__global__ void kSumPartials(const float* __restrict__ P1, const float* __restrict__ P2, const float* __restrict__ P3,
-                             float* __restrict__ grad) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < kHid * kIn) {
-    float s = 0.0f;
-    for (int k = 0; k < kSplitK; ++k) s += P1[(int64_t)k * kHid * kIn + i];
-    grad[kOffW1 + i] = s;
-  }
-  if (i < kHid * kHid) {
-    float s2 = 0.0f, s3 = 0.0f;
-    for (int k = 0; k < kSplitK; ++k) {
-      s2 += P2[(int64_t)k * kHid * kHid + i];
-      s3 += P3[(int64_t)k * kHid * kHid + i];
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const float other = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + o], o);
+      v[i] = (up ? v[i + o] : v[i]) + other;
     }
-    grad[kOffW2 + i] = s2;
-    grad[kOffW3 + i] = s3;
   }
+  return v[0];
+}
+
+__global__ void __launch_bounds__(kTrainThreads, 1)
+    kMlpGradientFused(const float* __restrict__ X, const float* __restrict__ y, const BatchRows rows, int64_t n,
+                      float scale, const uint8_t* __restrict__ img, const float* __restrict__ P,
+                      float* __restrict__ part, int* __restrict__ err) {
+  using namespace umma;
+  extern __shared__ uint8_t smemRaw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
+  uint8_t* sW1 = smem;
+  uint8_t* sW2 = sW1 + 16384;
+  uint8_t* sW3 = sW2 + 32768;
+  uint8_t* sX = sW3 + 32768;
+  uint8_t* sH1 = sX + 16384;
+  uint8_t* sH2 = sH1 + 32768;
+  uint8_t* sD = sH2 + 32768;
+  float* sBias = (float*)(sD + 32768);     // b1, b2, b3, w4 (128 each)
+  float* sPart = sBias + 4 * 128;          // [group][row] partial sums
+  float* sRow = sPart + kOutParts * 128;   // the loss gradient of each row
+  uint64_t* mbar = (uint64_t*)(sRow + 128);
+  uint32_t* tslot = (uint32_t*)(mbar + 2);
+  const int tid = threadIdx.x, grp = tid >> 7, row = tid & 127, warp = tid >> 5, lane = tid & 31;
+  const uint32_t bar = smemAddr(mbar), barW = smemAddr(mbar + 1);
+  if (warp == 0) tmemAlloc(smemAddr(tslot), 512);
+  if (tid == 0) {
+    mbarInit(bar, 1);
+    mbarInit(barW, 1);
+    mbarArriveExpectTx(barW, kImgBytes);
+#pragma unroll
+    for (int k = 0; k < kImgWeights / 16384; ++k) bulkLoad(smemAddr(sW1 + k * 16384), img + k * 16384, 16384, barW);
+    bulkLoad(smemAddr(sBias), img + kImgWeights, kImgBytes - kImgWeights, barW);
+  }
+  fenceBefore();
+  __syncthreads();
+  fenceAfter();
+  bool ok = mbarWait(barW, 0);
+  const uint32_t acc = *tslot, dW3 = acc + 128, dW2 = acc + 256, dW1 = acc + 384;
+  const uint32_t tl = (uint32_t)((warp & 3) * 32) << 16;  // the warp's TMEM lanes
+  const int n0 = 32 * grp;                                // the group's columns
+  const uint32_t myAcc = acc + tl + (uint32_t)n0;
+  const float *b1 = sBias + n0, *b2 = b1 + 128, *b3 = b1 + 256, *w4 = b1 + 384;
+  const float b4 = P[kOffB4];
+  constexpr uint32_t idKK = idescBf16(128, 128), idKM = idKK | kMnB, idMM = idKK | kMnA | kMnB,
+                     idMM64 = idescBf16(128, 64) | kMnA | kMnB;
+  const bool xVec = ((uintptr_t)X & 15) == 0;
+  uint32_t phase = 0;
+  float gB1 = 0.f, gB2 = 0.f, gB3 = 0.f, gW4 = 0.f, gB4 = 0.f, sq = 0.f;
+  float v[32], z[32];
+
+  // operands written by every thread -> one thread's products -> its barrier
+  auto begin = [&] {
+    fenceProxyAsync();
+    fenceBefore();
+    __syncthreads();
+    if (tid == 0) fenceAfter();
+  };
+  auto wait = [&] {
+    ok = mbarWait(bar, phase) && ok;
+    phase ^= 1u;
+    fenceAfter();
+  };
+  // acc = A B^T, A and B K-major, kBlocks blocks of 64 along K
+  auto layer = [&](const uint8_t* A, const uint8_t* B, int kBlocks) {
+    for (int kb = 0; kb < kBlocks; ++kb) {
+      const uint64_t da = descSw128(smemAddr(A + kb * 16384)), db = descSw128(smemAddr(B + kb * 16384));
+#pragma unroll
+      for (int k = 0; k < 4; ++k) mma(acc, da + 2 * k, db + 2 * k, idKK, (kb > 0 || k > 0) ? 1u : 0u);
+    }
+  };
+  // acc = dZ W (dZ K-major, W's rows are K)
+  auto back = [&](const uint8_t* W) {
+    const uint64_t db = descSw128Mn(smemAddr(W));
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+      mma(acc, descSw128(smemAddr(sD + (s >> 2) * 16384)) + 2 * (s & 3), db + 128 * s, idKM, s > 0 ? 1u : 0u);
+  };
+  // dW += dZ^T H over the tile's rows
+  auto weights = [&](uint32_t d, const uint8_t* H, uint32_t id, bool more) {
+    const uint64_t da = descSw128Mn(smemAddr(sD)), db = descSw128Mn(smemAddr(H));
+#pragma unroll
+    for (int s = 0; s < 8; ++s) mma(d, da + 128 * s, db + 128 * s, id, (more || s > 0) ? 1u : 0u);
+  };
+  // this thread's 32 columns of its row, BF16, into a K-major tile; v becomes the rounded values
+  auto store = [&](uint8_t* T) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const uint4 q = packBf16x8(v + 8 * h);
+      const __nv_bfloat162* qb = (const __nv_bfloat162*)&q;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __bfloat1622float2(qb[e]);
+        v[8 * h + 2 * e] = f.x;
+        v[8 * h + 2 * e + 1] = f.y;
+      }
+      const int c = (n0 >> 3) + h;
+      *(uint4*)(T + (c >> 3) * 16384 + swizzledChunk(row, c & 7)) = q;
+    }
+  };
+
+  const int64_t tiles = (n + 127) / 128;
+  bool more = false;
+  for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const int64_t m = t * 128 + row;
+    // features -> BF16, 16-byte chunks of the swizzled tile (rows past the batch: zeros)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int p = tid + q * kTrainThreads, pr = p >> 3, pc = p & 7;
+      const int64_t mr = t * 128 + pr;
+      float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (mr < n) {
+        const float* src = X + rows(mr) * kIn + pc * 8;
+        if (xVec) {
+          *(float4*)f = __ldg((const float4*)src);
+          *(float4*)(f + 4) = __ldg((const float4*)src + 1);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] = src[e];
+        }
+      }
+      *(uint4*)(sX + swizzledChunk(pr, pc)) = packBf16x8(f);
+    }
+    const float target = grp == 0 && m < n ? y[rows(m)] : 0.0f;
+    // forward
+    begin();
+    if (tid == 0) {
+      layer(sX, sW1, 1);
+      commit(bar);
+    }
+    wait();
+    tmemLoad32(myAcc, v);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = geluF(v[j] + b1[j]);
+    store(sH1);
+    begin();
+    if (tid == 0) {
+      layer(sH1, sW2, 2);
+      commit(bar);
+    }
+    wait();
+    tmemLoad32(myAcc, v);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = geluF(v[j] + b2[j]);
+    store(sH2);
+    begin();
+    if (tid == 0) {
+      layer(sH2, sW3, 2);
+      commit(bar);
+    }
+    wait();
+    tmemLoad32(myAcc, z);
+    float o = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      z[j] += b3[j];
+      v[j] = __bfloat162float(__float2bfloat16_rn(geluF(z[j])));
+      o += v[j] * w4[j];
+    }
+    sPart[grp * 128 + row] = o;
+    __syncthreads();
+    if (grp == 0) {
+      float d = 0.0f;
+      if (m < n) {
+        float oo = sPart[row];
+#pragma unroll
+        for (int g = 1; g < kOutParts; ++g) oo += sPart[g * 128 + row];
+        oo += b4;
+        const float e = oo - target;
+        d = scale * e;
+        gB4 += d;
+        sq += e * e;
+      }
+      sRow[row] = d;
+    }
+    __syncthreads();
+    const float d = sRow[row];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] *= d;
+    gW4 += columnSum(v, lane);
+    // backward: dZ3, then dH2 and dW3; Z2 again, dZ2, dH1 and dW2; Z1 again, dZ1 and dW1
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = d * w4[j] * geluGrad(z[j]);
+    store(sD);
+    gB3 += columnSum(v, lane);
+    begin();
+    if (tid == 0) {
+      back(sW3);
+      commit(bar);
+      weights(dW3, sH2, idMM, more);
+    }
+    wait();
+    tmemLoad32(myAcc, v);
+    begin();
+    if (tid == 0) {
+      layer(sH1, sW2, 2);
+      commit(bar);  // with it dW3's products: dZ3 has been read
+    }
+    wait();
+    tmemLoad32(myAcc, z);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] *= geluGrad(z[j] + b2[j]);
+    store(sD);
+    gB2 += columnSum(v, lane);
+    begin();
+    if (tid == 0) {
+      back(sW2);
+      commit(bar);
+      weights(dW2, sH1, idMM, more);
+    }
+    wait();
+    tmemLoad32(myAcc, v);
+    begin();
+    if (tid == 0) {
+      layer(sX, sW1, 1);
+      commit(bar);
+    }
+    wait();
+    tmemLoad32(myAcc, z);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] *= geluGrad(z[j] + b1[j]);
+    store(sD);
+    gB1 += columnSum(v, lane);
+    begin();
+    if (tid == 0) {
+      weights(dW1, sX, idMM64, more);
+      commit(bar);
+    }
+    wait();  // X and dZ1 have been read: the next tile's may come
+    more = true;
+  }
+  // the CTA's sums: weight gradients (row o of this thread), then the columns' and rows' sums
+  float* out = part + (int64_t)blockIdx.x * kPartStride;
+  tmemLoad32(dW3 + tl + (uint32_t)n0, v);
+#pragma unroll
+  for (int j = 0; j < 32; j += 4) *(float4*)(out + kOffW3 + row * kHid + n0 + j) = *(const float4*)(v + j);
+  tmemLoad32(dW2 + tl + (uint32_t)n0, v);
+#pragma unroll
+  for (int j = 0; j < 32; j += 4) *(float4*)(out + kOffW2 + row * kHid + n0 + j) = *(const float4*)(v + j);
+  {
+    float u[16];
+    tmemLoad16(dW1 + tl + (uint32_t)(16 * grp), u);
+#pragma unroll
+    for (int j = 0; j < 16; j += 4) *(float4*)(out + kOffW1 + row * kIn + 16 * grp + j) = *(const float4*)(u + j);
+  }
+  float* sums = (float*)sX;  // [warp of 32 rows][4][128 columns], then two per warp of group 0
+  const int col = n0 + lane, quarter = warp & 3;
+  sums[(quarter * 4 + 0) * 128 + col] = gB1;
+  sums[(quarter * 4 + 1) * 128 + col] = gB2;
+  sums[(quarter * 4 + 2) * 128 + col] = gB3;
+  sums[(quarter * 4 + 3) * 128 + col] = gW4;
+  if (grp == 0) {
+    for (int o = 16; o > 0; o >>= 1) {
+      gB4 += __shfl_down_sync(0xffffffffu, gB4, o);
+      sq += __shfl_down_sync(0xffffffffu, sq, o);
+    }
+    if (lane == 0) {
+      sums[16 * 128 + 2 * warp] = gB4;
+      sums[16 * 128 + 2 * warp + 1] = sq;
+    }
+  }
+  fenceBefore();
+  __syncthreads();
+  if (warp == 0) tmemFree(*tslot, 512);
+  const int64_t off[4] = {kOffB1, kOffB2, kOffB3, kOffW4};
+  {
+    float s = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s += sums[(q * 4 + grp) * 128 + row];
+    out[(grp == 0 ? off[0] : grp == 1 ? off[1] : grp == 2 ? off[2] : off[3]) + row] = s;
+  }
+  if (tid < 2) {
+    float s = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s += sums[16 * 128 + 2 * q + tid];
+    out[tid == 0 ? kOffB4 : kNumParams] = s;
+  }
+  if (!ok) atomicExch(err, 1);
+}
+
+// The CTAs' sums added in CTA order: the gradient, and the mean squared error.
+__global__ void __launch_bounds__(128) kSumPartials(const float* __restrict__ part, int ctas, int64_t n,
+                                                    float* __restrict__ grad, float* __restrict__ loss) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i > kNumParams) return;
+  float s = 0.0f;
+  int c = 0;
+  for (; c + 8 <= ctas; c += 8) {
+    float p[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) p[k] = part[(int64_t)(c + k) * kPartStride + i];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s += p[k];
+  }
+  for (; c < ctas; ++c) s += part[(int64_t)c * kPartStride + i];
+  if (i < kNumParams) grad[i] = s;
+  else loss[0] = s / (float)n;
 }
 
 // Adam (Kingma & Ba): m = b1 m + (1-b1) g; v = b2 v + (1-b2) g^2; p -= lr mhat / (sqrt(vhat) + eps).
@@ -789,42 +868,6 @@ __global__ void kAdam(float* __restrict__ P, float* __restrict__ Mo, float* __re
   Mo[i] = m;
   Ve[i] = v;
   P[i] -= lr * (m / c1) / (sqrtf(v / c2) + eps);
-}
-
-// Random batch: rows idx of the dataset (features n x 64 FP32, targets n).
-__global__ void kGatherBatch(const float* __restrict__ X, const float* __restrict__ y, int64_t n, uint64_t seed,
-                             uint64_t step, int64_t B, bf16* __restrict__ Xb, bf16* __restrict__ Xt,
-                             float* __restrict__ yb) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= B) return;
-  // splitmix64 of (seed, step, i)
-  uint64_t z = seed + 0x9E3779B97F4A7C15ull * (step * (uint64_t)B + (uint64_t)i + 1);
-  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-  z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-  z ^= z >> 31;
-  const int64_t r = (int64_t)(z % (uint64_t)n);
-  yb[i] = y[r];
-  const float* src = X + r * kIn;
-  if (((uintptr_t)X & 15) == 0) {  // the row in 16-byte pieces, the BF16 row out in 16-byte pieces
-#pragma unroll
-    for (int k = 0; k < kIn; k += 8) {
-      const float4 a = *(const float4*)(src + k), b = *(const float4*)(src + k + 4);
-      const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-      __align__(16) bf16 q[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        q[e] = __float2bfloat16_rn(f[e]);
-        Xt[(int64_t)(k + e) * B + i] = q[e];
-      }
-      *(uint4*)(Xb + i * kIn + k) = *(const uint4*)q;
-    }
-  } else {
-    for (int k = 0; k < kIn; ++k) {
-      const bf16 v = __float2bfloat16_rn(src[k]);
-      Xb[i * kIn + k] = v;
-      Xt[(int64_t)k * B + i] = v;
-    }
-  }
 }
 
 template <int N, class Epi>
@@ -857,12 +900,12 @@ struct its_mlp {
   float* G = nullptr;
   float* loss = nullptr;
   int64_t step = 0;
-  bf16 *W1, *W1t, *W2, *W2t, *W3, *W3t;
+  bf16 *W1, *W2, *W3;
   float* w4r;
   uint8_t* img;  // the fused inference kernel's shared-memory image of the parameters
   // batch buffers
-  bf16 *Xb, *Xt, *H1, *H1t, *H2, *H2t, *H3t, *dZ3, *dZ3t, *dZ2, *dZ2t, *dZ1t;
-  float *Z1, *Z2, *yb, *dOut, *sqErr, *out, *part1, *part2, *part3;
+  bf16 *Xb, *H1, *H2;
+  float* part;  // the gradient's sums, a slot per CTA
   int* err;
   std::vector<void*> allocs;
   template <typename T>
@@ -876,8 +919,7 @@ struct its_mlp {
 namespace its {
 
 static its_status mlpCast(its_mlp* h) {
-  kCastWeights<<<gridFor(kHid * kHid, 256), 256, 0, h->ctx->stream>>>(h->P, h->W1, h->W1t, h->W2, h->W2t, h->W3,
-                                                                      h->W3t, h->w4r);
+  kCastWeights<<<gridFor(kHid * kHid, 256), 256, 0, h->ctx->stream>>>(h->P, h->W1, h->W2, h->W3, h->w4r);
   ITS_LAUNCHED(h->ctx);
   kPackFusedImage<<<gridFor(128 * 8 + 2 * 128 * 16, 256), 256, 0, h->ctx->stream>>>(h->P, h->W1, h->W2, h->W3, h->w4r,
                                                                                     h->img);
@@ -885,42 +927,26 @@ static its_status mlpCast(its_mlp* h) {
   return ITS_OK;
 }
 
-// Forward of n <= cap rows already in h->Xb; training forms the loss gradients too.
-static its_status mlpForward(its_mlp* h, int64_t n, bool train, const float* y, float* out) {
+// Forward of n <= cap rows already in h->Xb, layer by layer.
+static its_status mlpForward(its_mlp* h, int64_t n, float* out) {
   its_ctx* ctx = h->ctx;
   its_status st;
-  const int64_t ldt = h->cap;
-  EpiHidden e1{h->P + kOffB1, train ? h->Z1 : nullptr, h->H1, train ? h->H1t : nullptr, ldt};
-  if ((st = gemm<kHid>(ctx, h->Xb, kIn, n, h->W1, kIn, kIn, 1, e1, h->err)) != ITS_OK) return st;
-  EpiHidden e2{h->P + kOffB2, train ? h->Z2 : nullptr, h->H2, train ? h->H2t : nullptr, ldt};
-  if ((st = gemm<kHid>(ctx, h->H1, kHid, n, h->W2, kHid, kHid, 1, e2, h->err)) != ITS_OK) return st;
-  EpiOutput e3{h->P + kOffB3, h->w4r, h->P + kOffB4, out, y, 2.0f / (float)n, train ? h->H3t : nullptr,
-               h->dZ3, h->dZ3t, ldt, h->dOut, h->sqErr};
+  if ((st = gemm<kHid>(ctx, h->Xb, kIn, n, h->W1, kIn, kIn, 1, EpiHidden{h->P + kOffB1, h->H1}, h->err)) != ITS_OK ||
+      (st = gemm<kHid>(ctx, h->H1, kHid, n, h->W2, kHid, kHid, 1, EpiHidden{h->P + kOffB2, h->H2}, h->err)) != ITS_OK)
+    return st;
+  const EpiOutput e3{h->P + kOffB3, h->w4r, h->P + kOffB4, out};
   return gemm<kHid>(ctx, h->H2, kHid, n, h->W3, kHid, kHid, 1, e3, h->err);
 }
 
-// Gradient of the mean squared error over the n rows in h->Xb/h->Xt (targets yb) into h->G.
-static its_status mlpGradient(its_mlp* h, int64_t n) {
+// Gradient of the mean squared error over n rows of X (targets y), drawn as rows says, into h->G.
+static its_status mlpGradient(its_mlp* h, const float* X, const float* y, const BatchRows& rows, int64_t n) {
   its_ctx* ctx = h->ctx;
-  its_status st;
-  const int64_t ldt = h->cap;
-  if ((st = mlpForward(h, n, true, h->yb, nullptr)) != ITS_OK) return st;
-  // dH2 = dZ3 W3 -> dZ2; dH1 = dZ2 W2 -> dZ1 (transposed only)
-  EpiBack b2{h->Z2, h->dZ2, h->dZ2t, ldt};
-  if ((st = gemm<kHid>(ctx, h->dZ3, kHid, n, h->W3t, kHid, kHid, 1, b2, h->err)) != ITS_OK) return st;
-  EpiBack b1{h->Z1, nullptr, h->dZ1t, ldt};
-  if ((st = gemm<kHid>(ctx, h->dZ2, kHid, n, h->W2t, kHid, kHid, 1, b1, h->err)) != ITS_OK) return st;
-  // weight gradients dW_l = dZ_l^T H_{l-1}: split-K over the batch
-  EpiPartial<kHid> p3{h->part3, kHid};
-  if ((st = gemm<kHid>(ctx, h->dZ3t, ldt, kHid, h->H2t, ldt, n, kSplitK, p3, h->err)) != ITS_OK) return st;
-  EpiPartial<kHid> p2{h->part2, kHid};
-  if ((st = gemm<kHid>(ctx, h->dZ2t, ldt, kHid, h->H1t, ldt, n, kSplitK, p2, h->err)) != ITS_OK) return st;
-  EpiPartial<kIn> p1{h->part1, kHid};
-  if ((st = gemm<kIn>(ctx, h->dZ1t, ldt, kHid, h->Xt, ldt, n, kSplitK, p1, h->err)) != ITS_OK) return st;
-  kSumPartials<<<gridFor(kHid * kHid, 256), 256, 0, ctx->stream>>>(h->part1, h->part2, h->part3, h->G);
+  const int64_t tiles = (n + 127) / 128;
+  const int ctas = (int)(tiles < ctx->numSMs ? tiles : ctx->numSMs);
+  kMlpGradientFused<<<ctas, kTrainThreads, kTrainSmem, ctx->stream>>>(X, y, rows, n, 2.0f / (float)n, h->img, h->P,
+                                                                     h->part, h->err);
   ITS_LAUNCHED(ctx);
-  kSmallGrads<<<4 * kHid + 2, 256, 0, ctx->stream>>>(h->dZ1t, h->dZ2t, h->dZ3t, h->H3t, h->dOut, h->sqErr, n, ldt, h->G,
-                                                     h->loss);
+  kSumPartials<<<gridFor(kNumParams + 1, 128), 128, 0, ctx->stream>>>(h->part, ctas, n, h->G, h->loss);
   ITS_LAUNCHED(ctx);
   return ITS_OK;
 }
@@ -990,13 +1016,8 @@ its_status its_mlp_create(its_ctx* ctx, int64_t batch, its_mlp** out) {
     if (s == ITS_OK) s = h->alloc(p, c);
   };
   A(&h->P, kNumParams); A(&h->Mo, kNumParams); A(&h->Ve, kNumParams); A(&h->G, kNumParams); A(&h->loss, 1);
-  A(&h->W1, kHid * kIn); A(&h->W1t, kHid * kIn); A(&h->W2, kHid * kHid); A(&h->W2t, kHid * kHid);
-  A(&h->W3, kHid * kHid); A(&h->W3t, kHid * kHid); A(&h->w4r, kHid); A(&h->img, kImgBytes);
-  A(&h->Xb, B * kIn); A(&h->Xt, B * kIn); A(&h->H1, B * kHid); A(&h->H1t, B * kHid); A(&h->H2, B * kHid);
-  A(&h->H2t, B * kHid); A(&h->H3t, B * kHid); A(&h->dZ3, B * kHid); A(&h->dZ3t, B * kHid); A(&h->dZ2, B * kHid);
-  A(&h->dZ2t, B * kHid); A(&h->dZ1t, B * kHid); A(&h->Z1, B * kHid); A(&h->Z2, B * kHid); A(&h->yb, B);
-  A(&h->dOut, B); A(&h->sqErr, B); A(&h->out, B); A(&h->part1, (int64_t)kSplitK * kHid * kIn);
-  A(&h->part2, (int64_t)kSplitK * kHid * kHid); A(&h->part3, (int64_t)kSplitK * kHid * kHid); A(&h->err, 1);
+  A(&h->W1, kHid * kIn); A(&h->W2, kHid * kHid); A(&h->W3, kHid * kHid); A(&h->w4r, kHid); A(&h->img, kImgBytes);
+  A(&h->Xb, B * kIn); A(&h->H1, B * kHid); A(&h->H2, B * kHid); A(&h->part, ctx->numSMs * kPartStride); A(&h->err, 1);
   if (s != ITS_OK) {
     for (void* p : h->allocs) devFree(ctx, p);
     delete h;
@@ -1007,8 +1028,9 @@ its_status its_mlp_create(its_ctx* ctx, int64_t batch, its_mlp** out) {
   cudaMemsetAsync(h->Ve, 0, kNumParams * 4, ctx->stream);
   cudaMemsetAsync(h->err, 0, 4, ctx->stream);
   cudaMemsetAsync(h->img, 0, kImgBytes, ctx->stream);
-  // the fused inference kernel's shared memory, set here once (not inside a graph capture)
+  // the fused kernels' shared memory, set here once (not inside a graph capture)
   ITS_CU(ctx, cudaFuncSetAttribute(kMlpForwardFused, cudaFuncAttributeMaxDynamicSharedMemorySize, kFusedSmem));
+  ITS_CU(ctx, cudaFuncSetAttribute(kMlpGradientFused, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem));
   *out = h;
   return ITS_OK;
 }
@@ -1098,9 +1120,9 @@ its_status its_mlp_forward_layers(its_mlp* h, const float* X, int64_t n, float* 
   if ((st = o.stage(ctx, out, n)) != ITS_OK) return st;
   for (int64_t r0 = 0; r0 < n; r0 += h->cap) {
     const int64_t rows = n - r0 < h->cap ? n - r0 : h->cap;
-    kFeaturesBf16<<<gridFor(rows * kIn, 256), 256, 0, ctx->stream>>>(x.d + r0 * kIn, rows, h->Xb, nullptr, 0);
+    kFeaturesBf16<<<gridFor(rows * kIn, 256), 256, 0, ctx->stream>>>(x.d + r0 * kIn, rows, h->Xb);
     ITS_LAUNCHED(ctx);
-    if ((st = mlpForward(h, rows, false, nullptr, o.d + r0)) != ITS_OK) return st;
+    if ((st = mlpForward(h, rows, o.d + r0)) != ITS_OK) return st;
   }
   if ((st = o.finish(ctx)) != ITS_OK) return st;
   return checkErr(h);
@@ -1116,11 +1138,7 @@ its_status its_mlp_gradient(its_mlp* h, const float* X, const float* y, int64_t 
   its_status st;
   if ((st = x.stage(ctx, X, n * kIn)) != ITS_OK) return st;
   if ((st = yy.stage(ctx, y, n)) != ITS_OK) return st;
-  // columns of the transposed operands are laid out with the batch capacity as leading size
-  kFeaturesBf16<<<gridFor(n * kIn, 256), 256, 0, ctx->stream>>>(x.d, n, h->Xb, h->Xt, h->cap);
-  ITS_LAUNCHED(ctx);
-  ITS_CU(ctx, cudaMemcpyAsync(h->yb, yy.d, n * 4, cudaMemcpyDeviceToDevice, ctx->stream));
-  if ((st = mlpGradient(h, n)) != ITS_OK) return st;
+  if ((st = mlpGradient(h, x.d, yy.d, BatchRows{0, 0, 0}, n)) != ITS_OK) return st;
   ITS_CU(ctx, cudaMemcpyAsync(grad, h->G, kNumParams * 4, cudaMemcpyDefault, ctx->stream));
   if (loss) ITS_CU(ctx, cudaMemcpyAsync(loss, h->loss, 4, cudaMemcpyDefault, ctx->stream));
   return checkErr(h);
@@ -1141,10 +1159,8 @@ its_status its_mlp_train(its_mlp* h, const float* X, const float* y, int64_t n, 
   DevBuf<float> curve;
   if ((st = curve.alloc(ctx, steps > 0 ? steps : 1)) != ITS_OK) return st;
   for (int64_t s = 0; s < steps; ++s) {
-    kGatherBatch<<<gridFor(h->cap, 256), 256, 0, ctx->stream>>>(x.d, yy.d, n, seed, (uint64_t)s, h->cap, h->Xb, h->Xt,
-                                                               h->yb);
-    ITS_LAUNCHED(ctx);
-    if ((st = mlpGradient(h, h->cap)) != ITS_OK) return st;
+    const BatchRows rows{n, seed, (uint64_t)s * (uint64_t)h->cap};
+    if ((st = mlpGradient(h, x.d, yy.d, rows, h->cap)) != ITS_OK) return st;
     if ((st = mlpAdam(h, lr)) != ITS_OK) return st;
     ITS_CU(ctx, cudaMemcpyAsync(curve.p + s, h->loss, 4, cudaMemcpyDeviceToDevice, ctx->stream));
   }

@@ -32,6 +32,20 @@ __device__ __forceinline__ uint64_t descSw128(uint32_t saddr) {
   return d;
 }
 
+// The same blocks (R rows of 64 bf16, the next 64 columns 16 KB on) as an operand whose M or N index
+// runs along the row and whose K index is the row: "MN-major" in the instruction descriptor. Leading
+// offset: the next 64 of M or N; stride offset: the next 8 of K; 16 of K are 2 KB (128 in the
+// descriptor's units). A transposed product needs no transposed copy.
+__device__ __forceinline__ uint64_t descSw128Mn(uint32_t saddr) {
+  uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFFu);
+  d |= (uint64_t)(16384u >> 4) << 16;
+  d |= (uint64_t)(1024u >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+constexpr uint32_t kMnA = 1u << 15, kMnB = 1u << 16;  // A, B MN-major (instruction descriptor)
+
 // Instruction descriptor of kind::f16: F32 accumulator (bits 4-5 = 1), A and B BF16 (bits 7-9
 // and 10-12 = 1), both K-major (bits 15, 16 = 0), N/8 at bits 17-22, M/16 at bits 24-28.
 __host__ __device__ constexpr uint32_t idescBf16(int M, int N) {
