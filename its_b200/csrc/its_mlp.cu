@@ -5,11 +5,11 @@
 //
 // Network: 64 features -> 128 GELU -> 128 GELU -> 128 GELU -> 1, BF16 weights and
 // activations, FP32 accumulation; FP32 master weights trained with Adam on a mean squared
-// error. Every layer product is one tcgen05 GEMM (kUmmaGemm): 128 rows per CTA, operands
-// staged in shared memory in the 128-byte-swizzled K-major layout, the accumulator in TMEM,
-// the epilogue (bias, GELU, output dot product, loss gradient, GELU derivative) fused and
-// read back with tcgen05.ld. Weight gradients are split-K GEMMs over the batch whose
-// partials are summed in a fixed order, so a training step is deterministic.
+// error. Inference and the training step are one persistent kernel each (kMlpForwardFused,
+// kMlpGradientFused): tcgen05 products of 128 rows, operands in shared memory in the
+// 128-byte-swizzled layout, accumulators in TMEM, everything between two products in the epilogue.
+// Partial sums are added in a fixed order, so a training step is deterministic. The forward pass
+// also runs layer by layer (kUmmaGemm), the same bits.
 //
 // Parameters (flat FP32): W1[128x64] b1[128] W2[128x128] b2[128] W3[128x128] b3[128]
 // w4[128] b4[1] (W[o][i]: output o, input i).
@@ -55,12 +55,15 @@ __device__ __forceinline__ float2 geluF2(float2 z) {
   const float2 h = __fmul2_rn(make_float2(0.5f, 0.5f), z);
   return __ffma2_rn(h, make_float2(tanhApprox(u.x), tanhApprox(u.y)), h);
 }
-// d gelu / dz = (1 + t)/2 + z/2 (1 - t^2) sqrt(2/pi) (1 + 3 * 0.044715 z^2), t = tanh(u)
-__device__ __forceinline__ float geluGrad(float z) {
-  const float z2 = z * z;
-  const float t = tanhApprox(z * fmaf(kGeluK0 * kGeluK1, z2, kGeluK0));
-  const float du = fmaf(3.0f * kGeluK0 * kGeluK1, z2, kGeluK0);
-  return fmaf(0.5f * z * du, fmaf(-t, t, 1.0f), 0.5f * (1.0f + t));
+// d gelu / dz = (1 + t)/2 + z/2 (1 - t^2) sqrt(2/pi) (1 + 3 * 0.044715 z^2), t = tanh(u); two lanes
+__device__ __forceinline__ float2 geluGrad2(float2 z) {
+  const float2 k0 = make_float2(kGeluK0, kGeluK0), half = make_float2(0.5f, 0.5f), one = make_float2(1.0f, 1.0f);
+  const float2 z2 = __fmul2_rn(z, z);
+  const float2 u = __fmul2_rn(z, __ffma2_rn(make_float2(kGeluK0 * kGeluK1, kGeluK0 * kGeluK1), z2, k0));
+  const float2 t = make_float2(tanhApprox(u.x), tanhApprox(u.y));
+  const float2 du = __ffma2_rn(make_float2(3.0f * kGeluK0 * kGeluK1, 3.0f * kGeluK0 * kGeluK1), z2, k0);
+  return __ffma2_rn(__fmul2_rn(__fmul2_rn(half, z), du), __ffma2_rn(make_float2(-t.x, -t.y), t, one),
+                    __fmul2_rn(half, __fadd2_rn(one, t)));
 }
 
 // ---- one tcgen05 GEMM: C[m][n] = sum_k A[m][k] B[n][k] over this CTA's K range -------------
@@ -520,18 +523,19 @@ __global__ void kCastWeights(const float* __restrict__ P, bf16* __restrict__ W1,
 // and back without leaving the SM. Shared memory holds the weights (80 KB) and the tile's features,
 // H1, H2 and dZ (112 KB), each once, row by row: the transposed products (dH = dZ W, dW = dZ^T H)
 // read the same blocks MN-major. TMEM holds one 128-column accumulator for the layers and, across
-// the CTA's tiles, the three weight gradients (320 columns). gelu' needs the pre-activations in
+// the CTA's tiles, the weight and bias gradients (320 + 48 columns). gelu' needs the pre-activations in
 // FP32: they are formed again by the same products just before they are used, instead of being
-// kept. Bias and output-weight gradients are summed over a warp's rows by exchanges, a column per
-// lane. Every CTA leaves its sums in a slot of its own, which kSumPartials adds in CTA order, so a
+// kept. The bias gradients are products with a tile of ones; the output weights' are summed over a
+// warp's rows by exchanges, a column per lane, in FP32. Every CTA leaves its sums in a slot of its own, which kSumPartials adds in CTA order, so a
 // step is deterministic. The forward values, the loss gradient and every dZ are those of a pass
 // layer by layer, bit for bit; the weight gradients are grouped by CTA. (Layer by layer, with the
 // activations, their transposes and FP32 pre-activations through memory, 75-84 MB a layer: 253 us in
-// 11 launches at 65,536 rows; now TRAINUS.)
+// 11 launches at 65,536 rows; now 66 + 8 us.)
 constexpr int kTrainThreads = 512;
 constexpr int64_t kPartStride = (kNumParams + 1 + 3) / 4 * 4;  // the parameters' order, then the squared errors
-constexpr int kTrainSmem = 16384 + 32768 + 32768 /*W1 W2 W3*/ + 16384 /*X*/ + 3 * 32768 /*H1 H2 dZ*/ +
-                           4 * 128 * 4 /*b1 b2 b3 w4*/ + kOutParts * 128 * 4 /*partial sums*/ + 128 * 4 /*d*/ + 64 + 1024;
+constexpr int kTrainSmem = 16384 + 32768 + 32768 /*W1 W2 W3*/ + 2 * 16384 /*X, this tile's and the next's*/ + 3 * 32768 /*H1 H2 dZ*/ +
+                           4096 /*ones*/ + 4 * 128 * 4 /*b1 b2 b3 w4*/ + kOutParts * 128 * 4 /*partial sums*/ + 128 * 4 /*d*/ +
+                           64 + 1024;
 
 // Where a batch's row m lies in the dataset: itself, or a random row (splitmix64 of seed, step and m).
 struct BatchRows {
@@ -572,41 +576,45 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
   uint8_t* sW2 = sW1 + 16384;
   uint8_t* sW3 = sW2 + 32768;
   uint8_t* sX = sW3 + 32768;
-  uint8_t* sH1 = sX + 16384;
+  uint8_t* sH1 = sX + 2 * 16384;
   uint8_t* sH2 = sH1 + 32768;
   uint8_t* sD = sH2 + 32768;
-  float* sBias = (float*)(sD + 32768);     // b1, b2, b3, w4 (128 each)
+  uint8_t* sOne = sD + 32768;              // 16 rows of 128 ones: dZ^T 1 is the bias gradient
+  float* sBias = (float*)(sOne + 4096);    // b1, b2, b3, w4 (128 each)
   float* sPart = sBias + 4 * 128;          // [group][row] partial sums
   float* sRow = sPart + kOutParts * 128;   // the loss gradient of each row
   uint64_t* mbar = (uint64_t*)(sRow + 128);
-  uint32_t* tslot = (uint32_t*)(mbar + 2);
+  uint32_t* tslot = (uint32_t*)(mbar + 3);
   const int tid = threadIdx.x, grp = tid >> 7, row = tid & 127, warp = tid >> 5, lane = tid & 31;
-  const uint32_t bar = smemAddr(mbar), barW = smemAddr(mbar + 1);
+  const uint32_t bar = smemAddr(mbar), barW = smemAddr(mbar + 1), barD = smemAddr(mbar + 2);
   if (warp == 0) tmemAlloc(smemAddr(tslot), 512);
   if (tid == 0) {
     mbarInit(bar, 1);
     mbarInit(barW, 1);
+    mbarInit(barD, 1);
     mbarArriveExpectTx(barW, kImgBytes);
 #pragma unroll
     for (int k = 0; k < kImgWeights / 16384; ++k) bulkLoad(smemAddr(sW1 + k * 16384), img + k * 16384, 16384, barW);
     bulkLoad(smemAddr(sBias), img + kImgWeights, kImgBytes - kImgWeights, barW);
   }
+  if (tid < 256) *(uint4*)(sOne + 16 * tid) = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
   fenceBefore();
   __syncthreads();
   fenceAfter();
   bool ok = mbarWait(barW, 0);
-  const uint32_t acc = *tslot, dW3 = acc + 128, dW2 = acc + 256, dW1 = acc + 384;
+  const uint32_t acc = *tslot, dW3 = acc + 128, dW2 = acc + 256, dW1 = acc + 384, dB = acc + 448;
   const uint32_t tl = (uint32_t)((warp & 3) * 32) << 16;  // the warp's TMEM lanes
   const int n0 = 32 * grp;                                // the group's columns
   const uint32_t myAcc = acc + tl + (uint32_t)n0;
   const float *b1 = sBias + n0, *b2 = b1 + 128, *b3 = b1 + 256, *w4 = b1 + 384;
   const float b4 = P[kOffB4];
   constexpr uint32_t idKK = idescBf16(128, 128), idKM = idKK | kMnB, idMM = idKK | kMnA | kMnB,
-                     idMM64 = idescBf16(128, 64) | kMnA | kMnB;
+                     idMM64 = idescBf16(128, 64) | kMnA | kMnB, idMK16 = idescBf16(128, 16) | kMnA;
   const bool xVec = ((uintptr_t)X & 15) == 0;
-  uint32_t phase = 0;
-  float gB1 = 0.f, gB2 = 0.f, gB3 = 0.f, gW4 = 0.f, gB4 = 0.f, sq = 0.f;
-  float v[32], z[32];
+  uint32_t phase = 0, phaseD = 0;
+  float gW4 = 0.f, gB4 = 0.f, sq = 0.f;
+  __align__(8) float v[32];
+  float2* v2 = (float2*)v;
 
   // operands written by every thread -> one thread's products -> its barrier
   auto begin = [&] {
@@ -618,6 +626,12 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
   auto wait = [&] {
     ok = mbarWait(bar, phase) && ok;
     phase ^= 1u;
+    fenceAfter();
+  };
+  // ... and the products that read dZ's tile, committed to a barrier of their own
+  auto waitD = [&] {
+    ok = mbarWait(barD, phaseD) && ok;
+    phaseD ^= 1u;
     fenceAfter();
   };
   // acc = A B^T, A and B K-major, kBlocks blocks of 64 along K
@@ -635,39 +649,48 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     for (int s = 0; s < 8; ++s)
       mma(acc, descSw128(smemAddr(sD + (s >> 2) * 16384)) + 2 * (s & 3), db + 128 * s, idKM, s > 0 ? 1u : 0u);
   };
-  // dW += dZ^T H over the tile's rows
-  auto weights = [&](uint32_t d, const uint8_t* H, uint32_t id, bool more) {
-    const uint64_t da = descSw128Mn(smemAddr(sD)), db = descSw128Mn(smemAddr(H));
+  // dW += dZ^T H over the tile's rows, and db += dZ^T 1
+  auto weights = [&](uint32_t d, const uint8_t* H, uint32_t id, uint32_t db, bool more) {
+    const uint64_t da = descSw128Mn(smemAddr(sD)), dh = descSw128Mn(smemAddr(H));
 #pragma unroll
-    for (int s = 0; s < 8; ++s) mma(d, da + 128 * s, db + 128 * s, id, (more || s > 0) ? 1u : 0u);
+    for (int s = 0; s < 8; ++s) {
+      mma(d, da + 128 * s, dh + 128 * s, id, (more || s > 0) ? 1u : 0u);
+      mma(db, da + 128 * s, descSw128(smemAddr(sOne + (s >> 2) * 2048)) + 2 * (s & 3), idMK16, (more || s > 0) ? 1u : 0u);
+    }
   };
-  // this thread's 32 columns of its row, BF16, into a K-major tile; v becomes the rounded values
+  // this thread's 32 columns of its row, BF16, into a K-major tile
   auto store = [&](uint8_t* T) {
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
-      const uint4 q = packBf16x8(v + 8 * h);
-      const __nv_bfloat162* qb = (const __nv_bfloat162*)&q;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = __bfloat1622float2(qb[e]);
-        v[8 * h + 2 * e] = f.x;
-        v[8 * h + 2 * e + 1] = f.y;
-      }
       const int c = (n0 >> 3) + h;
-      *(uint4*)(T + (c >> 3) * 16384 + swizzledChunk(row, c & 7)) = q;
+      *(uint4*)(T + (c >> 3) * 16384 + swizzledChunk(row, c & 7)) = packBf16x8(v + 8 * h);
+    }
+  };
+  // v = gelu(v + b), and v *= gelu'(the accumulator + b)
+  auto activate = [&](const float* b) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v2[j] = geluF2(__fadd2_rn(v2[j], ((const float2*)b)[j]));
+  };
+  auto derive = [&](const float* b) {
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      __align__(8) float z[16];
+      tmemLoad16(myAcc + 16 * half, z);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float2 g = geluGrad2(__fadd2_rn(((const float2*)z)[j], ((const float2*)b)[8 * half + j]));
+        v2[8 * half + j] = __fmul2_rn(v2[8 * half + j], g);
+      }
     }
   };
 
-  const int64_t tiles = (n + 127) / 128;
-  bool more = false;
-  for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-    const int64_t m = t * 128 + row;
-    // features -> BF16, 16-byte chunks of the swizzled tile (rows past the batch: zeros)
+  // features -> BF16, 16-byte chunks of the swizzled tile (rows past the batch: zeros)
+  auto features = [&](int64_t t, uint8_t* T) {
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       const int p = tid + q * kTrainThreads, pr = p >> 3, pc = p & 7;
       const int64_t mr = t * 128 + pr;
-      float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      __align__(16) float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       if (mr < n) {
         const float* src = X + rows(mr) * kIn + pc * 8;
         if (xVec) {
@@ -678,19 +701,29 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
           for (int e = 0; e < 8; ++e) f[e] = src[e];
         }
       }
-      *(uint4*)(sX + swizzledChunk(pr, pc)) = packBf16x8(f);
+      *(uint4*)(T + swizzledChunk(pr, pc)) = packBf16x8(f);
     }
+  };
+
+  const int64_t tiles = (n + 127) / 128;
+  bool more = false;
+  features(blockIdx.x, sX);
+  begin();
+  if (tid == 0) {
+    layer(sX, sW1, 1);
+    commit(bar);
+  }
+  int cur = 0;
+  for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const int64_t m = t * 128 + row;
+    const uint8_t* sXt = sX + cur * 16384;
+    uint8_t* sXn = sX + (cur ^ 1) * 16384;
+    const bool next = t + gridDim.x < tiles;
     const float target = grp == 0 && m < n ? y[rows(m)] : 0.0f;
-    // forward
-    begin();
-    if (tid == 0) {
-      layer(sX, sW1, 1);
-      commit(bar);
-    }
+    // forward (the first layer's product is under way)
     wait();
     tmemLoad32(myAcc, v);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = geluF(v[j] + b1[j]);
+    activate(b1);
     store(sH1);
     begin();
     if (tid == 0) {
@@ -699,22 +732,25 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     }
     wait();
     tmemLoad32(myAcc, v);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = geluF(v[j] + b2[j]);
+    activate(b2);
     store(sH2);
     begin();
     if (tid == 0) {
       layer(sH2, sW3, 2);
       commit(bar);
     }
-    wait();
-    tmemLoad32(myAcc, z);
+    wait();  // with it the previous tile's dW1: its features and dZ1 have been read
+    if (next) features(t + gridDim.x, sXn);
+    tmemLoad32(myAcc, v);
     float o = 0.0f;
+    __nv_bfloat162 h3[16];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      z[j] += b3[j];
-      v[j] = __bfloat162float(__float2bfloat16_rn(geluF(z[j])));
-      o += v[j] * w4[j];
+    for (int j = 0; j < 16; ++j) {
+      v2[j] = __fadd2_rn(v2[j], ((const float2*)b3)[j]);
+      h3[j] = __float22bfloat162_rn(geluF2(v2[j]));
+      const float2 p = __fmul2_rn(__bfloat1622float2(h3[j]), ((const float2*)w4)[j]);
+      o += p.x;
+      o += p.y;
     }
     sPart[grp * 128 + row] = o;
     __syncthreads();
@@ -734,126 +770,140 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     }
     __syncthreads();
     const float d = sRow[row];
+    const float2 d2 = make_float2(d, d);
+    // backward: dZ3 and dH2; Z2 again, with dW3 behind it, dZ2 and dH1; Z1 again, with dW2 behind it,
+    // dZ1; dW1, with the next tile's first layer behind it
 #pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] *= d;
-    gW4 += columnSum(v, lane);
-    // backward: dZ3, then dH2 and dW3; Z2 again, dZ2, dH1 and dW2; Z1 again, dZ1 and dW1
-#pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = d * w4[j] * geluGrad(z[j]);
+    for (int j = 0; j < 16; ++j)
+      v2[j] = __fmul2_rn(__fmul2_rn(d2, ((const float2*)w4)[j]), geluGrad2(v2[j]));
     store(sD);
-    gB3 += columnSum(v, lane);
     begin();
     if (tid == 0) {
       back(sW3);
       commit(bar);
-      weights(dW3, sH2, idMM, more);
     }
+    // the output weights' gradient while the product runs
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v2[j] = __fmul2_rn(__bfloat1622float2(h3[j]), d2);
+    gW4 += columnSum(v, lane);
     wait();
     tmemLoad32(myAcc, v);
     begin();
     if (tid == 0) {
       layer(sH1, sW2, 2);
-      commit(bar);  // with it dW3's products: dZ3 has been read
+      commit(bar);
+      weights(dW3, sH2, idMM, dB + 32, more);
+      commit(barD);
     }
     wait();
-    tmemLoad32(myAcc, z);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] *= geluGrad(z[j] + b2[j]);
+    derive(b2);
+    waitD();
     store(sD);
-    gB2 += columnSum(v, lane);
     begin();
     if (tid == 0) {
       back(sW2);
       commit(bar);
-      weights(dW2, sH1, idMM, more);
     }
     wait();
     tmemLoad32(myAcc, v);
     begin();
     if (tid == 0) {
-      layer(sX, sW1, 1);
+      layer(sXt, sW1, 1);
       commit(bar);
+      weights(dW2, sH1, idMM, dB + 16, more);
+      commit(barD);
     }
     wait();
-    tmemLoad32(myAcc, z);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] *= geluGrad(z[j] + b1[j]);
+    derive(b1);
+    waitD();
     store(sD);
-    gB1 += columnSum(v, lane);
     begin();
     if (tid == 0) {
-      weights(dW1, sX, idMM64, more);
+      weights(dW1, sXt, idMM64, dB, more);
+      if (next) layer(sXn, sW1, 1);
       commit(bar);
     }
-    wait();  // X and dZ1 have been read: the next tile's may come
     more = true;
+    cur ^= 1;
   }
+  wait();  // the last tile's dW1
   // the CTA's sums: weight gradients (row o of this thread), then the columns' and rows' sums
   float* out = part + (int64_t)blockIdx.x * kPartStride;
+  // (four columns of all rows after one another, so that a warp's stores are contiguous)
   tmemLoad32(dW3 + tl + (uint32_t)n0, v);
 #pragma unroll
-  for (int j = 0; j < 32; j += 4) *(float4*)(out + kOffW3 + row * kHid + n0 + j) = *(const float4*)(v + j);
+  for (int j = 0; j < 32; j += 4)
+    *(float4*)(out + kOffW3 + (n0 + j) * 128 + row * 4) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
   tmemLoad32(dW2 + tl + (uint32_t)n0, v);
 #pragma unroll
-  for (int j = 0; j < 32; j += 4) *(float4*)(out + kOffW2 + row * kHid + n0 + j) = *(const float4*)(v + j);
+  for (int j = 0; j < 32; j += 4)
+    *(float4*)(out + kOffW2 + (n0 + j) * 128 + row * 4) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
   {
     float u[16];
     tmemLoad16(dW1 + tl + (uint32_t)(16 * grp), u);
 #pragma unroll
-    for (int j = 0; j < 16; j += 4) *(float4*)(out + kOffW1 + row * kIn + 16 * grp + j) = *(const float4*)(u + j);
+    for (int j = 0; j < 16; j += 4)
+      *(float4*)(out + kOffW1 + (16 * grp + j) * 128 + row * 4) = make_float4(u[j], u[j + 1], u[j + 2], u[j + 3]);
   }
-  float* sums = (float*)sX;  // [warp of 32 rows][4][128 columns], then two per warp of group 0
-  const int col = n0 + lane, quarter = warp & 3;
-  sums[(quarter * 4 + 0) * 128 + col] = gB1;
-  sums[(quarter * 4 + 1) * 128 + col] = gB2;
-  sums[(quarter * 4 + 2) * 128 + col] = gB3;
-  sums[(quarter * 4 + 3) * 128 + col] = gW4;
+  if (grp < 3) {  // the bias gradients: each of the 16 columns holds them
+    float u[16];
+    tmemLoad16(dB + tl + (uint32_t)(16 * grp), u);
+    out[(grp == 0 ? kOffB1 : grp == 1 ? kOffB2 : kOffB3) + row] = u[0];
+  }
+  float* sums = (float*)sX;  // [quarter of the rows][128 columns], then two per warp of group 0
+  sums[(warp & 3) * 128 + n0 + lane] = gW4;
   if (grp == 0) {
     for (int o = 16; o > 0; o >>= 1) {
       gB4 += __shfl_down_sync(0xffffffffu, gB4, o);
       sq += __shfl_down_sync(0xffffffffu, sq, o);
     }
     if (lane == 0) {
-      sums[16 * 128 + 2 * warp] = gB4;
-      sums[16 * 128 + 2 * warp + 1] = sq;
+      sums[4 * 128 + 2 * warp] = gB4;
+      sums[4 * 128 + 2 * warp + 1] = sq;
     }
   }
   fenceBefore();
   __syncthreads();
   if (warp == 0) tmemFree(*tslot, 512);
-  const int64_t off[4] = {kOffB1, kOffB2, kOffB3, kOffW4};
-  {
-    float s = 0.0f;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) s += sums[(q * 4 + grp) * 128 + row];
-    out[(grp == 0 ? off[0] : grp == 1 ? off[1] : grp == 2 ? off[2] : off[3]) + row] = s;
-  }
+  if (grp == 0) out[kOffW4 + row] = ((sums[row] + sums[128 + row]) + sums[256 + row]) + sums[384 + row];
   if (tid < 2) {
     float s = 0.0f;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) s += sums[16 * 128 + 2 * q + tid];
+    for (int q = 0; q < 4; ++q) s += sums[4 * 128 + 2 * q + tid];
     out[tid == 0 ? kOffB4 : kNumParams] = s;
   }
   if (!ok) atomicExch(err, 1);
 }
 
-// The CTAs' sums added in CTA order: the gradient, and the mean squared error.
-__global__ void __launch_bounds__(128) kSumPartials(const float* __restrict__ part, int ctas, int64_t n,
-                                                    float* __restrict__ grad, float* __restrict__ loss) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i > kNumParams) return;
+// The CTAs' sums added in CTA order, in four runs that are then added in order: the gradient, and the
+// mean squared error behind it. A block takes 64 values of the slots, a quarter of the CTAs per warp pair.
+__global__ void __launch_bounds__(256) kSumPartials(const float* __restrict__ part, int ctas, int64_t n,
+                                                    float* __restrict__ grad) {
+  __shared__ float sRun[4][64];
+  const int64_t i = blockIdx.x * 64ll + (threadIdx.x & 63);
+  const int run = threadIdx.x >> 6, per = (ctas + 3) / 4, c1 = min(ctas, (run + 1) * per);
   float s = 0.0f;
-  int c = 0;
-  for (; c + 8 <= ctas; c += 8) {
-    float p[8];
+  if (i <= kNumParams) {
+    int c = run * per;
+    for (; c + 16 <= c1; c += 16) {
+      float p[16];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) p[k] = part[(int64_t)(c + k) * kPartStride + i];
+      for (int k = 0; k < 16; ++k) p[k] = part[(int64_t)(c + k) * kPartStride + i];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) s += p[k];
+      for (int k = 0; k < 16; ++k) s += p[k];
+    }
+    for (; c < c1; ++c) s += part[(int64_t)c * kPartStride + i];
   }
-  for (; c < ctas; ++c) s += part[(int64_t)c * kPartStride + i];
-  if (i < kNumParams) grad[i] = s;
-  else loss[0] = s / (float)n;
+  sRun[run][threadIdx.x & 63] = s;
+  __syncthreads();
+  if (run > 0 || i > kNumParams) return;
+  s = ((sRun[0][threadIdx.x] + sRun[1][threadIdx.x]) + sRun[2][threadIdx.x]) + sRun[3][threadIdx.x];
+  int64_t to = i;
+  for (int l = 0; l < 3; ++l) {  // the weights' slots run four columns at a time: back to row-major
+    const int64_t off = l == 0 ? kOffW1 : l == 1 ? kOffW2 : kOffW3, cols = l == 0 ? kIn : kHid, e = i - off;
+    if (e >= 0 && e < kHid * cols) to = off + ((e & 511) >> 2) * cols + (e >> 9) * 4 + (e & 3);
+  }
+  grad[to] = i < kNumParams ? s : s / (float)n;
 }
 
 // Adam (Kingma & Ba): m = b1 m + (1-b1) g; v = b2 v + (1-b2) g^2; p -= lr mhat / (sqrt(vhat) + eps).
@@ -897,8 +947,9 @@ struct its_mlp {
   float* P = nullptr;
   float* Mo = nullptr;
   float* Ve = nullptr;
-  float* G = nullptr;
-  float* loss = nullptr;
+  float* G = nullptr;     // the gradient; behind it the mean squared error and the error flag
+  float* loss = nullptr;  // behind the gradient
+  float* host = nullptr;  // page-locked: the gradient and the two words behind it
   int64_t step = 0;
   bf16 *W1, *W2, *W3;
   float* w4r;
@@ -946,7 +997,7 @@ static its_status mlpGradient(its_mlp* h, const float* X, const float* y, const 
   kMlpGradientFused<<<ctas, kTrainThreads, kTrainSmem, ctx->stream>>>(X, y, rows, n, 2.0f / (float)n, h->img, h->P,
                                                                      h->part, h->err);
   ITS_LAUNCHED(ctx);
-  kSumPartials<<<gridFor(kNumParams + 1, 128), 128, 0, ctx->stream>>>(h->part, ctas, n, h->G, h->loss);
+  kSumPartials<<<gridFor(kNumParams + 1, 64), 256, 0, ctx->stream>>>(h->part, ctas, n, h->G);
   ITS_LAUNCHED(ctx);
   return ITS_OK;
 }
@@ -1015,13 +1066,19 @@ its_status its_mlp_create(its_ctx* ctx, int64_t batch, its_mlp** out) {
   auto A = [&](auto** p, int64_t c) {
     if (s == ITS_OK) s = h->alloc(p, c);
   };
-  A(&h->P, kNumParams); A(&h->Mo, kNumParams); A(&h->Ve, kNumParams); A(&h->G, kNumParams); A(&h->loss, 1);
+  A(&h->P, kNumParams); A(&h->Mo, kNumParams); A(&h->Ve, kNumParams); A(&h->G, kNumParams + 2);
   A(&h->W1, kHid * kIn); A(&h->W2, kHid * kHid); A(&h->W3, kHid * kHid); A(&h->w4r, kHid); A(&h->img, kImgBytes);
-  A(&h->Xb, B * kIn); A(&h->H1, B * kHid); A(&h->H2, B * kHid); A(&h->part, ctx->numSMs * kPartStride); A(&h->err, 1);
+  A(&h->Xb, B * kIn); A(&h->H1, B * kHid); A(&h->H2, B * kHid); A(&h->part, ctx->numSMs * kPartStride);
   if (s != ITS_OK) {
     for (void* p : h->allocs) devFree(ctx, p);
     delete h;
     return s;
+  }
+  h->loss = h->G + kNumParams;
+  h->err = (int*)(h->G + kNumParams + 1);
+  if (cudaMallocHost((void**)&h->host, (kNumParams + 2) * 4) != cudaSuccess) {
+    cudaGetLastError();
+    h->host = nullptr;  // gradients then go to the caller's memory directly
   }
   cudaMemsetAsync(h->P, 0, kNumParams * 4, ctx->stream);
   cudaMemsetAsync(h->Mo, 0, kNumParams * 4, ctx->stream);
@@ -1039,6 +1096,7 @@ its_status its_mlp_free(its_mlp* h) {
   if (!h) return ITS_ERR_INVALID;
   cudaStreamSynchronize(h->ctx->stream);
   for (void* p : h->allocs) devFree(h->ctx, p);
+  if (h->host) cudaFreeHost(h->host);
   delete h;
   return ITS_OK;
 }
@@ -1139,6 +1197,17 @@ its_status its_mlp_gradient(its_mlp* h, const float* X, const float* y, int64_t 
   if ((st = x.stage(ctx, X, n * kIn)) != ITS_OK) return st;
   if ((st = yy.stage(ctx, y, n)) != ITS_OK) return st;
   if ((st = mlpGradient(h, x.d, yy.d, BatchRows{0, 0, 0}, n)) != ITS_OK) return st;
+  if (h->host && ptrClass(grad, ctx->device) == PtrClass::Pageable &&
+      (!loss || ptrClass(loss, ctx->device) == PtrClass::Pageable)) {
+    // one copy for the gradient, the loss and the flag (three to pageable memory took 40 us)
+    ITS_CU(ctx, cudaMemcpyAsync(h->host, h->G, (kNumParams + 2) * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    ITS_CU(ctx, cudaStreamSynchronize(ctx->stream));
+    std::memcpy(grad, h->host, kNumParams * 4);
+    if (loss) *loss = h->host[kNumParams];
+    int e;
+    std::memcpy(&e, h->host + kNumParams + 1, 4);
+    return e ? setError(ctx, ITS_ERR_TIMEOUT, "share network: a tensor-core wait ran out") : ITS_OK;
+  }
   ITS_CU(ctx, cudaMemcpyAsync(grad, h->G, kNumParams * 4, cudaMemcpyDefault, ctx->stream));
   if (loss) ITS_CU(ctx, cudaMemcpyAsync(loss, h->loss, 4, cudaMemcpyDefault, ctx->stream));
   return checkErr(h);
