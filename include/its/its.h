@@ -379,7 +379,7 @@ its_status its_mlp_forward_async(its_mlp* mlp, const float* features, int64_t n,
 its_status its_mlp_forward_tiles_async(its_mlp* mlp, const void* tiles, int64_t n, float* out, int after_kernel);
 /* Waits for the context's stream; ITS_ERR_TIMEOUT if a network kernel's bounded wait ran out. */
 its_status its_mlp_check(its_mlp* mlp);
-/* The same predictions layer by layer through the training kernels (bit-identical). */
+/* The same predictions layer by layer (bit-identical). */
 its_status its_mlp_forward_layers(its_mlp* mlp, const float* features, int64_t n, float* out);
 /* Gradient of mean((out - y)^2) over n rows (n <= batch, a multiple of 64), no update. */
 its_status its_mlp_gradient(its_mlp* mlp, const float* features, const float* y, int64_t n, float* grad,

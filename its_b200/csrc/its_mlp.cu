@@ -1165,7 +1165,7 @@ its_status its_mlp_check(its_mlp* h) {
   return checkErr(h);
 }
 
-// The same predictions layer by layer (the training kernels' forward); identical to
+// The same predictions layer by layer; identical to
 // its_mlp_forward bit for bit (a test hook).
 its_status its_mlp_forward_layers(its_mlp* h, const float* X, int64_t n, float* out) {
   if (!h || (n > 0 && (!X || !out)) || n < 0) return ITS_ERR_INVALID;
