@@ -16,77 +16,120 @@
 // differ from the reference's by rounding only: the hats are centred on the exact lattice
 // positions, the representative vertex positions of the octree differ from them by ulps.
 #include <cmath>
-#include <vector>
 
 #include "its_op.cuh"
 #include "its_svo.cuh"
 
 namespace its {
 
+// Depth d's dense lattice: its first point and its points per axis.
+template <typename T>
+struct CascadeLevels {
+  T* field[kMaxDepth];
+  int M[kMaxDepth];
+};
+
 template <typename T>
 __global__ void kScatterCorners(int64_t n, const uint64_t* __restrict__ vertKey, const double* __restrict__ lambda,
-                                const int64_t* __restrict__ off, const int64_t* __restrict__ Ms, T* __restrict__ D) {
+                                CascadeLevels<T> L) {
   const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (v >= n) return;
   const VertCoord c = decodeVertKey(vertKey[v]);
-  const int64_t M = Ms[c.d];
-  D[off[c.d] + c.X + M * (c.Y + M * (int64_t)c.Z)] = (T)lambda[v];
+  const int64_t M = L.M[c.d];
+  L.field[c.d][c.X + M * (c.Y + M * (int64_t)c.Z)] = (T)lambda[v];
 }
 
-// fine = (accumulate ? fine : 0) + the trilinear prolongation of coarse by the factor 2^s
-// (fine has Mf = (Mc - 1) 2^s + 1 points per axis, x fastest). One thread per coarse x
-// interval and fine (y, z): it reads the interval's ends on the <= 4 coarse rows around
-// (y, z) and writes the 2^s fine points of the interval (the last coarse point: one), so a
-// warp's stores are contiguous. Blocks of 32 intervals x 8 fine rows; z per block.
-template <typename T, int S>
-__global__ void __launch_bounds__(256) kProlong(const T* __restrict__ coarse, int Mc, T* __restrict__ fine,
-                                                int accumulate) {
-  constexpr int F = 1 << S;
+// fine = (kAdd ? fine : 0) + the trilinear prolongation of coarse by the factor 2^S (fine has
+// Mf = (Mc - 1) 2^S + 1 points per axis, x fastest). A thread has one fine x and one coarse y
+// interval and walks up `cells` coarse z intervals, 2^S x 2^S points each; the next plane of the
+// coarse field, and the next old values, are on their way meanwhile. Threads run along the rows and
+// on into the next interval's, so that a block's stores are runs of 256 points: bound by the writes.
+// A thread per coarse x interval and fine (y, z) stored every 2^S-th point and read a cell's
+// corners 18 times for the 8 points of S = 1; whole FP64 fields of 513 points per axis from 65, 129,
+// 257 and 513: 612, 532, 526 and 942 us before, 221, 213, 335 and 685 now (1.08 GB: 166 us).
+template <typename T, int S, bool kAdd>
+__global__ void __launch_bounds__(256) kProlong(const T* coarse, int Mc, T* fine, int cells) {
+  constexpr int F = 1 << S, kOld = kAdd ? F * F : 1;
   const int Mf = (Mc - 1) * F + 1;
-  const int xc = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y, z = blockIdx.z;
-  if (xc >= Mc || y >= Mf) return;
-  const int ry = y & (F - 1), rz = z & (F - 1);
-  const int cy = y >> S, cz = z >> S;
-  const T wy1 = (T)ry / (T)F, wz1 = (T)rz / (T)F;  // exact: F is a power of two
-  const bool xr = xc + 1 < Mc;                       // the interval has a right end
-  const T* base = coarse + ((int64_t)cz * Mc + cy) * Mc + xc;
-  const int64_t rowY = Mc, rowZ = (int64_t)Mc * Mc;
-  // the coarse field at x = xc and xc + 1, interpolated in y and z
-  T a0 = base[0], a1 = xr ? base[1] : T(0);
-  if (ry) {
-    a0 = (T(1) - wy1) * a0 + wy1 * base[rowY];
-    if (xr) a1 = (T(1) - wy1) * a1 + wy1 * base[rowY + 1];
-  }
-  if (rz) {
-    T b0 = base[rowZ], b1 = xr ? base[rowZ + 1] : T(0);
-    if (ry) {
-      b0 = (T(1) - wy1) * b0 + wy1 * base[rowZ + rowY];
-      if (xr) b1 = (T(1) - wy1) * b1 + wy1 * base[rowZ + rowY + 1];
-    }
-    a0 = (T(1) - wz1) * a0 + wz1 * b0;
-    a1 = (T(1) - wz1) * a1 + wz1 * b1;
-  }
-  T* out = fine + ((int64_t)z * Mf + y) * Mf + (int64_t)xc * F;
+  const unsigned column = blockIdx.x * 256 + threadIdx.x;
+  const int yc = column / (unsigned)Mf, x = column - yc * Mf;
+  const int zBegin = blockIdx.y * cells, zEnd = min(zBegin + cells, Mc);  // the last has one plane only
+  gridDependencyWait();
+  gridDependents();
+  if (yc >= Mc) return;
+  const int rx = x & (F - 1);
+  const bool xr = rx != 0, yr = yc + 1 < Mc;
+  const T wx1 = (T)rx / (T)F;  // exact: F is a power of two
+  const int64_t outY = Mf, outZ = (int64_t)Mf * Mf, rowZ = (int64_t)Mc * Mc;
+  const T* plane = coarse + (zBegin * rowZ + (int64_t)yc * Mc + (x >> S));
+  T* out = fine + ((int64_t)zBegin * F * Mf + yc * F) * Mf + x;
+  T lo[4], hi[4], up[4], old[kOld], oldUp[kOld];
+  // corner x | y << 1 of a plane, where a point of the thread's takes it
+  auto corners = [&](T (&c)[4], const T* p, bool in) {
 #pragma unroll
-  for (int r = 0; r < F; ++r) {
-    if (r > 0 && !xr) break;
-    const T w1 = (T)r / (T)F;
-    const T v = r ? (T(1) - w1) * a0 + w1 * a1 : a0;
-    out[r] = accumulate ? out[r] + v : v;
+    for (int k = 0; k < 4; ++k)
+      c[k] = in && ((k & 1) == 0 || xr) && ((k & 2) == 0 || yr) ? p[(k & 1) + (k & 2 ? Mc : 0)] : T(0);
+  };
+  auto olds = [&](T (&o)[kOld], const T* p, int cz) {
+    if constexpr (kAdd) {
+#pragma unroll
+      for (int k = 0; k < F * F; ++k)
+        o[k] = (k % F == 0 || yr) && cz < Mc && (k < F || cz + 1 < Mc) ? p[(k % F) * outY + (k / F) * outZ] : T(0);
+    }
+  };
+  corners(lo, plane, true);
+  corners(hi, plane + rowZ, zBegin + 1 < Mc);
+  olds(old, out, zBegin);
+  for (int cz = zBegin; cz < zEnd; ++cz) {
+    const bool more = cz + 1 < zEnd;
+    corners(up, plane + 2 * rowZ, more && cz + 2 < Mc);
+    olds(oldUp, out + F * outZ, more ? cz + 1 : Mc);
+#pragma unroll
+    for (int k = 0; k < F * F; ++k) {
+      const int ry = k % F, rz = k / F;
+      if ((ry > 0 && !yr) || (rz > 0 && cz + 1 >= Mc)) continue;
+      const T wy1 = (T)ry / (T)F, wz1 = (T)rz / (T)F;
+      // the field at the x interval's ends, interpolated in y and z
+      T a0 = lo[0], a1 = lo[1];
+      if (ry) {
+        a0 = (T(1) - wy1) * a0 + wy1 * lo[2];
+        a1 = (T(1) - wy1) * a1 + wy1 * lo[3];
+      }
+      if (rz) {
+        T b0 = hi[0], b1 = hi[1];
+        if (ry) {
+          b0 = (T(1) - wy1) * b0 + wy1 * hi[2];
+          b1 = (T(1) - wy1) * b1 + wy1 * hi[3];
+        }
+        a0 = (T(1) - wz1) * a0 + wz1 * b0;
+        a1 = (T(1) - wz1) * a1 + wz1 * b1;
+      }
+      const T v = xr ? (T(1) - wx1) * a0 + wx1 * a1 : a0;
+      out[ry * outY + rz * outZ] = kAdd ? old[kAdd ? k : 0] + v : v;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      lo[k] = hi[k];
+      hi[k] = up[k];
+    }
+#pragma unroll
+    for (int k = 0; k < kOld; ++k) old[k] = oldUp[k];
+    plane += rowZ;
+    out += F * outZ;
   }
 }
 
-template <typename T>
-static its_status prolong(its_ctx* ctx, const T* coarse, int64_t Mc, T* fine, int s, int accumulate) {
-  const int64_t Mf = (Mc - 1) * ((int64_t)1 << s) + 1;
-  const dim3 grid((unsigned)((Mc + 31) / 32), (unsigned)((Mf + 7) / 8), (unsigned)Mf), block(32, 8);
-  switch (s) {
-    case 1: kProlong<T, 1><<<grid, block, 0, ctx->stream>>>(coarse, (int)Mc, fine, accumulate); break;
-    case 2: kProlong<T, 2><<<grid, block, 0, ctx->stream>>>(coarse, (int)Mc, fine, accumulate); break;
-    default: kProlong<T, 3><<<grid, block, 0, ctx->stream>>>(coarse, (int)Mc, fine, accumulate); break;
-  }
-  ITS_LAUNCHED(ctx);
-  return ITS_OK;
+// dependent: the previous operation in the stream is a kernel. A walk is as long as leaves the
+// chip ten thousand threads per SM, several rounds, and at most 32 rows: longer ones write too
+// many places at once (257 -> 513 points per axis, the whole field: 434, 370, 351, 335 us for
+// 1, 2, 4, 8 intervals and 387 for 16; 129 -> 513: 224, 214, 230 for 1, 2, 4).
+template <typename T, int S, bool kAdd>
+static its_status prolong(its_ctx* ctx, bool dependent, const T* coarse, int Mc, T* fine) {
+  const int64_t Mf = (int64_t)(Mc - 1) * (1 << S) + 1, columns = Mf * Mc, kMost = S == 1 ? 8 : S == 2 ? 2 : 1;
+  const int cells = (int)std::min<int64_t>(std::max<int64_t>(columns * Mc / (ctx->numSMs * 10240), 1), kMost);
+  const dim3 grid((unsigned)((columns + 255) / 256), (unsigned)((Mc + cells - 1) / cells));
+  return launchDependent(ctx, dependent, kProlong<T, S, kAdd>, grid, 256, 0, ctx->stream, coarse, Mc, fine,
+                         cells);
 }
 
 // Whether the lattice (origin, width, res) is the octree's box at res_octree * 2^s points: per
@@ -110,46 +153,35 @@ template <typename T>
 static its_status cascade(its_ctx* ctx, const SvoDevice& d, const double* lambda, int res, int s, T* out) {
   its_status st;
   const int D = d.depth;
-  std::vector<int64_t> M(D), off(D + 1, 0);
-  for (int k = 0; k < D; ++k) {
-    M[k] = (int64_t)(d.res >> k) + 1;
-    off[k + 1] = off[k] + M[k] * M[k] * M[k];
-  }
+  CascadeLevels<T> L = {};
   // with s == 0 the output is depth 0's lattice itself
-  const int64_t inner = s == 0 ? off[D] - off[1] : off[D];
-  DevBuf<T> lat;
-  DevBuf<int64_t> tab;
-  if ((st = lat.alloc(ctx, std::max<int64_t>(inner, 1))) != ITS_OK || (st = tab.alloc(ctx, 2 * (D + 1))) != ITS_OK)
-    return st;
-  std::vector<int64_t> h(2 * (D + 1), 0);
-  for (int k = 0; k < D; ++k) h[k] = M[k];
-  for (int k = 0; k < D; ++k) h[D + 1 + k] = s == 0 ? (k == 0 ? 0 : off[k] - off[1]) : off[k];
-  ITS_CU(ctx, cudaMemcpyAsync(tab.p, h.data(), h.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
-  auto level = [&](int k) -> T* { return s == 0 ? (k == 0 ? out : lat.p + (off[k] - off[1])) : lat.p + off[k]; };
-  ITS_CU(ctx, cudaMemsetAsync(lat.p, 0, std::max<int64_t>(inner, 1) * sizeof(T), ctx->stream));
-  if (s == 0) ITS_CU(ctx, cudaMemsetAsync(out, 0, M[0] * M[0] * M[0] * sizeof(T), ctx->stream));
-  if (d.numVerts > 0) {
-    if (s == 0) {
-      // depth 0 goes to the output, the rest to the scratch lattices (offsets already shifted)
-      kScatterCorners<T><<<gridFor(d.vertCount[0], 256), 256, 0, ctx->stream>>>(d.vertCount[0], d.vertKey, lambda,
-                                                                               tab.p + D + 1, tab.p, out);
-      ITS_LAUNCHED(ctx);
-      const int64_t rest = d.numVerts - d.vertStart[1 < D ? 1 : D];
-      if (rest > 0) {
-        kScatterCorners<T><<<gridFor(rest, 256), 256, 0, ctx->stream>>>(rest, d.vertKey + d.vertStart[1], lambda +
-                                                                         d.vertStart[1], tab.p + D + 1, tab.p, lat.p);
-        ITS_LAUNCHED(ctx);
-      }
-    } else {
-      kScatterCorners<T><<<gridFor(d.numVerts, 256), 256, 0, ctx->stream>>>(d.numVerts, d.vertKey, lambda,
-                                                                           tab.p + D + 1, tab.p, lat.p);
-      ITS_LAUNCHED(ctx);
-    }
+  int64_t inner = 0;
+  for (int k = 0; k < D; ++k) {
+    L.M[k] = (d.res >> k) + 1;
+    if (k > 0 || s > 0) inner += (int64_t)L.M[k] * L.M[k] * L.M[k];
   }
-  for (int k = D - 2; k >= 0; --k)
-    if ((st = prolong<T>(ctx, level(k + 1), M[k + 1], level(k), 1, 1)) != ITS_OK) return st;
-  if (s > 0 && (st = prolong<T>(ctx, level(0), M[0], out, s, 0)) != ITS_OK) return st;
-  return ITS_OK;
+  DevBuf<T> lat;
+  if ((st = lat.alloc(ctx, std::max<int64_t>(inner, 1))) != ITS_OK) return st;
+  T* next = lat.p;
+  for (int k = 0; k < D; ++k) {
+    L.field[k] = k == 0 && s == 0 ? out : next;
+    if (k > 0 || s > 0) next += (int64_t)L.M[k] * L.M[k] * L.M[k];
+  }
+  ITS_CU(ctx, cudaMemsetAsync(lat.p, 0, std::max<int64_t>(inner, 1) * sizeof(T), ctx->stream));
+  if (s == 0) ITS_CU(ctx, cudaMemsetAsync(out, 0, (int64_t)L.M[0] * L.M[0] * L.M[0] * sizeof(T), ctx->stream));
+  if (d.numVerts > 0) {
+    kScatterCorners<T><<<gridFor(d.numVerts, 256), 256, 0, ctx->stream>>>(d.numVerts, d.vertKey, lambda, L);
+    ITS_LAUNCHED(ctx);
+  }
+  bool kernelBefore = d.numVerts > 0;
+  for (int k = D - 2; k >= 0; --k, kernelBefore = true)
+    if ((st = prolong<T, 1, true>(ctx, kernelBefore, L.field[k + 1], L.M[k + 1], L.field[k])) != ITS_OK) return st;
+  switch (s) {
+    case 0: return ITS_OK;
+    case 1: return prolong<T, 1, false>(ctx, kernelBefore, L.field[0], L.M[0], out);
+    case 2: return prolong<T, 2, false>(ctx, kernelBefore, L.field[0], L.M[0], out);
+    default: return prolong<T, 3, false>(ctx, kernelBefore, L.field[0], L.M[0], out);
+  }
 }
 
 template <typename T>
