@@ -118,14 +118,19 @@ void releasePlan(its_ctx* ctx, SpmvPlan* P) {
 // so that it leaves in runs. (Ranked round by round across the block, with four barriers a round,
 // the scatter took 20 us for 196,681 pairs, in 48 tiles; 10^7 pairs take the same 64 us, bound by
 // the 64-byte runs that go to 256 places.)
+//
+// The launches are dependent. A scatter ranks its keys while the counts are scanned: the keys were
+// complete before the counting grid, which lets the scan start only after its own wait.
 constexpr int kRsThreads = 256, kRsWarps = kRsThreads / 32;
 
 template <int ITEMS>
-__global__ void __launch_bounds__(kRsThreads) kRadixUpsweep(const uint32_t* __restrict__ keys, int64_t n, int shift,
-                                                            uint32_t* __restrict__ tileHist, int64_t nb) {
+__global__ void __launch_bounds__(kRsThreads) kRadixUpsweep(const uint32_t* keys, int64_t n, int shift, uint32_t* tileHist,
+                                                            int64_t nb) {
   __shared__ uint32_t hist[kRsWarps / 2][256];  // a copy per warp pair: equal digits meet less often
   const int warp = threadIdx.x >> 5;
   for (int w = 0; w < kRsWarps / 2; ++w) hist[w][threadIdx.x] = 0;
+  gridDependencyWait();
+  gridDependents();
   const int64_t base = (int64_t)blockIdx.x * (kRsThreads * ITEMS) + threadIdx.x;
   uint32_t key[ITEMS];
 #pragma unroll
@@ -145,10 +150,11 @@ __global__ void __launch_bounds__(kRsThreads) kRadixUpsweep(const uint32_t* __re
 }
 
 // Block d: digit d's counts over the tiles, scanned in place; their total to totals[d].
-__global__ void __launch_bounds__(kScanThreads) kRadixScan(uint32_t* __restrict__ tileHist, int64_t nb,
-                                                           uint32_t* __restrict__ totals) {
+__global__ void __launch_bounds__(kScanThreads) kRadixScan(uint32_t* tileHist, int64_t nb, uint32_t* totals) {
   uint32_t* row = tileHist + (int64_t)blockIdx.x * nb;
   uint32_t carry = 0;
+  gridDependents();
+  gridDependencyWait();
   for (int64_t i0 = 0; i0 < nb; i0 += kScanTile) {
     uint32_t v[kScanItems], s = 0;
     const int64_t at = i0 + (int64_t)threadIdx.x * kScanItems;
@@ -171,12 +177,10 @@ __global__ void __launch_bounds__(kScanThreads) kRadixScan(uint32_t* __restrict_
 }
 
 template <int ITEMS>
-__global__ void __launch_bounds__(kRsThreads, 6) kRadixDownsweep(const uint32_t* __restrict__ keys,
-                                                              const uint32_t* __restrict__ vals, int64_t n, int shift,
-                                                              const uint32_t* __restrict__ tileOffsets, int64_t nb,
-                                                              const uint32_t* __restrict__ totals,
-                                                              uint32_t* __restrict__ keysOut,
-                                                              uint32_t* __restrict__ valsOut) {
+__global__ void __launch_bounds__(kRsThreads, 6) kRadixDownsweep(const uint32_t* keys, const uint32_t* vals, int64_t n,
+                                                              int shift, const uint32_t* tileOffsets, int64_t nb,
+                                                              const uint32_t* totals, uint32_t* keysOut,
+                                                              uint32_t* valsOut) {
   static_assert(kRsThreads == 256 && kScanThreads == 256, "a thread per digit");
   __shared__ uint32_t sKey[kRsThreads * ITEMS], sVal[kRsThreads * ITEMS];
   __shared__ uint32_t warpCnt[kRsWarps][256];
@@ -189,7 +193,7 @@ __global__ void __launch_bounds__(kRsThreads, 6) kRadixDownsweep(const uint32_t*
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
     const bool in = mine + 32 * j < n;
-    key[j] = in ? keys[mine + 32 * j] : 0u;
+    key[j] = in ? __ldcg(keys + mine + 32 * j) : 0u;
   }
 #pragma unroll
   for (int w = 0; w < kRsWarps; ++w) warpCnt[w][t] = 0;
@@ -218,6 +222,8 @@ __global__ void __launch_bounds__(kRsThreads, 6) kRadixDownsweep(const uint32_t*
       sum += c;
     }
     const uint32_t first = blockExclusiveScan<uint32_t>(sum, total);
+    gridDependencyWait();
+    gridDependents();
     const uint32_t global = blockExclusiveScan<uint32_t>(totals[t], total) + tileOffsets[(int64_t)t * nb + blockIdx.x];
     sFirst[t] = first;
     sDst[t] = global - first;
@@ -246,13 +252,14 @@ template <int ITEMS>
 static its_status radixPass(its_ctx* ctx, const uint32_t* sk, const uint32_t* sv, uint32_t* dk, uint32_t* dv, int64_t n,
                             int shift, uint32_t* hist, int64_t nb) {
   uint32_t* totals = hist + 256 * nb;
-  kRadixUpsweep<ITEMS><<<(unsigned)nb, kRsThreads, 0, ctx->stream>>>(sk, n, shift, hist, nb);
-  ITS_LAUNCHED(ctx);
-  kRadixScan<<<256, kScanThreads, 0, ctx->stream>>>(hist, nb, totals);
-  ITS_LAUNCHED(ctx);
-  kRadixDownsweep<ITEMS><<<(unsigned)nb, kRsThreads, 0, ctx->stream>>>(sk, sv, n, shift, hist, nb, totals, dk, dv);
-  ITS_LAUNCHED(ctx);
-  return ITS_OK;
+  its_status st;
+  // the first pass's keys may come from a copy
+  if ((st = launchDependent(ctx, shift > 0, kRadixUpsweep<ITEMS>, (unsigned)nb, kRsThreads, 0, ctx->stream, sk, n, shift,
+                            hist, nb)) != ITS_OK ||
+      (st = launchDependent(ctx, true, kRadixScan, 256, kScanThreads, 0, ctx->stream, hist, nb, totals)) != ITS_OK)
+    return st;
+  return launchDependent(ctx, true, kRadixDownsweep<ITEMS>, (unsigned)nb, kRsThreads, 0, ctx->stream, sk, sv, n, shift,
+                         (const uint32_t*)hist, nb, (const uint32_t*)totals, dk, dv);
 }
 
 its_status radixSortPairs(its_ctx* ctx, const uint32_t* keys, const uint32_t* vals, uint32_t* keysOut,
