@@ -328,38 +328,38 @@ __global__ void __launch_bounds__(kUpLeaves) kBottomUp(const double* __restrict_
 
 // The nodes above the blocks' maximal subtrees, a thread per subtree: the first arrival's sums
 // wait at its first leaf's place; a node's place is its left child's, whose sums the merging
-// thread has read by then.
+// thread has read by then. A chain of global round trips, one node after another: a node's links
+// come in while the sums before it go out (131 -> 108 us at 1,048,576 triangles).
 __global__ void __launch_bounds__(128) kClimbTop(BvhDevice B, double* __restrict__ raw, const int2* __restrict__ top,
                                                  const unsigned* __restrict__ topCount, BoxF* __restrict__ box,
                                                  FwnNode* __restrict__ fwn) {
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= *topCount) return;
-  int64_t node = top[k].x, first = top[k].y;
+  int64_t first = top[k].y;
   NodeSums S;
   double* mine = (double*)&S;
 #pragma unroll
   for (int w = 0; w < kSumWords; ++w) mine[w] = raw[kSumWords * first + w];
-  while (true) {
-    const int32_t par = B.parent[node];
-    if (par < 0) return;
+  int32_t par = B.parent[top[k].x];
+  while (par >= 0) {
+    const int32_t r0 = B.range[2 * (int64_t)par], l = B.left[par], r = B.right[par], above = B.parent[par];
     __threadfence();
     if (atomicAdd(B.flag + par, 1u) == 0) return;  // first arrival: the sibling merges
     __threadfence();
-    const int32_t r0 = B.range[2 * (int64_t)par], l = B.left[par], r = B.right[par];
-    const int64_t rFirst = r < 0 ? -(int64_t)r - 1 : B.range[2 * (int64_t)r];
+    const int64_t rFirst = r < 0 ? -(int64_t)r - 1 : r;  // a right child's number is its first leaf's
     const volatile double* src = raw + kSumWords * (first == r0 ? rFirst : (int64_t)r0);
     NodeSums O;
     double* other = (double*)&O;
 #pragma unroll
     for (int w = 0; w < kSumWords; ++w) other[w] = src[w];
     mergeSums(S, O);
-    node = par;
     first = r0;
     volatile double* dst = raw + kSumWords * first;
 #pragma unroll
     for (int w = 0; w < kSumWords; ++w) dst[w] = mine[w];
     box[par] = outwardBox(S);
     fwn[par] = fwnNode(S, l, r);
+    par = above;
   }
 }
 
