@@ -25,15 +25,30 @@
 namespace its {
 
 
+// Bound by latency: a chain of round trips to L2 (the vectors, a block's partial sums and ticket,
+// the last block's sums of them, the scalars). What a round trip does not depend on is read
+// before it: a thread's first two entries and the scalars at once, four partial sums together.
 template <class Op>
 __global__ void __launch_bounds__(kRedThreads) kReduce(Op op, int64_t n, double* partials, CgScalars* S,
                                                        int honorDone) {
   gridDependencyWait();
   gridDependents();
+  const int64_t stride = (int64_t)gridDim.x * kRedThreads;
+  int64_t i = blockIdx.x * (int64_t)kRedThreads + threadIdx.x;
+  typename Op::In v0{}, v1{};
+  if (i < n) v0 = op.load(i);
+  if (i + stride < n) v1 = op.load(i + stride);
+  CgScalars s;  // thread 0's, for the finalize; the tickets are not its
+  if (threadIdx.x == 0) s = *S;
   if (honorDone && S->done) return;
   double a = 0.0, b = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)kRedThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kRedThreads)
-    op.terms(i, a, b);
+  while (i < n) {
+    op.terms(i, v0, a, b);
+    if (i + stride < n) op.terms(i + stride, v1, a, b);
+    i += 2 * stride;
+    if (i < n) v0 = op.load(i);
+    if (i + stride < n) v1 = op.load(i + stride);
+  }
   blockSum2(a, b);
   __shared__ bool last;
   if (threadIdx.x == 0) {
@@ -47,13 +62,35 @@ __global__ void __launch_bounds__(kRedThreads) kReduce(Op op, int64_t n, double*
   if (!last) return;
   __threadfence();
   double ta = 0.0, tb = 0.0;
-  for (unsigned k = threadIdx.x; k < gridDim.x; k += kRedThreads) {
-    ta += ((volatile double*)partials)[2 * k];
-    tb += ((volatile double*)partials)[2 * k + 1];
+  for (unsigned k = threadIdx.x; k < gridDim.x; k += 4 * kRedThreads) {
+    double2 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (k + u * kRedThreads < gridDim.x) v[u] = __ldcg((const double2*)partials + k + u * kRedThreads);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (k + u * kRedThreads < gridDim.x) {
+        ta += v[u].x;
+        tb += v[u].y;
+      }
   }
   blockSum2(ta, tb);
   if (threadIdx.x == 0) {
-    op.finalize(S, ta, tb);
+    op.finalize(&s, ta, tb);
+    S->absNew = s.absNew;
+    S->alpha = s.alpha;
+    S->beta = s.beta;
+    S->tn = s.tn;
+    S->rr = s.rr;
+    S->nrr = s.nrr;
+    S->nrz = s.nrz;
+    S->rhsNorm2 = s.rhsNorm2;
+    S->bNorm2 = s.bNorm2;
+    S->threshold = s.threshold;
+    S->iter = s.iter;
+    S->done = s.done;
+    S->converged = s.converged;
+    S->breakdown = s.breakdown;
     S->tickets[op.slot] = 0;
   }
 }

@@ -34,7 +34,8 @@ __device__ inline void blockSum2(double& a, double& b) {
 }
 
 // Grid reduction with a last-block finalize. Op provides
-//   __device__ void terms(int64_t i, double& a, double& b) const  (may also update vectors)
+//   __device__ In load(int64_t i) const                                 (all that terms reads)
+//   __device__ void terms(int64_t i, const In& v, double& a, double& b) const  (may also update vectors)
 //   __device__ void finalize(CgScalars* S, double a, double b) const
 //   int slot
 
@@ -43,11 +44,15 @@ struct OpInitResidual {  // r = b - t (t = A x0), or r = b
   const double* t;
   double* r;
   int slot = 0;
-  __device__ void terms(int64_t i, double& a, double& c) const {
-    const double v = t ? b[i] - t[i] : b[i];
+  struct In {
+    double b, t;
+  };
+  __device__ In load(int64_t i) const { return {b[i], t ? t[i] : 0.0}; }
+  __device__ void terms(int64_t i, const In& in, double& a, double& c) const {
+    const double v = t ? in.b - in.t : in.b;
     r[i] = v;
-    a += v * v;      // |r|^2
-    c += b[i] * b[i];  // |b|^2
+    a += v * v;        // |r|^2
+    c += in.b * in.b;  // |b|^2
   }
   __device__ void finalize(CgScalars* S, double rr, double bb) const {
     S->rr = rr;
@@ -57,7 +62,9 @@ struct OpInitResidual {  // r = b - t (t = A x0), or r = b
 struct OpRhsNorm {  // |A^T b|^2
   const double* atb;
   int slot = 1;
-  __device__ void terms(int64_t i, double& a, double&) const { a += atb[i] * atb[i]; }
+  using In = double;
+  __device__ In load(int64_t i) const { return atb[i]; }
+  __device__ void terms(int64_t, In v, double& a, double&) const { a += v * v; }
   __device__ void finalize(CgScalars* S, double v, double) const { S->rhsNorm2 = v; }
 };
 struct OpInitNormal {  // |n|^2, n.Dn, decide the zero-iteration exit, p = D n
@@ -66,12 +73,16 @@ struct OpInitNormal {  // |n|^2, n.Dn, decide the zero-iteration exit, p = D n
   double* p;
   float* pf;
   int slot = 2;
-  __device__ void terms(int64_t i, double& a, double& c) const {
-    const double z = invdiag[i] * nr[i];
+  struct In {
+    double nr, d;
+  };
+  __device__ In load(int64_t i) const { return {nr[i], invdiag[i]}; }
+  __device__ void terms(int64_t i, const In& in, double& a, double& c) const {
+    const double z = in.d * in.nr;
     p[i] = z;
     if (pf) pf[i] = (float)z;
-    a += nr[i] * nr[i];
-    c += nr[i] * z;
+    a += in.nr * in.nr;
+    c += in.nr * z;
   }
   __device__ void finalize(CgScalars* S, double nrr, double nrz) const {
     S->nrr = nrr;
@@ -100,7 +111,9 @@ struct OpInitNormal {  // |n|^2, n.Dn, decide the zero-iteration exit, p = D n
 struct OpTmpNorm {
   const double* t;
   int slot = 3;
-  __device__ void terms(int64_t i, double& a, double&) const { a += t[i] * t[i]; }
+  using In = double;
+  __device__ In load(int64_t i) const { return t[i]; }
+  __device__ void terms(int64_t, In v, double& a, double&) const { a += v * v; }
   __device__ void finalize(CgScalars* S, double tn, double) const {
     S->tn = tn;
     if (!(tn > 0.0)) {
@@ -119,10 +132,13 @@ struct OpUpdateXR {
   const double* p;
   const double* t;
   int slot = 4;
-  __device__ void terms(int64_t i, double& a, double&) const {
-    const double al = S->alpha;
-    x[i] += al * p[i];
-    const double v = r[i] - al * t[i];
+  struct In {
+    double al, x, p, r, t;
+  };
+  __device__ In load(int64_t i) const { return {S->alpha, x[i], p[i], r[i], t[i]}; }
+  __device__ void terms(int64_t i, const In& in, double& a, double&) const {
+    x[i] = in.x + in.al * in.p;
+    const double v = in.r - in.al * in.t;
     r[i] = v;
     if (rf) rf[i] = (float)v;
     a += v * v;
@@ -133,10 +149,14 @@ struct OpNormal {
   const double* nr;
   const double* invdiag;
   int slot = 5;
-  __device__ void terms(int64_t i, double& a, double& c) const {
-    const double z = invdiag[i] * nr[i];
-    a += nr[i] * nr[i];
-    c += nr[i] * z;
+  struct In {
+    double nr, d;
+  };
+  __device__ In load(int64_t i) const { return {nr[i], invdiag[i]}; }
+  __device__ void terms(int64_t, const In& in, double& a, double& c) const {
+    const double z = in.d * in.nr;
+    a += in.nr * in.nr;
+    c += in.nr * z;
   }
   __device__ void finalize(CgScalars* S, double nrr, double nrz) const {
     S->nrr = nrr;
