@@ -437,11 +437,13 @@ __global__ void __launch_bounds__(128) kWideNodes(BvhDevice B, const BoxF* __res
 constexpr int kWalkThreads = 128, kGroups = kWalkThreads / 8;
 // The tree's keys are 30 bits of position and an index: at most 62 binary levels. A wide node
 // spans at least three of them and leaves seven others on the stack. The winding walk takes eight
-// nodes at a time (each may leave two) while its stack is short, else one at a time, which adds
-// at most one entry per level (short below 32, 64, 128, 256 or 400 entries: 5.8, 4.6, 4.6, 5.0,
-// 5.5 ms for the call: a longer stack takes shared memory from the L1 and the resident blocks).
+// nodes at a time (each may leave two) while its stack is short, else one at a time with none on
+// their way, which adds at most one entry per level (short below 32, 64, 128, 256 or 400 entries,
+// without the second buffer: 5.8, 4.6, 4.6, 5.0, 5.5 ms for the call: a longer stack takes shared
+// memory from the L1 and the resident blocks). When it stops being short it has at most 72
+// entries, and eight nodes on their way leave 16 more.
 constexpr int kTreeLevels = 62, kNearStack = 7 * ((kTreeLevels + 2) / 3) + 8;
-constexpr int kWideFwn = 64, kFwnStack = kWideFwn + 16 + kTreeLevels + 2;
+constexpr int kWideFwn = 64, kFwnStack = kWideFwn + 24 + kTreeLevels + 2;
 
 // The next query of each of the warp's groups that needs one, or -1.
 __device__ __forceinline__ int64_t takeQuery(bool need, int lane, int64_t m, unsigned long long* counter) {
@@ -572,6 +574,18 @@ __global__ void __launch_bounds__(kWalkThreads, 6) kNearest(const double* __rest
   }
 }
 
+// Sixteen bytes from global to shared memory, without registers.
+__device__ __forceinline__ void copyAsync16(void* to, const void* from) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from)
+               : "memory");
+}
+__device__ __forceinline__ void copyAsyncCommit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// All but the last N groups of this thread's copies are there.
+template <int N>
+__device__ __forceinline__ void copyAsyncWait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // The sign: the fast winding number's sum over the binary tree. A group takes up to eight nodes
 // from the top of its stack, a lane each: a far node adds its expansion, a near one puts its
 // inner children back on the stack and its leaves on a list, whose exact solid angles are formed
@@ -582,28 +596,33 @@ __global__ void __launch_bounds__(kWalkThreads, 6) kNearest(const double* __rest
 // the nodes that they disagree on read a third of the records and were no faster (1.82 to 2.3 ms):
 // too few walks are in flight, over too much of the tree.
 //
+// The next eight records are fetched (cp.async, a line of 128 bytes by eight lanes) before the
+// current ones are looked at, from what the stack holds then: waiting for L2 was three fifths of the walk's time.
+// The second buffer takes the sixth block of an SM. Signed distance at 196,518 points and 1,048,576
+// faces: 4.02 -> 3.22 ms; at 200,000 and 20,000 faces 1.16 -> 0.99 ms and 518 -> 467 us.
+//
 // The distances are not read: this grid starts in the places that the nearest walk's blocks leave,
 // whose last walks are long (23 % of its time with a chip partly idle), and writes a byte per
 // query; kSigns puts the signs on. Signed distance at 196,518 corners: 4.51 -> 4.08 ms; at 2,000
 // faces 560 -> 444 us.
-__global__ void __launch_bounds__(kWalkThreads, 6) kWinding(const double* __restrict__ P, int64_t m,
+__global__ void __launch_bounds__(kWalkThreads, 5) kWinding(const double* __restrict__ P, int64_t m,
                                                          const uint32_t* __restrict__ order,
                                                          const FwnNode* __restrict__ W, const double* __restrict__ tris,
                                                          int64_t n, uint8_t* __restrict__ inside,
                                                          unsigned long long* __restrict__ counter) {
   __shared__ int32_t sStack[kGroups][kFwnStack];
-  __shared__ double2 sRec[kGroups][64];    // eight records; piece p of record r at p ^ r
+  __shared__ double2 sRec[2][kGroups][64];  // eight records, twice; piece p of record r at p ^ r
   __shared__ int32_t sLeaves[kGroups][24];  // fewer than eight are left before sixteen more can come
   const int lane = threadIdx.x & 31, j = lane & 7, shift = lane & 24;
   const unsigned below = (1u << j) - 1u;
   int32_t* stack = sStack[threadIdx.x >> 3];
   int32_t* leaves = sLeaves[threadIdx.x >> 3];
-  double2* rec = sRec[threadIdx.x >> 3];
   int64_t qi = -1;
   bool drained = false;  // no query is left for this group
   D3 q{0, 0, 0};
   double w = 0.0;
-  int sp = 0, nl = 0;
+  int sp = 0, nl = 0, buf = 0;
+  int here = 0, coming = 0;  // records in this buffer, and on their way to the other
   while (true) {
     const int64_t got = takeQuery(qi < 0 && !drained, lane, m, counter);
     drained = drained || (qi < 0 && got < 0);
@@ -620,22 +639,23 @@ __global__ void __launch_bounds__(kWalkThreads, 6) kWinding(const double* __rest
     }
     if (!__any_sync(0xffffffffu, qi >= 0)) break;
     __syncwarp();
-    const int take = sp > kWideFwn ? 1 : (sp < 8 ? sp : 8);
-    const bool have = j < take;
-    const int32_t node = have ? stack[sp - take + j] : 0;
-    sp -= take;
-    __syncwarp();
-    // the records come in a line at a time, a lane per 16 bytes (a lane loading its own record
-    // touches a line per lane and load: the L1 ran at 74 % and held the walk up)
+    // the next records set out before these are looked at
+    coming = sp > kWideFwn ? (here ? 0 : 1) : (sp < 8 ? sp : 8);
+    const int32_t node = j < coming ? stack[sp - coming + j] : 0;
+    sp -= coming;
+    double2* to = sRec[buf ^ 1][threadIdx.x >> 3];
 #pragma unroll
     for (int o = 0; o < 8; ++o) {
       const int32_t no = __shfl_sync(0xffffffffu, node, o, 8);
-      if (o < take) rec[8 * o + (j ^ o)] = __ldg((const double2*)(W + no) + j);
+      if (o < coming) copyAsync16(&to[8 * o + (j ^ o)], (const double2*)(W + no) + j);
     }
+    copyAsyncCommit();
+    copyAsyncWait<1>();
     __syncwarp();
+    const double2* rec = sRec[buf][threadIdx.x >> 3];
     bool near = false;
     int32_t c0 = 0, c1 = 0;
-    if (have) {
+    if (j < here) {
       FwnNode nd;
 #pragma unroll
       for (int p = 0; p < 8; ++p) ((double2*)&nd)[p] = rec[8 * j + (p ^ j)];
@@ -653,6 +673,8 @@ __global__ void __launch_bounds__(kWalkThreads, 6) kWinding(const double* __rest
         c1 = nd.child[1];
       }
     }
+    here = coming;
+    buf ^= 1;
     const unsigned i0 = (__ballot_sync(0xffffffffu, near && c0 >= 0) >> shift) & 0xffu;
     const unsigned i1 = (__ballot_sync(0xffffffffu, near && c1 >= 0) >> shift) & 0xffu;
     const unsigned l0 = (__ballot_sync(0xffffffffu, near && c0 < 0) >> shift) & 0xffu;
@@ -668,7 +690,7 @@ __global__ void __launch_bounds__(kWalkThreads, 6) kWinding(const double* __rest
     nl += __popc(l0) + __popc(l1);
     __syncwarp();
     // solid angles, once some group has eight leaves or nothing else to do; the others' along
-    while (__any_sync(0xffffffffu, nl >= 8 || (sp == 0 && nl > 0))) {
+    while (__any_sync(0xffffffffu, nl >= 8 || (sp == 0 && here == 0 && nl > 0))) {
       const int t = nl < 8 ? nl : 8;
       if (j < t) {
         D3 a, b, c;
@@ -678,7 +700,7 @@ __global__ void __launch_bounds__(kWalkThreads, 6) kWinding(const double* __rest
       nl -= t;
       __syncwarp();
     }
-    const bool done = qi >= 0 && sp == 0;  // its leaves are summed by now
+    const bool done = qi >= 0 && sp == 0 && here == 0;  // its leaves are summed by now
     if (!__any_sync(0xffffffffu, done)) continue;
     const double total = groupSum(done ? w : 0.0);
     if (done) {
@@ -789,7 +811,7 @@ its_status sdfBvh(its_ctx* ctx, const double* dP, int64_t m, const double* dV, c
   const unsigned blocks = (unsigned)std::min<int64_t>(gridFor(m, kGroups), 6ll * ctx->numSMs);  // six fit an SM
   kNearest<<<blocks, kWalkThreads, 0, ctx->stream>>>(dP, m, qorder.p, wide.p, tris.p, dOut, counters.p);
   ITS_LAUNCHED(ctx);
-  if ((st = launchDependent(ctx, true, kWinding, blocks, kWalkThreads, 0, ctx->stream, dP, m, qorder.p, fwn.p, tris.p,
+  if ((st = launchDependent(ctx, true, kWinding, (unsigned)std::min<int64_t>(gridFor(m, kGroups), 5ll * ctx->numSMs), kWalkThreads, 0, ctx->stream, dP, m, qorder.p, fwn.p, tris.p,
                             nf, inside.p, counters.p + 1)) != ITS_OK)
     return st;
   kSigns<<<gridFor(m, 256), 256, 0, ctx->stream>>>(inside.p, dOut, m);
