@@ -783,6 +783,7 @@ constexpr int kSignWords = 16;  // words of 32 lattice points per warp
 template <typename T>
 __global__ void __launch_bounds__(kScanThreads) kMcSigns(const T* __restrict__ field, int64_t total, double iso,
                                                          uint32_t* __restrict__ signs, unsigned* __restrict__ zero) {
+  gridDependents();
   if (blockIdx.x == 0 && threadIdx.x == 0) *zero = 0u;  // the listed tiles' counter
   const int lane = threadIdx.x & 31;
   const int64_t w0 = ((int64_t)blockIdx.x * (kScanThreads / 32) + (threadIdx.x >> 5)) * kSignWords;
@@ -805,12 +806,12 @@ __global__ void __launch_bounds__(kScanThreads) kMcSigns(const T* __restrict__ f
 }
 
 // The bit of lattice point p, and the 32 bits from it on.
-__device__ __forceinline__ unsigned signBit(const uint32_t* __restrict__ signs, int64_t p) {
-  return (__ldg(signs + (p >> 5)) >> (p & 31)) & 1u;
+__device__ __forceinline__ unsigned signBit(const uint32_t* signs, int64_t p) {
+  return (signs[p >> 5] >> (p & 31)) & 1u;
 }
-__device__ __forceinline__ uint32_t signWindow(const uint32_t* __restrict__ signs, int64_t p) {
+__device__ __forceinline__ uint32_t signWindow(const uint32_t* signs, int64_t p) {
   const uint32_t* w = signs + (p >> 5);
-  return __funnelshift_r(__ldg(w), __ldg(w + 1), (unsigned)(p & 31));
+  return __funnelshift_r(w[0], w[1], (unsigned)(p & 31));
 }
 // Bits 0..3 of b, one per byte.
 __device__ __forceinline__ uint32_t spread4(uint32_t b) { return ((b & 15u) * 0x00204081u) & 0x01010101u; }
@@ -829,7 +830,7 @@ static FastDiv fastDiv(int d) { return {d > 1 ? ~0ull / (unsigned)d + 1ull : 0ul
 // A warp takes kTiles consecutive tiles of 32 x ITEMS voxels, their windows loaded together. A run
 // that crosses a row's end joins the windows of the two rows.
 template <int ITEMS, int kTiles>
-__global__ void __launch_bounds__(kScanThreads) kMcCases(const uint32_t* __restrict__ signs, int R, FastDiv byR,
+__global__ void __launch_bounds__(kScanThreads) kMcCases(const uint32_t* signs, int R, FastDiv byR,
                                                          uint8_t* __restrict__ cube, int64_t numTiles,
                                                          unsigned long long* __restrict__ tileSums,
                                                          uint32_t* __restrict__ listed, unsigned* __restrict__ numListed) {
@@ -838,6 +839,9 @@ __global__ void __launch_bounds__(kScanThreads) kMcCases(const uint32_t* __restr
   const int lane = threadIdx.x & 31;
   const int64_t nvox = (int64_t)R * R * R, M = (int64_t)R + 1;
   const int64_t tile0 = ((int64_t)blockIdx.x * (kScanThreads / 32) + (threadIdx.x >> 5)) * kTiles;
+  sCount[threadIdx.x] = (unsigned char)(cMcCase[threadIdx.x] & 15ull);
+  gridDependencyWait();
+  gridDependents();
   uint32_t c[kTiles][4], n[kTiles][4];  // the corners at x and x + 1 of (y, z), (y+1, z), (y, z+1), (y+1, z+1)
   bool whole[kTiles];
 #pragma unroll
@@ -864,7 +868,6 @@ __global__ void __launch_bounds__(kScanThreads) kMcCases(const uint32_t* __restr
       }
     }
   }
-  sCount[threadIdx.x] = (unsigned char)(cMcCase[threadIdx.x] & 15ull);
   __syncthreads();
   unsigned sums[kTiles];
 #pragma unroll
@@ -943,10 +946,10 @@ __global__ void __launch_bounds__(kScanThreads) kMcCases(const uint32_t* __restr
 // and writes its point, so neighbouring lanes write neighbouring vertices.
 template <typename T, int ITEMS>
 __global__ void __launch_bounds__(kScanThreads) kMcEmit(McCaseT<T> mc, FastDiv byR, double3 o, double3 vs,
-                                                        const uint8_t* __restrict__ cube,
-                                                        const unsigned long long* __restrict__ tileOffsets,
-                                                        const uint32_t* __restrict__ listed,
-                                                        const unsigned* __restrict__ numListed,
+                                                        const uint8_t* cube,
+                                                        const unsigned long long* tileOffsets,
+                                                        const uint32_t* listed,
+                                                        const unsigned* numListed,
                                                         double* __restrict__ tri, unsigned long long capacity) {
   constexpr int kTile = 32 * ITEMS;
   static_assert(15 * kTile < 65536, "voxel and vertex counts share 32 bits");
@@ -961,6 +964,7 @@ __global__ void __launch_bounds__(kScanThreads) kMcEmit(McCaseT<T> mc, FastDiv b
   uint8_t* sPlace = sPlaces[warp];
   __shared__ uint64_t sTable[256];  // per-lane indices: shared memory, not the constant cache
   sTable[threadIdx.x] = cMcCase[threadIdx.x];
+  gridDependencyWait();
   __syncthreads();
   const int64_t nvox = (int64_t)R * R * R, M = (int64_t)R + 1;
   const unsigned n = *numListed, step = gridDim.x * (kScanThreads / 32);
@@ -1430,41 +1434,47 @@ its_status marchingCubesT(its_ctx* ctx, const FT* field, int res, const double o
   const int itemsOf[3] = {8, 16, 4};
   const int64_t points = M * M * M, signBlocks = (points + 32 * kSignWords * (kScanThreads / 32) - 1) /
                                                  (32 * kSignWords * (kScanThreads / 32));
-  DevBuf<unsigned long long> sums, tot;
-  DevBuf<uint32_t> signs, listed;  // a window reads the word after its own
-  DevBuf<unsigned> numListed;
-  if ((st = tot.alloc(ctx, 1)) != ITS_OK || (st = numListed.alloc(ctx, 1)) != ITS_OK ||
-      (st = signs.alloc(ctx, signBlocks * (kScanThreads / 32) * kSignWords + 1)) != ITS_OK)
-    return st;
+  const int64_t signWords = signBlocks * (kScanThreads / 32) * kSignWords + 1;  // a window reads the word after its own
+  // one scratch for all: the total, the listed tiles' counter, the tiles' sums, their list, the signs
+  // (with five allocations and ordinary launches 64^3 took 62 us, now 50)
+  DevBuf<unsigned long long> scratch;
+  unsigned long long *tot = nullptr, *sums = nullptr;
+  unsigned* numListed = nullptr;
+  uint32_t *listed = nullptr, *signs = nullptr;
+  auto place = [&](int64_t nt) -> its_status {
+    const int64_t ns = nt + spineTops(nt), nl = T.d ? (nt + 1) / 2 : 0, need = 2 + ns + nl + (signWords + 1) / 2;
+    if ((int64_t)scratch.n < need && (st = scratch.alloc(ctx, need)) != ITS_OK) return st;
+    tot = scratch.p;
+    numListed = (unsigned*)(scratch.p + 1);
+    sums = scratch.p + 2;
+    listed = T.d ? (uint32_t*)(sums + ns) : nullptr;
+    signs = (uint32_t*)(sums + ns + nl);
+    return ITS_OK;
+  };
   const double3 o3 = make_double3(origin[0], origin[1], origin[2]);
   const double3 v3 = make_double3(width[0] / res, width[1] / res, width[2] / res);
   auto runTiles = [&](auto itemsTag) -> its_status {
     constexpr int kItems = decltype(itemsTag)::value;
     const int64_t nt = (nvox + 32 * kItems - 1) / (32 * kItems);
-    if ((int64_t)sums.n != nt + spineTops(nt) &&
-        ((st = sums.alloc(ctx, nt + spineTops(nt))) != ITS_OK || (T.d && (st = listed.alloc(ctx, nt)) != ITS_OK)))
-      return st;
+    if ((st = place(nt)) != ITS_OK) return st;
+    kMcSigns<FT><<<(unsigned)signBlocks, kScanThreads, 0, ctx->stream>>>(F.d, points, iso, signs, numListed);
+    ITS_LAUNCHED(ctx);
     // four tiles per warp once that many keep every SM full of warps
     constexpr int kWarps = kScanThreads / 32;
-    if (nt >= 4ll * 64 * ctx->numSMs)
-      kMcCases<kItems, 4><<<(unsigned)((nt + 4 * kWarps - 1) / (4 * kWarps)), kScanThreads, 0, ctx->stream>>>(
-          signs.p, res, fastDiv(res), cubeD, nt, sums.p, listed.p, numListed.p);
-    else
-      kMcCases<kItems, 1><<<(unsigned)((nt + kWarps - 1) / kWarps), kScanThreads, 0, ctx->stream>>>(
-          signs.p, res, fastDiv(res), cubeD, nt, sums.p, listed.p, numListed.p);
-    ITS_LAUNCHED(ctx);
-    if ((st = scanSpine<unsigned long long>(ctx, sums.p, nt, tot.p, sums.p + nt)) != ITS_OK) return st;
-    if (T.d) {
-      kMcEmit<FT, kItems><<<(unsigned)std::min<int64_t>((nt + kWarps - 1) / kWarps, 8ll * ctx->numSMs), kScanThreads, 0,
-                            ctx->stream>>>(mc, fastDiv(res), o3, v3, cubeD, sums.p, listed.p, numListed.p, T.d,
-                                           (unsigned long long)capacity);
-      ITS_LAUNCHED(ctx);
-    }
-    return ITS_OK;
+    const bool four = nt >= 4ll * 64 * ctx->numSMs;
+    const int64_t perBlock = (four ? 4 : 1) * kWarps;
+    auto* cases = four ? kMcCases<kItems, 4> : kMcCases<kItems, 1>;
+    if ((st = launchDependent(ctx, true, cases, (unsigned)((nt + perBlock - 1) / perBlock), kScanThreads, 0, ctx->stream,
+                              (const uint32_t*)signs, res, fastDiv(res), cubeD, nt, sums, listed, numListed)) != ITS_OK)
+      return st;
+    if ((st = scanSpine<unsigned long long>(ctx, sums, nt, tot, sums + nt)) != ITS_OK) return st;
+    if (!T.d) return ITS_OK;
+    return launchDependent(ctx, true, kMcEmit<FT, kItems>,
+                           (unsigned)std::min<int64_t>((nt + kWarps - 1) / kWarps, 8ll * ctx->numSMs), kScanThreads, 0,
+                           ctx->stream, mc, fastDiv(res), o3, v3, (const uint8_t*)cubeD, (const unsigned long long*)sums,
+                           (const uint32_t*)listed, (const unsigned*)numListed, T.d, (unsigned long long)capacity);
   };
   auto run = [&](int i) -> its_status {
-    kMcSigns<FT><<<(unsigned)signBlocks, kScanThreads, 0, ctx->stream>>>(F.d, points, iso, signs.p, numListed.p);
-    ITS_LAUNCHED(ctx);
     if (itemsOf[i] == 16) return runTiles(std::integral_constant<int, 16>());
     if (itemsOf[i] == 4) return runTiles(std::integral_constant<int, 4>());
     return runTiles(std::integral_constant<int, 8>());
@@ -1479,7 +1489,7 @@ its_status marchingCubesT(its_ctx* ctx, const FT* field, int res, const double o
   if ((st = tuneChoice(ctx, key, 3, def, run, &choice)) != ITS_OK) return st;
   if ((st = run(choice)) != ITS_OK) return st;
   unsigned long long total = 0;
-  if ((st = readScalar(ctx, tot.p, &total)) != ITS_OK) return st;
+  if ((st = readScalar(ctx, (const unsigned long long*)tot, &total)) != ITS_OK) return st;
   *num_verts = (int64_t)total;
   // only the vertices written leave the device (the rest of a host buffer is left untouched)
   T.count = 3 * (size_t)std::min<int64_t>(capacity, (int64_t)total);

@@ -59,6 +59,8 @@ __global__ void kScanUpsweep(F f, int64_t n, T* blockSums) {
 // Both passes read eight sums per step, so that the loads of a run are in flight together.
 template <typename T>
 __global__ void kScanSpine(T* blockSums, int64_t nb, T* total) {
+  gridDependents();
+  gridDependencyWait();
   const int64_t per = (nb + kScanThreads - 1) / kScanThreads;
   const int64_t b0 = (int64_t)threadIdx.x * per, b1 = b0 + per < nb ? b0 + per : nb;
   T s = 0;
@@ -98,7 +100,9 @@ constexpr int64_t kSpineOneBlock = 8192;
 constexpr int kSpineTile = kScanThreads * 8;
 inline int64_t spineTops(int64_t nb) { return nb > kSpineOneBlock ? (nb + kSpineTile - 1) / kSpineTile : 0; }
 template <typename T>
-__global__ void __launch_bounds__(kScanThreads) kSpineTiles(T* __restrict__ sums, int64_t nb, T* __restrict__ tops) {
+__global__ void __launch_bounds__(kScanThreads) kSpineTiles(T* sums, int64_t nb, T* tops) {
+  gridDependents();
+  gridDependencyWait();
   const int64_t i0 = (int64_t)blockIdx.x * kSpineTile + (int64_t)threadIdx.x * 8;
   T v[8];
   T s = 0;
@@ -118,8 +122,9 @@ __global__ void __launch_bounds__(kScanThreads) kSpineTiles(T* __restrict__ sums
   if (threadIdx.x == 0) tops[blockIdx.x] = tot;
 }
 template <typename T>
-__global__ void __launch_bounds__(kScanThreads) kSpineAdd(T* __restrict__ sums, int64_t nb,
-                                                         const T* __restrict__ tops) {
+__global__ void __launch_bounds__(kScanThreads) kSpineAdd(T* sums, int64_t nb, const T* tops) {
+  gridDependents();
+  gridDependencyWait();
   const T add = tops[blockIdx.x];
   const int64_t i0 = (int64_t)blockIdx.x * kSpineTile;
   for (int k = threadIdx.x; k < kSpineTile; k += kScanThreads)
@@ -154,22 +159,20 @@ struct StorePrefix {
 };
 
 // The spine: nb block sums scanned in place (exclusive), their total to *total (may be NULL);
-// above kSpineOneBlock sums tops holds spineTops(nb) elements of scratch.
+// above kSpineOneBlock sums tops holds spineTops(nb) elements of scratch. The previous operation in
+// the stream is the kernel that wrote the sums.
 template <typename T>
 its_status scanSpine(its_ctx* ctx, T* sums, int64_t nb, T* total, T* tops) {
-  if (nb <= kSpineOneBlock) {
-    kScanSpine<T><<<1, kScanThreads, 0, ctx->stream>>>(sums, nb, total);
-    ITS_LAUNCHED(ctx);
-    return ITS_OK;
-  }
+  if (nb <= kSpineOneBlock)
+    return launchDependent(ctx, true, kScanSpine<T>, 1, kScanThreads, 0, ctx->stream, sums, nb, total);
   const int64_t nt = spineTops(nb);
-  kSpineTiles<T><<<(unsigned)nt, kScanThreads, 0, ctx->stream>>>(sums, nb, tops);
-  ITS_LAUNCHED(ctx);
-  kScanSpine<T><<<1, kScanThreads, 0, ctx->stream>>>(tops, nt, total);
-  ITS_LAUNCHED(ctx);
-  kSpineAdd<T><<<(unsigned)nt, kScanThreads, 0, ctx->stream>>>(sums, nb, tops);
-  ITS_LAUNCHED(ctx);
-  return ITS_OK;
+  its_status st;
+  if ((st = launchDependent(ctx, true, kSpineTiles<T>, (unsigned)nt, kScanThreads, 0, ctx->stream, sums, nb, tops)) !=
+          ITS_OK ||
+      (st = launchDependent(ctx, true, kScanSpine<T>, 1, kScanThreads, 0, ctx->stream, tops, nt, total)) != ITS_OK)
+    return st;
+  return launchDependent(ctx, true, kSpineAdd<T>, (unsigned)nt, kScanThreads, 0, ctx->stream, sums, nb,
+                         (const T*)tops);
 }
 
 // Short scans in one launch: one block takes the tiles in turn.
