@@ -236,10 +236,13 @@ static its_status cubicGrid(its_ctx* ctx, const SvoDevice& d, const double* lam,
   kCubicTables<<<gridFor(n, 256), 256, 0, ctx->stream>>>(g, o, vs, M, tabW.p, tabB.p);
   ITS_LAUNCHED(ctx);
   const int cap = (int)cubicStage(d, vs, kZ);
-  const int bytes = (int)sizeof(CubStage<kZ>) + cap * 8 + cap / 4 + 16;  // a box column holds at least four
-  ITS_CU(ctx, cudaFuncSetAttribute(kCubicEvalGrid<kZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  // (a box column holds at least four entries)
+  auto bytes = [](int entries) { return (int)sizeof(CubStage<kZ>) + entries * 8 + entries / 4 + 16; };
+  // The attribute is the function's, for every thread of the process: the most that any call asks for,
+  // so that a call in another context cannot lower it between here and the launch.
+  ITS_CU(ctx, cudaFuncSetAttribute(kCubicEvalGrid<kZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes(kCubMaxStage)));
   const dim3 grid((unsigned)((M + kCubX - 1) / kCubX), (unsigned)((M + kCubY - 1) / kCubY), (unsigned)((M + kZ - 1) / kZ));
-  kCubicEvalGrid<kZ><<<grid, kCubThreads, bytes, ctx->stream>>>(g, lam, o, vs, tabW.p, tabB.p, M, cap, out);
+  kCubicEvalGrid<kZ><<<grid, kCubThreads, bytes(cap), ctx->stream>>>(g, lam, o, vs, tabW.p, tabB.p, M, cap, out);
   ITS_LAUNCHED(ctx);
   return ITS_OK;
 }
