@@ -212,21 +212,23 @@ __global__ void __launch_bounds__(kCubThreads, 3) kCubicEvalGrid(const __grid_co
     if (first[2] + q < M) out[xi + M * (yj + M * (first[2] + q))] = acc[q];
 }
 
-// Staged coefficients of a brick of z points deep, at most (over the depths; one more per axis than
-// exact, for the rounding of the cell quotients).
-static int64_t cubicStage(const SvoDevice& d, double3 vs, int z) {
+// Coefficients that a brick of z points deep stages, at most, over the depths; -1 where they may not
+// all fit, or where the lattice does not run forwards.
+static int cubicStage(const SvoDevice& d, double3 vs, int64_t M, int z) {
   double n = 0.0;
   for (int k = 0; k < d.depth; ++k) {
-    const double w = d.unit[0] * (double)(1u << k), m = (double)(d.res >> k) + 8.0;
-    auto side = [&](int points, double v) { return std::min(std::floor((points - 1) * std::fabs(v) / w) + 6.0, m + 6.0); };
+    const double w = d.unit[0] * (double)(1u << k), all = (double)(d.res >> k) + 11.0;  // (cells are clamped)
+    auto side = [&](int points, double v) {
+      return std::min(std::floor((double)(std::min<int64_t>(points, M) - 1) * v / w + 1e-6) + 5.0, all);
+    };
     n += side(kCubX, vs.x) * side(kCubY, vs.y) * side(z, vs.z);
   }
-  return n < (double)kCubMaxStage ? (int64_t)n : kCubMaxStage;  // (also where n is not a number)
+  return vs.x > 0.0 && vs.y > 0.0 && vs.z > 0.0 && n <= (double)kCubMaxStage ? (int)n : -1;
 }
 
 template <int kZ>
 static its_status cubicGrid(its_ctx* ctx, const SvoDevice& d, const double* lam, double3 o, double3 vs, int64_t M,
-                            double* out) {
+                            int cap, double* out) {
   const CubicGen g = cubicGen(d, nullptr);
   const int64_t n = (int64_t)d.depth * 3 * M;
   DevBuf<double> tabW;
@@ -235,7 +237,6 @@ static its_status cubicGrid(its_ctx* ctx, const SvoDevice& d, const double* lam,
   if ((st = tabW.alloc(ctx, 4 * n)) != ITS_OK || (st = tabB.alloc(ctx, n)) != ITS_OK) return st;
   kCubicTables<<<gridFor(n, 256), 256, 0, ctx->stream>>>(g, o, vs, M, tabW.p, tabB.p);
   ITS_LAUNCHED(ctx);
-  const int cap = (int)cubicStage(d, vs, kZ);
   // (a box column holds at least four entries)
   auto bytes = [](int entries) { return (int)sizeof(CubStage<kZ>) + entries * 8 + entries / 4 + 16; };
   // The attribute is the function's, for every thread of the process: the most that any call asks for,
@@ -245,6 +246,17 @@ static its_status cubicGrid(its_ctx* ctx, const SvoDevice& d, const double* lam,
   kCubicEvalGrid<kZ><<<grid, kCubThreads, bytes(cap), ctx->stream>>>(g, lam, o, vs, tabW.p, tabB.p, M, cap, out);
   ITS_LAUNCHED(ctx);
   return ITS_OK;
+}
+
+// Lattice point i (x fastest), one thread each: for lattices too coarse for bricks.
+__global__ void __launch_bounds__(128) kCubicEvalLattice(const __grid_constant__ CubicGen g,
+                                                         const double* __restrict__ lambda, double3 o, double3 vs,
+                                                         int64_t M, double* __restrict__ out) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= M * M * M) return;
+  const int64_t ix = i % M, iy = (i / M) % M, iz = i / (M * M);
+  const double x[3] = {o.x + (double)ix * vs.x, o.y + (double)iy * vs.y, o.z + (double)iz * vs.z};
+  out[i] = g.eval(x, lambda);
 }
 
 // Start of each vertex's run in the vertex-sorted face corners (every pointer written once).
@@ -338,11 +350,22 @@ its_status its_eval_grid_cubic(its_svo* svo, const double* lambda, const double 
     return st;
   const double3 o = make_double3(origin[0], origin[1], origin[2]);
   const double3 vs = make_double3(width[0] / res, width[1] / res, width[2] / res);
-  // bricks of 8 points deep where two blocks per SM come of them, else of 4 (65^3 points on an octree
-  // of 64: 101 us with 8, 76 with 4; 129^3 on one of 32: 175 and 207)
+  // Bricks where every depth's box fits, 8 points deep where two blocks per SM come of them, else 4
+  // (65^3 points on an octree of 64: 101 us with 8, 76 with 4; 129^3 on one of 32: 175 and 207). Coarser
+  // lattices point by point: a brick's threads would look the corners of a whole depth up for their
+  // points, one after another (us by points and in bricks: 9^3 on an octree of 32 77 and 117, 33^3 on
+  // 64 96 and 414, 65^3 on 256 277 and 640; where only the finest depth does not fit, bricks may win,
+  // 129^3 on 256 1640 and 1030, or lose, 171^3 on 256 3590 and 4330).
   const int64_t deep = ((M + kCubX - 1) / kCubX) * ((M + kCubY - 1) / kCubY) * ((M + 7) / 8);
-  st = deep >= 2 * ctx->numSMs ? cubicGrid<8>(ctx, svo->d, L.d, o, vs, M, O.d)
-                               : cubicGrid<4>(ctx, svo->d, L.d, o, vs, M, O.d);
+  const int cap8 = deep >= 2 * ctx->numSMs ? cubicStage(svo->d, vs, M, 8) : -1, cap4 = cubicStage(svo->d, vs, M, 4);
+  if (cap8 >= 0) {
+    st = cubicGrid<8>(ctx, svo->d, L.d, o, vs, M, cap8, O.d);
+  } else if (cap4 >= 0) {
+    st = cubicGrid<4>(ctx, svo->d, L.d, o, vs, M, cap4, O.d);
+  } else {
+    kCubicEvalLattice<<<gridFor(M * M * M, 128), 128, 0, ctx->stream>>>(cubicGen(svo->d, nullptr), L.d, o, vs, M, O.d);
+    ITS_LAUNCHED(ctx);
+  }
   if (st != ITS_OK) return st;
   if ((st = O.finish(ctx)) != ITS_OK) return st;
   ITS_CU(ctx, cudaStreamSynchronize(ctx->stream));
