@@ -73,14 +73,20 @@ struct NodeSums {
 constexpr int kSumWords = sizeof(NodeSums) / 8;
 constexpr int kTriWords = 10;  // a leaf triangle's nine coordinates, padded to whole 16-byte loads
 
+// Per block: the centroids' bounds, and the largest coordinate's size (its upper word: the exponent counts).
+constexpr int kBoundWords = 7;
 __global__ void kCentroidBounds(const double* __restrict__ V, const int32_t* __restrict__ F, int64_t nf,
                                 double* __restrict__ partial) {
   double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300};
+  int size = 0;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nf; t += (int64_t)gridDim.x * blockDim.x) {
     for (int a = 0; a < 3; ++a) {
-      const double c = (V[3 * F[3 * t] + a] + V[3 * F[3 * t + 1] + a] + V[3 * F[3 * t + 2] + a]) / 3.0;
+      const double p0 = V[3 * F[3 * t] + a], p1 = V[3 * F[3 * t + 1] + a], p2 = V[3 * F[3 * t + 2] + a];
+      const double c = (p0 + p1 + p2) / 3.0;
       mn[a] = fmin(mn[a], c);
       mx[a] = fmax(mx[a], c);
+      size = max(size, max(__double2hiint(p0) & 0x7fffffff,
+                           max(__double2hiint(p1) & 0x7fffffff, __double2hiint(p2) & 0x7fffffff)));
     }
   }
   for (int a = 0; a < 3; ++a)
@@ -88,15 +94,22 @@ __global__ void kCentroidBounds(const double* __restrict__ V, const int32_t* __r
       mn[a] = fmin(mn[a], __shfl_down_sync(0xffffffffu, mn[a], o));
       mx[a] = fmax(mx[a], __shfl_down_sync(0xffffffffu, mx[a], o));
     }
-  __shared__ double s[8][6];
+  size = __reduce_max_sync(0xffffffffu, size);
+  __shared__ double s[8][kBoundWords];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0)
+  if (lane == 0) {
     for (int a = 0; a < 3; ++a) { s[w][a] = mn[a]; s[w][3 + a] = mx[a]; }
+    s[w][6] = size;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int k = 1; k < (int)(blockDim.x >> 5); ++k)
+    for (int k = 1; k < (int)(blockDim.x >> 5); ++k) {
       for (int a = 0; a < 3; ++a) { mn[a] = fmin(mn[a], s[k][a]); mx[a] = fmax(mx[a], s[k][3 + a]); }
-    for (int a = 0; a < 3; ++a) { partial[6 * blockIdx.x + a] = mn[a]; partial[6 * blockIdx.x + 3 + a] = mx[a]; }
+      size = max(size, (int)s[k][6]);
+    }
+    double* p = partial + kBoundWords * blockIdx.x;
+    for (int a = 0; a < 3; ++a) { p[a] = mn[a]; p[3 + a] = mx[a]; }
+    p[6] = size;
   }
 }
 
@@ -155,12 +168,12 @@ __global__ void kBuildInternal(const uint32_t* __restrict__ codes, int64_t n, in
   parent[R < 0 ? (n - 1) + (-R - 1) : R] = (int32_t)i;
 }
 
-// The node's box, rounded outward.
-__device__ __forceinline__ BoxF outwardBox(const NodeSums& S) {
+// The node's box times scale, a power of two, rounded outward.
+__device__ __forceinline__ BoxF outwardBox(const NodeSums& S, double scale) {
   BoxF b;
   for (int a = 0; a < 3; ++a) {
-    b.lo[a] = __double2float_rd(S.lo[a]);
-    b.hi[a] = __double2float_ru(S.hi[a]);
+    b.lo[a] = __double2float_rd(__dmul_rd(S.lo[a], scale));
+    b.hi[a] = __double2float_ru(__dmul_ru(S.hi[a], scale));
   }
   return b;
 }
@@ -217,9 +230,10 @@ __device__ __forceinline__ FwnNode fwnNode(const NodeSums& S, int32_t left, int3
 // us at 1,048,576 triangles; now 183 us and kClimbTop.
 constexpr int kUpLeaves = 128;
 __global__ void __launch_bounds__(kUpLeaves) kBottomUp(const double* __restrict__ V, const int32_t* __restrict__ F,
-                                                       BvhDevice B, double* __restrict__ raw, int2* __restrict__ top,
-                                                       unsigned* __restrict__ topCount, BoxF* __restrict__ box,
-                                                       FwnNode* __restrict__ fwn, double* __restrict__ tris) {
+                                                       BvhDevice B, double scale, double* __restrict__ raw,
+                                                       int2* __restrict__ top, unsigned* __restrict__ topCount,
+                                                       BoxF* __restrict__ box, FwnNode* __restrict__ fwn,
+                                                       double* __restrict__ tris) {
   __shared__ double sSum[kSumWords][2 * kUpLeaves];
   __shared__ unsigned sFlag[kUpLeaves];
   __shared__ int32_t sParent[2 * kUpLeaves], sLeft[kUpLeaves], sRight[kUpLeaves];
@@ -269,7 +283,7 @@ __global__ void __launch_bounds__(kUpLeaves) kBottomUp(const double* __restrict_
     for (int r = 0; r < 3; ++r)
       for (int j = 0; j < 3; ++j) S.sm[3 * r + j] = an[r] * ((p[0][j] + p[1][j] + p[2][j]) / 3.0);
     S.area = ar;
-    box[(n - 1) + k] = outwardBox(S);
+    box[(n - 1) + k] = outwardBox(S, scale);
   }
   __syncthreads();
   int place = -1;  // of the maximal subtree that this thread ends at
@@ -319,7 +333,7 @@ __global__ void __launch_bounds__(kUpLeaves) kBottomUp(const double* __restrict_
     double* to = (double*)&N;
 #pragma unroll
     for (int w = 0; w < kSumWords; ++w) to[w] = sSum[w][kUpLeaves + i];
-    box[k] = outwardBox(N);
+    box[k] = outwardBox(N, scale);
     fwn[k] = fwnNode(N, sLeft[i], sRight[i]);
   }
   __syncthreads();
@@ -330,7 +344,8 @@ __global__ void __launch_bounds__(kUpLeaves) kBottomUp(const double* __restrict_
 // wait at its first leaf's place; a node's place is its left child's, whose sums the merging
 // thread has read by then. A chain of global round trips, one node after another: a node's links
 // come in while the sums before it go out (131 -> 108 us at 1,048,576 triangles).
-__global__ void __launch_bounds__(128) kClimbTop(BvhDevice B, double* __restrict__ raw, const int2* __restrict__ top,
+__global__ void __launch_bounds__(128) kClimbTop(BvhDevice B, double scale, double* __restrict__ raw,
+                                                 const int2* __restrict__ top,
                                                  const unsigned* __restrict__ topCount, BoxF* __restrict__ box,
                                                  FwnNode* __restrict__ fwn) {
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -357,7 +372,7 @@ __global__ void __launch_bounds__(128) kClimbTop(BvhDevice B, double* __restrict
     volatile double* dst = raw + kSumWords * first;
 #pragma unroll
     for (int w = 0; w < kSumWords; ++w) dst[w] = mine[w];
-    box[par] = outwardBox(S);
+    box[par] = outwardBox(S, scale);
     fwn[par] = fwnNode(S, l, r);
     par = above;
   }
@@ -479,10 +494,17 @@ __device__ __forceinline__ double groupSum(double v) {
 // bound of its box's squared distance (FP32, every operation rounded down) is beyond the best
 // squared distance times (1 + 1e-12), so the minimum is the IEEE value the brute force finds.
 // A bucket's triangles are tested together, one per lane.
+//
+// kScaled: boxes, queries and bounds times the power of two that brings the mesh's largest coordinate to
+// 1/2 .. 1, where the squares stay within FP32's range. Unscaled, a mesh at 2^-80 or 2^80 had every bound
+// 0 or infinite and every triangle tested (200,000 faces and points: 508 and 520 ms, scaled 3.1, as at
+// scale 1). A kernel of its own: on ordinary meshes the multiplications cost 1 % of the call.
+template <bool kScaled>
 __global__ void __launch_bounds__(kWalkThreads, 6) kNearest(const double* __restrict__ P, int64_t m,
                                                          const uint32_t* __restrict__ order,
                                                          const WideNode* __restrict__ wide,
-                                                         const double* __restrict__ tris, double* __restrict__ out,
+                                                         const double* __restrict__ tris, double scale, double slack,
+                                                         double* __restrict__ out,
                                                          unsigned long long* __restrict__ counter) {
   __shared__ int2 sStack[kGroups][kNearStack];  // wide node, lower bound
   const int lane = threadIdx.x & 31, j = lane & 7, shift = lane & 24;
@@ -504,8 +526,8 @@ __global__ void __launch_bounds__(kWalkThreads, 6) kNearest(const double* __rest
       const double x[3] = {q.x, q.y, q.z};
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        qlo[a] = __double2float_rd(x[a]);
-        qhi[a] = __double2float_ru(x[a]);
+        qlo[a] = __double2float_rd(kScaled ? __dmul_rd(x[a], scale) : x[a]);
+        qhi[a] = __double2float_ru(kScaled ? __dmul_ru(x[a], scale) : x[a]);
       }
       best = 1.7976931348623157e308;
       bound = __int_as_float(0x7f800000);
@@ -553,7 +575,7 @@ __global__ void __launch_bounds__(kWalkThreads, 6) kNearest(const double* __rest
         t2 = fmin(t2, pointTriSqDist(q, a, b, c));
       }
       best = fmin(best, groupMin(t2));
-      bound = __double2float_ru(best * (1.0 + 1e-12));
+      bound = __double2float_ru(kScaled ? __dmul_ru(best, slack) : best * (1.0 + 1e-12));
     }
     // wide nodes within the bound, the nearest on top
     const bool push = w.leaves == 0 && d <= bound;
@@ -750,15 +772,24 @@ its_status sdfBvh(its_ctx* ctx, const double* dP, int64_t m, const double* dV, c
   // centroid bounds for the Morton quantisation
   const unsigned pb = 256;
   DevBuf<double> part;
-  if ((st = part.alloc(ctx, 6 * pb)) != ITS_OK) return st;
+  if ((st = part.alloc(ctx, kBoundWords * pb)) != ITS_OK) return st;
   kCentroidBounds<<<pb, 256, 0, ctx->stream>>>(dV, dF, nf, part.p);
   ITS_LAUNCHED(ctx);
-  std::vector<double> hp(6 * pb);
-  ITS_CU(ctx, cudaMemcpyAsync(hp.data(), part.p, 6 * pb * 8, cudaMemcpyDeviceToHost, ctx->stream));
+  std::vector<double> hp(kBoundWords * pb);
+  ITS_CU(ctx, cudaMemcpyAsync(hp.data(), part.p, kBoundWords * pb * 8, cudaMemcpyDeviceToHost, ctx->stream));
   ITS_CU(ctx, cudaStreamSynchronize(ctx->stream));
   double bl[3] = {1e300, 1e300, 1e300}, bh[3] = {-1e300, -1e300, -1e300};
-  for (unsigned k = 0; k < pb; ++k)
-    for (int a = 0; a < 3; ++a) { bl[a] = std::min(bl[a], hp[6 * k + a]); bh[a] = std::max(bh[a], hp[6 * k + 3 + a]); }
+  int size = 0;
+  for (unsigned k = 0; k < pb; ++k) {
+    const double* p = &hp[kBoundWords * k];
+    for (int a = 0; a < 3; ++a) { bl[a] = std::min(bl[a], p[a]); bh[a] = std::max(bh[a], p[3 + a]); }
+    size = std::max(size, (int)p[6]);
+  }
+  // Meshes between 2^-32 and 2^32 as they are: a distance of 1e-8 of them has an FP32 square, and so
+  // has one across them. Others scaled (within 2^+-500, so that the scale's square is a number too).
+  int exponent = size > 0 && size < 0x7ff00000 ? std::max(-500, std::min(500, 1022 - (size >> 20))) : 0;
+  if (std::abs(exponent) <= 32) exponent = 0;
+  const double scale = std::ldexp(1.0, exponent), slack = std::ldexp(1.0 + 1e-12, 2 * exponent);
   double inv[3];
   for (int a = 0; a < 3; ++a) inv[a] = bh[a] > bl[a] ? 1.0 / (bh[a] - bl[a]) : 0.0;
   kMortonCodes<<<gridFor(nf, 256), 256, 0, ctx->stream>>>(dV, dF, nf, make_double3(bl[0], bl[1], bl[2]),
@@ -788,11 +819,11 @@ its_status sdfBvh(its_ctx* ctx, const double* dP, int64_t m, const double* dV, c
       (st = box.alloc(ctx, nodes)) != ITS_OK || (st = fwn.alloc(ctx, inner)) != ITS_OK ||
       (st = wide.alloc(ctx, inner)) != ITS_OK)
     return st;
-  kBottomUp<<<gridFor(nf, kUpLeaves), kUpLeaves, 0, ctx->stream>>>(dV, dF, B, raw.p, top.p, topCount.p, box.p, fwn.p,
+  kBottomUp<<<gridFor(nf, kUpLeaves), kUpLeaves, 0, ctx->stream>>>(dV, dF, B, scale, raw.p, top.p, topCount.p, box.p, fwn.p,
                                                                tris.p);
   ITS_LAUNCHED(ctx);
   if (nf > kUpLeaves) {
-    kClimbTop<<<gridFor(nf, 128), 128, 0, ctx->stream>>>(B, raw.p, top.p, topCount.p, box.p, fwn.p);
+    kClimbTop<<<gridFor(nf, 128), 128, 0, ctx->stream>>>(B, scale, raw.p, top.p, topCount.p, box.p, fwn.p);
     ITS_LAUNCHED(ctx);
   }
   kWideNodes<<<gridFor(inner, 128), 128, 0, ctx->stream>>>(B, box.p, wide.p);
@@ -809,7 +840,7 @@ its_status sdfBvh(its_ctx* ctx, const double* dP, int64_t m, const double* dV, c
   ITS_LAUNCHED(ctx);
   if ((st = radixSortPairs(ctx, qc.p, qi.p, qsc.p, qorder.p, qtk.p, qtv.p, m, 30)) != ITS_OK) return st;
   const unsigned blocks = (unsigned)std::min<int64_t>(gridFor(m, kGroups), 6ll * ctx->numSMs);  // six fit an SM
-  kNearest<<<blocks, kWalkThreads, 0, ctx->stream>>>(dP, m, qorder.p, wide.p, tris.p, dOut, counters.p);
+  (exponent ? kNearest<true> : kNearest<false>)<<<blocks, kWalkThreads, 0, ctx->stream>>>(dP, m, qorder.p, wide.p, tris.p, scale, slack, dOut, counters.p);
   ITS_LAUNCHED(ctx);
   if ((st = launchDependent(ctx, true, kWinding, (unsigned)std::min<int64_t>(gridFor(m, kGroups), 5ll * ctx->numSMs), kWalkThreads, 0, ctx->stream, dP, m, qorder.p, fwn.p, tris.p,
                             nf, inside.p, counters.p + 1)) != ITS_OK)
