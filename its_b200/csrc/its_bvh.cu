@@ -458,6 +458,7 @@ constexpr int kWalkThreads = 128, kGroups = kWalkThreads / 8;
 // memory from the L1 and the resident blocks). When it stops being short it has at most 72
 // entries, and eight nodes on their way leave 16 more.
 constexpr int kTreeLevels = 62, kNearStack = 7 * ((kTreeLevels + 2) / 3) + 8;
+constexpr int kLeafRing = 32;  // leaves waiting in the winding walk, at most 23
 constexpr int kWideFwn = 64, kFwnStack = kWideFwn + 24 + kTreeLevels + 2;
 
 // The next query of each of the warp's groups that needs one, or -1.
@@ -612,7 +613,10 @@ __device__ __forceinline__ void copyAsyncWait() {
 // from the top of its stack, a lane each: a far node adds its expansion, a near one puts its
 // inner children back on the stack and its leaves on a list, whose exact solid angles are formed
 // eight at a time. The nodes accepted and opened are those of a walk one node at a time; the sum
-// is over lanes. A node costs about 65 FP64 operations, a query 414 nodes and 17 leaves at a tube of
+// is over lanes. When leaves are summed depends on the warp's other groups, which queries those hold on
+// a counter; so a query's k-th leaf is lane k mod 8's, added in that order to a sum of its own, and the
+// result is the same from call to call (a group that waited for eight of its own: 2,330 -> 2,390 us at
+// 200,000 faces). A node costs about 65 FP64 operations, a query 414 nodes and 17 leaves at a tube of
 // 1,048,576 faces; a far node's 1/R is rsqrt's, one rounding error like the square root and the
 // reciprocal before (2.06 -> 2.01 ms). Walks shared by clusters of 8 to 32 neighbouring queries down to
 // the nodes that they disagree on read a third of the records and were no faster (1.82 to 2.3 ms):
@@ -634,7 +638,7 @@ __global__ void __launch_bounds__(kWalkThreads, 5) kWinding(const double* __rest
                                                          unsigned long long* __restrict__ counter) {
   __shared__ int32_t sStack[kGroups][kFwnStack];
   __shared__ double2 sRec[2][kGroups][64];  // eight records, twice; piece p of record r at p ^ r
-  __shared__ int32_t sLeaves[kGroups][24];  // fewer than eight are left before sixteen more can come
+  __shared__ int32_t sLeaves[kGroups][kLeafRing];  // fewer than eight are left before sixteen more can come
   const int lane = threadIdx.x & 31, j = lane & 7, shift = lane & 24;
   const unsigned below = (1u << j) - 1u;
   int32_t* stack = sStack[threadIdx.x >> 3];
@@ -642,8 +646,9 @@ __global__ void __launch_bounds__(kWalkThreads, 5) kWinding(const double* __rest
   int64_t qi = -1;
   bool drained = false;  // no query is left for this group
   D3 q{0, 0, 0};
-  double w = 0.0;
-  int sp = 0, nl = 0, buf = 0;
+  double w = 0.0, wl = 0.0;  // the far nodes' sum, the leaves'
+  int sp = 0, buf = 0;
+  int first = 0, nl = 0;  // the query's first leaf in waiting, and how many wait
   int here = 0, coming = 0;  // records in this buffer, and on their way to the other
   while (true) {
     const int64_t got = takeQuery(qi < 0 && !drained, lane, m, counter);
@@ -651,9 +656,10 @@ __global__ void __launch_bounds__(kWalkThreads, 5) kWinding(const double* __rest
     if (got >= 0) {
       qi = order[got];
       q = D3{P[3 * qi], P[3 * qi + 1], P[3 * qi + 2]};
-      w = 0.0;
+      w = wl = 0.0;
       sp = n > 1 ? 1 : 0;
       nl = n > 1 ? 0 : 1;
+      first = 0;
       if (j == 0) {
         stack[0] = 0;
         leaves[0] = 0;
@@ -702,29 +708,31 @@ __global__ void __launch_bounds__(kWalkThreads, 5) kWinding(const double* __rest
     const unsigned l0 = (__ballot_sync(0xffffffffu, near && c0 < 0) >> shift) & 0xffu;
     const unsigned l1 = (__ballot_sync(0xffffffffu, near && c1 < 0) >> shift) & 0xffu;
     if (near) {
-      int at = sp + __popc(i0 & below) + __popc(i1 & below), al = nl + __popc(l0 & below) + __popc(l1 & below);
+      int at = sp + __popc(i0 & below) + __popc(i1 & below);
+      int al = first + nl + __popc(l0 & below) + __popc(l1 & below);
       if (c0 >= 0) stack[at++] = c0;
-      else leaves[al++] = -c0 - 1;
+      else leaves[al++ & (kLeafRing - 1)] = -c0 - 1;
       if (c1 >= 0) stack[at] = c1;
-      else leaves[al] = -c1 - 1;
+      else leaves[al & (kLeafRing - 1)] = -c1 - 1;
     }
     sp += __popc(i0) + __popc(i1);
     nl += __popc(l0) + __popc(l1);
     __syncwarp();
     // solid angles, once some group has eight leaves or nothing else to do; the others' along
     while (__any_sync(0xffffffffu, nl >= 8 || (sp == 0 && here == 0 && nl > 0))) {
-      const int t = nl < 8 ? nl : 8;
-      if (j < t) {
+      const int t = nl < 8 ? nl : 8, mine = (j - first) & 7;
+      if (mine < t) {
         D3 a, b, c;
-        loadTri(tris, leaves[nl - t + j], a, b, c);
-        w += solidAngle(q, a, b, c);
+        loadTri(tris, leaves[(first + mine) & (kLeafRing - 1)], a, b, c);
+        wl += solidAngle(q, a, b, c);
       }
       nl -= t;
+      first += t;
       __syncwarp();
     }
     const bool done = qi >= 0 && sp == 0 && here == 0;  // its leaves are summed by now
     if (!__any_sync(0xffffffffu, done)) continue;
-    const double total = groupSum(done ? w : 0.0);
+    const double total = groupSum(done ? w + wl : 0.0);
     if (done) {
       if (j == 0) inside[qi] = total / (4.0 * 3.14159265358979323846) > 0.5;
       qi = -1;
