@@ -1092,7 +1092,8 @@ static its_status evalGridTuned(its_ctx* ctx, const SvoDevice& d, const double* 
            cap;
   };
   std::vector<int> cand;
-  if (boxFits(4, kSepTileCap)) {
+  const bool coarse = !boxFits(4, kSepTileCap);
+  if (!coarse) {
     if (sizeof(T) == 8) cand = {0, 1, 2, 3};
     cand.push_back(4);
     if (boxFits(8, kSepTileCap)) cand.push_back(5);
@@ -1126,8 +1127,10 @@ static its_status evalGridTuned(its_ctx* ctx, const SvoDevice& d, const double* 
     }
     return ITS_ERR_STATE;
   };
+  // (a choice is a place in the list, and the box decides between two lists: a key for each)
   const std::string key = std::string("eval_grid/") + (sizeof(T) == 8 ? "f64" : "f32") + "/grid=" +
-                          std::to_string(res) + "/octree=" + std::to_string(d.res) + "/depth=" + std::to_string(d.depth);
+                          std::to_string(res) + "/octree=" + std::to_string(d.res) + "/depth=" + std::to_string(d.depth) +
+                          (coarse ? "/coarse" : "");
   int choice = 0;
   st = tuneChoice(ctx, key, (int)cand.size(), (int)cand.size() - 1, run, &choice);
   if (st != ITS_OK) return st;
