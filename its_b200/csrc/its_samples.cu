@@ -93,6 +93,10 @@ __device__ inline bool isLargeDouble(double l, double r) { return !(fabs(l - r) 
 // coordinate and its neighbours (3.1 million edge slots: 441 us a count with every node of the box
 // tested, 105 so). Same values, same tests. emit == nullptr only counts; else the points
 // go out in the reference's order, cell by cell (x fastest), planes x, y, z within a cell.
+// kPlanes = false tests every node of the box in both passes: for lattices so far from the origin that
+// their positions round by a part of a cell, where a point's cell quotient says nothing of the cells
+// that hold it. (Counted by planes, edges there lost up to two thirds of their hits, and a long edge's
+// sweep wrote more points than were counted.)
 constexpr int kEdgeList = 8;  // hits sorted in registers' reach; longer edges write by the full sweep
 template <class Hit>
 __device__ __forceinline__ void edgePlaneHits(const SampleParams& S, const double* p1, const double* dir, const int* lo,
@@ -110,7 +114,8 @@ __device__ __forceinline__ void edgePlaneHits(const SampleParams& S, const doubl
 #pragma unroll
       for (int e = 0; e < 3; ++e) q[e] = p1[e] + tt * dir[e];
       // (a cell quotient's rounding moves a floor by at most one)
-      const int jb = (int)floor((q[b] - org[b]) / w), jc = (int)floor((q[c] - org[c]) / w);
+      const int jb = clampi((int)floor((q[b] - org[b]) / w), -2, S.res + 1),
+                jc = clampi((int)floor((q[c] - org[c]) / w), -2, S.res + 1);
       for (int u = max(jb - 1, lo[b]); u <= min(jb + 1, hi[b]); ++u) {
         const double lb = latticePos(org[b], w, (uint32_t)u);
         if (!inRange(lb, lb + w, q[b])) continue;
@@ -125,6 +130,7 @@ __device__ __forceinline__ void edgePlaneHits(const SampleParams& S, const doubl
     }
   }
 }
+template <bool kPlanes>
 __device__ int edgeHits(const SampleParams& S, const double* p1, const double* p2, int count, double* emit) {
   const double dir[3] = {p2[0] - p1[0], p2[1] - p1[1], p2[2] - p1[2]};
   const double org[3] = {S.g.x, S.g.y, S.g.z};
@@ -135,11 +141,11 @@ __device__ int edgeHits(const SampleParams& S, const double* p1, const double* p
     hi[a] = clampi((d1 > d2 ? d1 : d2) + 1, 0, S.res - 1);
   }
   int n = 0;
-  if (!emit) {
+  if (kPlanes && !emit) {
     edgePlaneHits(S, p1, dir, lo, hi, [&](int, int, int, int, const double*) { ++n; });
     return n;
   }
-  if (count <= kEdgeList) {
+  if (kPlanes && count <= kEdgeList) {
     // a hit's place is the number of hits before it in (z, y, x, plane) order
     uint64_t key[kEdgeList];
     edgePlaneHits(S, p1, dir, lo, hi, [&](int x, int y, int z, int a, const double*) {
@@ -175,9 +181,11 @@ __device__ int edgeHits(const SampleParams& S, const double* p1, const double* p
           for (int c = 0; c < 3; ++c) q[c] = p1[c] + tt[a] * dir[c];
           const int b = a == 0 ? 1 : 0, c = a == 2 ? 1 : 2;
           if (inRange(lbb[b], lbb[b] + w, q[b]) && inRange(lbb[c], lbb[c] + w, q[c])) {
-            emit[3 * n] = q[0];
-            emit[3 * n + 1] = q[1];
-            emit[3 * n + 2] = q[2];
+            if (n < count) {  // (the counting pass: 0)
+              emit[3 * n] = q[0];
+              emit[3 * n + 1] = q[1];
+              emit[3 * n + 2] = q[2];
+            }
             ++n;
           }
         }
@@ -185,6 +193,7 @@ __device__ int edgeHits(const SampleParams& S, const double* p1, const double* p
   return n;
 }
 
+template <bool kPlanes>
 struct EdgeStep {
   SampleParams S;
   const double* V;
@@ -197,17 +206,18 @@ struct EdgeStep {
     if (!isUnique(slot)) return 0;
     const unsigned long long key = edgeKeyOf(F, slot);
     const uint32_t a = (uint32_t)(key >> 32), b = (uint32_t)(key & 0xffffffffu);
-    return (uint32_t)edgeHits(S, V + 3 * a, V + 3 * b, 0, nullptr);
+    return (uint32_t)edgeHits<kPlanes>(S, V + 3 * a, V + 3 * b, 0, nullptr);
   }
 };
+template <bool kPlanes>
 struct EdgeEmit {
-  EdgeStep es;
+  EdgeStep<kPlanes> es;
   double* out;
   __device__ void operator()(int64_t slot, uint32_t prefix, uint32_t count) const {
     if (!count) return;
     const unsigned long long key = edgeKeyOf(es.F, slot);
     const uint32_t a = (uint32_t)(key >> 32), b = (uint32_t)(key & 0xffffffffu);
-    edgeHits(es.S, es.V + 3 * a, es.V + 3 * b, (int)count, out + 3 * (int64_t)prefix);
+    edgeHits<kPlanes>(es.S, es.V + 3 * a, es.V + 3 * b, (int)count, out + 3 * (int64_t)prefix);
   }
 };
 
@@ -470,14 +480,20 @@ its_status its_shell_samples(its_svo* s, const double* verts, int64_t nverts, co
   ITS_CU(ctx, cudaMemsetAsync(eown.p, 0xFF, tsz * 4, ctx->stream));
   kEdgeInsert<<<gridFor(slots, 256), 256, 0, ctx->stream>>>(F.d, slots, ekeys.p, eown.p, tsz - 1);
   ITS_LAUNCHED(ctx);
-  EdgeStep es{S, V.d, F.d, ekeys.p, eown.p, tsz - 1};
   DevBuf<uint32_t> tot, ecnt, eoff, listed;
   DevBuf<unsigned> numListed;
   if ((st = tot.zeros(ctx, 3)) != ITS_OK || (st = ecnt.alloc(ctx, slots)) != ITS_OK ||
       (st = eoff.alloc(ctx, slots)) != ITS_OK || (st = listed.alloc(ctx, slots)) != ITS_OK ||
       (st = numListed.zeros(ctx, 2)) != ITS_OK)
     return st;
-  kCountHits<<<gridFor(slots, 128), 128, 0, ctx->stream>>>(es, slots, ecnt.p, listed.p, numListed.p);
+  // (coordinates up to 2^40 cells round by less than 2^-12 of one)
+  double far = 0.0;
+  for (int a = 0; a < 3; ++a) far = std::max(far, std::fabs(d.origin[a]) + S.w0 * S.res);
+  const bool planes = far <= 1e12 * S.w0;
+  const EdgeStep<true> es{S, V.d, F.d, ekeys.p, eown.p, tsz - 1};
+  const EdgeStep<false> esFar{S, V.d, F.d, ekeys.p, eown.p, tsz - 1};
+  if (planes) kCountHits<<<gridFor(slots, 128), 128, 0, ctx->stream>>>(es, slots, ecnt.p, listed.p, numListed.p);
+  else kCountHits<<<gridFor(slots, 128), 128, 0, ctx->stream>>>(esFar, slots, ecnt.p, listed.p, numListed.p);
   ITS_LAUNCHED(ctx);
   if ((st = scanExclusiveAlloc<uint32_t>(ctx, StoredCount{ecnt.p}, slots, StorePrefix<uint32_t>{eoff.p}, tot.p)) !=
       ITS_OK)
@@ -486,7 +502,11 @@ its_status its_shell_samples(its_svo* s, const double* verts, int64_t nverts, co
   if ((st = readScalar(ctx, tot.p, &nRaw)) != ITS_OK) return st;
   DevBuf<double> raw;
   if ((st = raw.alloc(ctx, 3 * (size_t)(nRaw ? nRaw : 1))) != ITS_OK) return st;
-  kEmitHits<<<emitBlocks(slots), 128, 0, ctx->stream>>>(EdgeEmit{es, raw.p}, listed.p, numListed.p, ecnt.p, eoff.p);
+  if (planes)
+    kEmitHits<<<emitBlocks(slots), 128, 0, ctx->stream>>>(EdgeEmit<true>{es, raw.p}, listed.p, numListed.p, ecnt.p, eoff.p);
+  else
+    kEmitHits<<<emitBlocks(slots), 128, 0, ctx->stream>>>(EdgeEmit<false>{esFar, raw.p}, listed.p, numListed.p, ecnt.p,
+                                                          eoff.p);
   ITS_LAUNCHED(ctx);
   ecnt.reset();
   eoff.reset();
