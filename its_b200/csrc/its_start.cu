@@ -346,9 +346,11 @@ its_status fitResidualEnqueue(its_ctx* ctx, its_svo* const* svos, int64_t count,
   DevBuf<double> H;
   if ((st = H.alloc(ctx, std::max<int64_t>(total, 1))) != ITS_OK) return st;
   // The bands: above the finest depth in one, or a depth each where those rows are many enough to
-  // outweigh the launches (24 octrees, 1.8 million rows above the finest depth: the residual 779 us
-  // in two bands, 354 a depth at a time; the benchmark tube's 54,000 take 20 us in one band, about
-  // the time of 8 launches that wait for one another). Mesh m owns slots [mFirst[m], mFirst[m+1]): its chunks, coarsest band first.
+  // outweigh the launches, which wait for one another. A residual call in two bands and a depth at a
+  // time, us, with the rows above the finest depth: 54,000 (the benchmark tube) 53 and 88; 108,000 78 and
+  // 92; 144,000 92 and 94; 180,000 107 and 100; 216,000 114 and 106; 431,000 209 and 179; 886,000 486 and
+  // 331 (one octree of 512, 196,000: 96 and 100). Mesh m owns slots [mFirst[m], mFirst[m+1]): its chunks,
+  // coarsest band first.
   int64_t above = 0;
   int maxDepth = 1;
   for (int64_t m = 0; m < count; ++m) {
