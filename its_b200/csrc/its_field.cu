@@ -163,16 +163,8 @@ __device__ inline double fieldAt(const EvalParams& P, const double* __restrict__
   return sum;
 }
 
-// Field on the (R+1)^3 lattice in bricks of 32 x 4 x 2 points (one per thread). For each
-// depth the brick's points fall in a small box of cells; the corners of that box (presence,
-// coefficient, representative position) are staged in shared memory once, and every point
-// then sums its 8 corners from there -- the same additions in the same order as fieldAt, so
-// the result is bit-identical, without the per-point lattice lookups (bitmap, rank, vertex
-// position) that made the point-wise kernel L2-bound. Depths whose corner box exceeds the
-// tile (grids much coarser than the octree) fall back to the point-wise lookups.
 constexpr int kBrickThreads = 256, kTileCap = 640;
-
-// Field on the (R+1)^3 lattice in bricks of 32 x 4 x 8 points; a thread evaluates a column of
+// The FP64 field on the (R+1)^3 lattice in bricks of 32 x 4 x 8 points; a thread evaluates a column of
 // 4 points along z. For each depth the brick's points fall in a small box of cells; the
 // corners of that box (presence, coefficient, representative position) are staged in shared
 // memory once, and every point then sums its 8 corners from there -- the same additions in
@@ -181,27 +173,12 @@ constexpr int kBrickThreads = 256, kTileCap = 640;
 // inputs, equal IEEE results); all quotients use divRn. Depths whose corner box has no
 // corner are skipped; depths whose box exceeds the tile (grids much coarser than the octree)
 // fall back to per-point lookups.
-template <typename T>
-__device__ __forceinline__ T quotT(T a, T w, T wi) {
-  if constexpr (sizeof(T) == 8) return divRn(a, w, wi);
-  else return a * wi;
-}
-template <typename T>
-__device__ __forceinline__ T hatT(T x, T p, T w, T wi) {
-  if constexpr (sizeof(T) == 8) {
-    return hat1r(x, p, w, wi);
-  } else {
-    if (x <= p - w || x >= p + w) return T(0);
-    return x <= p ? T(1) + (x - p) * wi : T(1) - (x - p) * wi;
-  }
-}
-
-template <typename T, int kBrickX, int kBrickY, int kZPer>
+template <int kBrickX, int kBrickY, int kZPer>
 __global__ void __launch_bounds__(kBrickThreads, 2)
     kEvalGridBricks(const __grid_constant__ EvalParams P, const double* __restrict__ lambda, double3 o, double3 vs,
-                    int R, T* __restrict__ field) {
+                    int R, double* __restrict__ field) {
   constexpr int kBrickZ = (kBrickThreads / (kBrickX * kBrickY)) * kZPer;
-  __shared__ T tLam[kTileCap], tPx[kTileCap], tPy[kTileCap], tPz[kTileCap];
+  __shared__ double tLam[kTileCap], tPx[kTileCap], tPy[kTileCap], tPz[kTileCap];
   __shared__ unsigned char tHas[kTileCap];
   __shared__ int64_t box[6];  // first and last cell per axis at the current depth
   const int64_t M = (int64_t)R + 1;
@@ -211,17 +188,16 @@ __global__ void __launch_bounds__(kBrickThreads, 2)
   const int64_t xi = x0 + (tid % kBrickX), yj = y0 + ((tid / kBrickX) % kBrickY);
   const int64_t zb = z0 + (int64_t)(tid / (kBrickX * kBrickY)) * kZPer;
   const bool inXY = xi < M && yj < M;
-  const T px = (T)(o.x + (double)xi * vs.x), py = (T)(o.y + (double)yj * vs.y);
-  const T gx = (T)P.g.x, gy = (T)P.g.y, gz = (T)P.g.z;
-  T pz[kZPer], sum[kZPer];
+  const double px = o.x + (double)xi * vs.x, py = o.y + (double)yj * vs.y;
+  const double gx = P.g.x, gy = P.g.y, gz = P.g.z;
+  double pz[kZPer], sum[kZPer];
 #pragma unroll
   for (int q = 0; q < kZPer; ++q) {
-    pz[q] = (T)(o.z + (double)(zb + q) * vs.z);
-    sum[q] = T(0);
+    pz[q] = o.z + (double)(zb + q) * vs.z;
+    sum[q] = 0.0;
   }
   for (int d = 0; d < P.depth; ++d) {
-    const double wd = P.w0 * (double)(1u << d), wid = P.winv[d];
-    const T w = (T)wd, wi = (T)wid;
+    const double w = P.w0 * (double)(1u << d), wi = P.winv[d];
     const LatticeIndex& L = P.lat[d];
     const int64_t lim = (int64_t)(P.res >> d);
     if (tid < 6) {
@@ -232,8 +208,7 @@ __global__ void __launch_bounds__(kBrickThreads, 2)
       const double oa = a == 0 ? o.x : a == 1 ? o.y : o.z, va = a == 0 ? vs.x : a == 1 ? vs.y : vs.z;
       const double ga = a == 0 ? P.g.x : a == 1 ? P.g.y : P.g.z;
       const double pa = oa + (double)cl * va;
-      box[tid] = sizeof(T) == 8 ? (int64_t)floor(divRn(pa - ga, wd, wid))
-                                : (int64_t)floorf(quotT<T>((T)pa - (T)ga, w, wi));
+      box[tid] = (int64_t)floor(divRn(pa - ga, w, wi));
     }
     __syncthreads();
     const int64_t cx0 = box[0], cy0 = box[2], cz0 = box[4];
@@ -250,15 +225,15 @@ __global__ void __launch_bounds__(kBrickThreads, 2)
           if (latticeHas(L, lin)) {
             const uint32_t v = latticeRank(L, lin);
             const double qx = P.vertPos[3 * v], qy = P.vertPos[3 * v + 1], qz = P.vertPos[3 * v + 2];
-            tLam[t] = (T)lambda[v];
-            tPx[t] = (T)qx;
-            tPy[t] = (T)qy;
-            tPz[t] = (T)qz;
+            tLam[t] = lambda[v];
+            tPx[t] = qx;
+            tPy[t] = qy;
+            tPz[t] = qz;
             // bit 0: present; bits 1-3: the x / y / z coordinate is the lattice coordinate
-            // g + w X, so the column's shared factor for that axis applies (FP32: always)
-            has = (unsigned char)(1 | ((sizeof(T) == 4 || qx == latticePos(P.g.x, wd, (uint32_t)Lx)) ? 2 : 0) |
-                                  ((sizeof(T) == 4 || qy == latticePos(P.g.y, wd, (uint32_t)Ly)) ? 4 : 0) |
-                                  ((sizeof(T) == 4 || qz == latticePos(P.g.z, wd, (uint32_t)Lz)) ? 8 : 0));
+            // g + w X, so the column's shared factor for that axis applies
+            has = (unsigned char)(1 | (qx == latticePos(P.g.x, w, (uint32_t)Lx) ? 2 : 0) |
+                                  (qy == latticePos(P.g.y, w, (uint32_t)Ly) ? 4 : 0) |
+                                  (qz == latticePos(P.g.z, w, (uint32_t)Lz) ? 8 : 0));
           }
         }
         tHas[t] = has;
@@ -269,24 +244,24 @@ __global__ void __launch_bounds__(kBrickThreads, 2)
       __syncthreads();
     }
     if (any && inXY) {
-      const int64_t cx = (int64_t)floor(quotT<T>(px - gx, w, wi)), cy = (int64_t)floor(quotT<T>(py - gy, w, wi));
+      const int64_t cx = (int64_t)floor(divRn(px - gx, w, wi)), cy = (int64_t)floor(divRn(py - gy, w, wi));
       // the lattice factors of this column's cell: x and y shared by its 4 points
-      const T fx[2] = {hatT<T>(px, (T)latticePos(P.g.x, wd, (uint32_t)cx), w, wi),
-                       hatT<T>(px, (T)latticePos(P.g.x, wd, (uint32_t)(cx + 1)), w, wi)};
-      const T fy[2] = {hatT<T>(py, (T)latticePos(P.g.y, wd, (uint32_t)cy), w, wi),
-                       hatT<T>(py, (T)latticePos(P.g.y, wd, (uint32_t)(cy + 1)), w, wi)};
+      const double fx[2] = {hat1r(px, latticePos(P.g.x, w, (uint32_t)cx), w, wi),
+                            hat1r(px, latticePos(P.g.x, w, (uint32_t)(cx + 1)), w, wi)};
+      const double fy[2] = {hat1r(py, latticePos(P.g.y, w, (uint32_t)cy), w, wi),
+                            hat1r(py, latticePos(P.g.y, w, (uint32_t)(cy + 1)), w, wi)};
 #pragma unroll
       for (int q = 0; q < kZPer; ++q) {
         if (zb + q >= M) break;
-        const T pzq = pz[q];
-        const int64_t cz = (int64_t)floor(quotT<T>(pzq - gz, w, wi));
-        const T fz[2] = {hatT<T>(pzq, (T)latticePos(P.g.z, wd, (uint32_t)cz), w, wi),
-                         hatT<T>(pzq, (T)latticePos(P.g.z, wd, (uint32_t)(cz + 1)), w, wi)};
-        T s = sum[q];
+        const double pzq = pz[q];
+        const int64_t cz = (int64_t)floor(divRn(pzq - gz, w, wi));
+        const double fz[2] = {hat1r(pzq, latticePos(P.g.z, w, (uint32_t)cz), w, wi),
+                              hat1r(pzq, latticePos(P.g.z, w, (uint32_t)(cz + 1)), w, wi)};
+        double s = sum[q];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const int ox = k & 1, oy = (k >> 1) & 1, oz = (k >> 2) & 1;
-          T lam;
+          double lam;
           unsigned f;
           int t = 0;
           uint32_t vv = 0;
@@ -301,21 +276,21 @@ __global__ void __launch_bounds__(kBrickThreads, 2)
             const uint32_t lin = (uint32_t)((Lx * L.M + Ly) * L.M + Lz);
             if (!latticeHas(L, lin)) continue;
             vv = latticeRank(L, lin);
-            lam = (T)lambda[vv];
-            f = sizeof(T) == 4 ? 15u : 1u;  // FP64: positions from the vertex array
+            lam = lambda[vv];
+            f = 1u;  // positions from the vertex array
           }
           // hat3 as the reference forms it: x, y, z factors with early exits; a factor at the
           // lattice coordinate is the column's shared one (equal inputs, equal IEEE result)
-          T hx, hy, hz;
+          double hx, hy, hz;
           if (f & 2) hx = fx[ox];
-          else hx = hatT<T>(px, tiled ? tPx[t] : (T)P.vertPos[3 * (int64_t)vv], w, wi);
-          if (hx <= T(0)) continue;
+          else hx = hat1r(px, tiled ? tPx[t] : P.vertPos[3 * (int64_t)vv], w, wi);
+          if (hx <= 0.0) continue;
           if (f & 4) hy = fy[oy];
-          else hy = hatT<T>(py, tiled ? tPy[t] : (T)P.vertPos[3 * (int64_t)vv + 1], w, wi);
-          if (hy <= T(0)) continue;
+          else hy = hat1r(py, tiled ? tPy[t] : P.vertPos[3 * (int64_t)vv + 1], w, wi);
+          if (hy <= 0.0) continue;
           if (f & 8) hz = fz[oz];
-          else hz = hatT<T>(pzq, tiled ? tPz[t] : (T)P.vertPos[3 * (int64_t)vv + 2], w, wi);
-          if (hz <= T(0)) continue;
+          else hz = hat1r(pzq, tiled ? tPz[t] : P.vertPos[3 * (int64_t)vv + 2], w, wi);
+          if (hz <= 0.0) continue;
           s += lam * (hx * hy * hz);
         }
         sum[q] = s;
@@ -1062,13 +1037,13 @@ __global__ void __launch_bounds__(kScanThreads) kMcEmit(McCaseT<T> mc, FastDiv b
 
 // Dense-field launch shapes (bricks of BX x BY x BZ points, a thread per column of ZPER
 // points); every shape computes the same bits, the autotuner picks the fastest.
-template <typename T, int BX, int BY, int ZPER>
+template <int BX, int BY, int ZPER>
 static its_status launchBricks(its_ctx* ctx, const EvalParams& P, const double* lam, double3 o, double3 vs, int res,
-                               T* field) {
+                               double* field) {
   constexpr int BZ = (kBrickThreads / (BX * BY)) * ZPER;
   const int64_t M = (int64_t)res + 1;
   const dim3 grid((unsigned)((M + BX - 1) / BX), (unsigned)((M + BY - 1) / BY), (unsigned)((M + BZ - 1) / BZ));
-  kEvalGridBricks<T, BX, BY, ZPER><<<grid, kBrickThreads, 0, ctx->stream>>>(P, lam, o, vs, res, field);
+  kEvalGridBricks<BX, BY, ZPER><<<grid, kBrickThreads, 0, ctx->stream>>>(P, lam, o, vs, res, field);
   ITS_LAUNCHED(ctx);
   return ITS_OK;
 }
@@ -1119,10 +1094,10 @@ static its_status evalGridTuned(its_ctx* ctx, const SvoDevice& d, const double* 
     }
     if constexpr (sizeof(T) == 8) {
       switch (cand[j]) {
-        case 1: return launchBricks<T, 32, 8, 2>(ctx, P, lam, o, vs, res, field);
-        case 2: return launchBricks<T, 64, 4, 2>(ctx, P, lam, o, vs, res, field);
-        case 3: return launchBricks<T, 16, 4, 4>(ctx, P, lam, o, vs, res, field);
-        default: return launchBricks<T, 32, 4, 4>(ctx, P, lam, o, vs, res, field);
+        case 1: return launchBricks<32, 8, 2>(ctx, P, lam, o, vs, res, field);
+        case 2: return launchBricks<64, 4, 2>(ctx, P, lam, o, vs, res, field);
+        case 3: return launchBricks<16, 4, 4>(ctx, P, lam, o, vs, res, field);
+        default: return launchBricks<32, 4, 4>(ctx, P, lam, o, vs, res, field);
       }
     }
     return ITS_ERR_STATE;
