@@ -66,19 +66,16 @@ __device__ __forceinline__ float2 geluGrad2(float2 z) {
                     __fmul2_rn(half, __fadd2_rn(one, t)));
 }
 
-// ---- one tcgen05 GEMM: C[m][n] = sum_k A[m][k] B[n][k] over this CTA's K range -------------
+// ---- one tcgen05 GEMM: C[m][n] = sum_k A[m][k] B[n][k], n < 128 -----------------------------
 // 128 rows per CTA and four warp groups: 64-wide K chunks are fetched by all 512 threads with
 // cp.async into one of two stages while the tensor core multiplies the other; the accumulator
 // (TMEM) is read back by each warp group for a quarter of the columns (thread = row, the TMEM
-// lane of its warp) and handed to the epilogue functor with that quarter.
+// lane of its warp) and handed to the epilogue functor with that quarter. K is a multiple of 64.
 constexpr int kGemmGroups = 4;
 constexpr int kGemmThreads = 128 * kGemmGroups;
-template <int N>
-struct GemmSmem {
-  static constexpr int kA = 128 * 128, kB = N * 128, kStage = kA + kB;
-  // two stages, the epilogue's per-group row partials and per-row value, mbarriers, TMEM slot
-  static constexpr int kBytes = 2 * kStage + (kGemmGroups + 1) * 128 * 4 + 64 + 1024;
-};
+constexpr int kGemmStage = 2 * 128 * 128;  // a chunk of A and one of B
+// two stages, the epilogue's per-group row partials, mbarriers, TMEM slot
+constexpr int kGemmSmem = 2 * kGemmStage + kGemmGroups * 128 * 4 + 64 + 1024;
 
 // 16 bytes global -> shared without staging through registers; bytes < 16 zero-fills the rest.
 __device__ __forceinline__ void cpAsync16(uint32_t dst, const void* src, uint32_t bytes) {
@@ -90,23 +87,19 @@ __device__ __forceinline__ void cpAsyncWait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(Pending) : "memory");
 }
 
-template <int N, class Epi>
-__global__ void __launch_bounds__(kGemmThreads, 2) kUmmaGemm(const bf16* __restrict__ A, int64_t lda, int64_t M,
-                                                             const bf16* __restrict__ B, int64_t ldb, int64_t K,
-                                                             int64_t kPerSplit, Epi epi, int* __restrict__ err) {
+template <class Epi>
+__global__ void __launch_bounds__(kGemmThreads, 2) kUmmaGemm(const bf16* __restrict__ A, int64_t M,
+                                                             const bf16* __restrict__ B, int K, Epi epi,
+                                                             int* __restrict__ err) {
   using namespace umma;
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
-  float* sPart = (float*)(smem + 2 * GemmSmem<N>::kStage);  // [group][row]
-  float* sRow = sPart + kGemmGroups * 128;                  // [row]
-  uint64_t* mbar = (uint64_t*)(sRow + 128);                 // one per stage
+  float* sPart = (float*)(smem + 2 * kGemmStage);          // [group][row]
+  uint64_t* mbar = (uint64_t*)(sPart + kGemmGroups * 128);  // one per stage
   uint32_t* slot = (uint32_t*)(mbar + 2);
   const int tid = threadIdx.x, warp = tid >> 5, grp = tid >> 7, row = tid & 127;
   const int64_t m0 = (int64_t)blockIdx.x * 128;
-  const int64_t k0 = (int64_t)blockIdx.z * kPerSplit;
-  const int64_t k1 = k0 + kPerSplit < K ? k0 + kPerSplit : K;
-  constexpr uint32_t kCols = N < 32 ? 32 : N;
-  if (warp == 0) tmemAlloc(smemAddr(slot), kCols);
+  if (warp == 0) tmemAlloc(smemAddr(slot), 128);
   if (tid == 0) {
     mbarInit(smemAddr(mbar), 1);
     mbarInit(smemAddr(mbar + 1), 1);
@@ -115,31 +108,24 @@ __global__ void __launch_bounds__(kGemmThreads, 2) kUmmaGemm(const bf16* __restr
   __syncthreads();
   fenceAfter();
   const uint32_t tmem = *slot;
-  constexpr uint32_t idesc = idescBf16(128, N);
-  // chunk kc into stage st; columns past the split's end (and rows past M) read as zeros
-  auto load = [&](int st, int64_t kc) {
-    uint8_t* sA = smem + st * GemmSmem<N>::kStage;
-    uint8_t* sB = sA + GemmSmem<N>::kA;
+  constexpr uint32_t idesc = idescBf16(128, 128);
+  // chunk kc into stage st; rows past M read as zeros
+  auto load = [&](int st, int kc) {
+    uint8_t* sA = smem + st * kGemmStage;
+    uint8_t* sB = sA + kGemmStage / 2;
     for (int i = tid; i < 128 * 8; i += kGemmThreads) {
-      const int r = i >> 3, c = i & 7;
-      const int64_t col = kc + c * 8, left = k1 - col;
-      const uint32_t bytes = (m0 + r < M && left > 0) ? (uint32_t)(left >= 8 ? 16 : 2 * left) : 0u;
-      cpAsync16(smemAddr(sA + swizzledChunk(r, c)), bytes ? (const void*)(A + (m0 + r) * lda + col) : (const void*)A,
-                bytes);
-    }
-    for (int i = tid; i < N * 8; i += kGemmThreads) {
-      const int r = i >> 3, c = i & 7;
-      const int64_t col = kc + c * 8, left = k1 - col;
-      const uint32_t bytes = left > 0 ? (uint32_t)(left >= 8 ? 16 : 2 * left) : 0u;
-      cpAsync16(smemAddr(sB + swizzledChunk(r, c)), bytes ? (const void*)(B + (int64_t)r * ldb + col) : (const void*)B,
-                bytes);
+      const int r = i >> 3, c = i & 7, col = kc + c * 8;
+      const bool in = m0 + r < M;
+      cpAsync16(smemAddr(sA + swizzledChunk(r, c)), in ? (const void*)(A + (m0 + r) * K + col) : (const void*)A,
+                in ? 16u : 0u);
+      cpAsync16(smemAddr(sB + swizzledChunk(r, c)), B + (int64_t)r * K + col, 16u);
     }
     cpAsyncCommit();
   };
-  const int nk = k1 > k0 ? (int)((k1 - k0 + 63) / 64) : 0;
+  const int nk = K / 64;
   uint32_t ph[2] = {0u, 0u};
   bool ok = true;
-  if (nk > 0) load(0, k0);
+  load(0, 0);
   for (int c = 0; c < nk; ++c) {
     const int st = c & 1;
     if (c + 1 < nk) {
@@ -147,7 +133,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) kUmmaGemm(const bf16* __restr
         ok = mbarWait(smemAddr(mbar + (st ^ 1)), ph[st ^ 1]) && ok;
         ph[st ^ 1] ^= 1u;
       }
-      load(st ^ 1, k0 + (int64_t)(c + 1) * 64);
+      load(st ^ 1, (c + 1) * 64);
       cpAsyncWait<1>();  // this chunk's copies (the next chunk's may still be in flight)
     } else {
       cpAsyncWait<0>();
@@ -156,44 +142,32 @@ __global__ void __launch_bounds__(kGemmThreads, 2) kUmmaGemm(const bf16* __restr
     __syncthreads();
     if (tid == 0) {
       fenceAfter();
-      const uint8_t* sA = smem + st * GemmSmem<N>::kStage;
-      const uint64_t da = descSw128(smemAddr(sA)), db = descSw128(smemAddr(sA + GemmSmem<N>::kA));
+      const uint8_t* sA = smem + st * kGemmStage;
+      const uint64_t da = descSw128(smemAddr(sA)), db = descSw128(smemAddr(sA + kGemmStage / 2));
 #pragma unroll
       for (int k = 0; k < 4; ++k) mma(tmem, da + 2 * k, db + 2 * k, idesc, (c > 0 || k > 0) ? 1u : 0u);
       commit(smemAddr(mbar + st));
     }
   }
-  if (nk > 0) {  // the last chunk's products (and with them every earlier one)
-    const int st = (nk - 1) & 1;
-    ok = mbarWait(smemAddr(mbar + st), ph[st]) && ok;
-  }
+  const int last = (nk - 1) & 1;  // the last chunk's products (and with them every earlier one)
+  ok = mbarWait(smemAddr(mbar + last), ph[last]) && ok;
   fenceAfter();
-  constexpr int C = N / kGemmGroups;
-  static_assert(C == 16 || C == 32, "a quarter of the columns per warp group");
+  constexpr int C = 128 / kGemmGroups;
+  static_assert(C == 32, "a quarter of the columns per warp group");
   float v[C];
   const uint32_t lane = (uint32_t)((warp & 3) * 32) << 16;
-  if constexpr (C == 32) {
-    tmemLoad32(tmem + lane + (uint32_t)(grp * C), v);
-  } else {
-    tmemLoad16(tmem + lane + (uint32_t)(grp * C), v);
-  }
-  if (k1 <= k0) {  // an empty split contributes zeros
-#pragma unroll
-    for (int j = 0; j < C; ++j) v[j] = 0.0f;
-  }
+  tmemLoad32(tmem + lane + (uint32_t)(grp * C), v);
   const int64_t m = m0 + row;
-  epi(m, ok && m < M, grp * C, v, sPart, sRow, grp, smem, m0, M);  // the stages are free: the products are done
+  epi(m, ok && m < M, grp * C, v, sPart, grp, smem, m0, M);  // the stages are free: the products are done
   fenceBefore();
   __syncthreads();
-  if (warp == 0) tmemFree(tmem, kCols);
+  if (warp == 0) tmemFree(tmem, 128);
   if (!ok && tid == 0) atomicExch(err, 1);
 }
 
 // ---- epilogues ----------------------------------------------------------------------------
 // Each is called by every thread with its row m, whether the row is written (valid), the first
-// column j0 of its warp group's quarter and that quarter's accumulators. The row-major stores
-// go out in 16-byte pieces (eight BF16 or four FP32 values per store); the transposed copies are
-// coalesced across the warp as they are.
+// column j0 of its warp group's quarter and that quarter's accumulators.
 __device__ __forceinline__ uint4 packBf16x8(const float* v) {
   uint4 r;
   __nv_bfloat162* q = (__nv_bfloat162*)&r;
@@ -228,7 +202,7 @@ struct EpiHidden {
   const float* bias;
   bf16* H;
   template <int C>
-  __device__ void operator()(int64_t m, bool valid, int j0, float (&v)[C], float*, float*, int, uint8_t* stage,
+  __device__ void operator()(int64_t m, bool valid, int j0, float (&v)[C], float*, int, uint8_t* stage,
                              int64_t m0, int64_t M) const {
     const int row = threadIdx.x & 127;
     if (valid) {
@@ -258,7 +232,7 @@ struct EpiOutput {
   const float* b4;
   float* out;
   template <int C>
-  __device__ void operator()(int64_t m, bool valid, int j0, float (&v)[C], float* sPart, float*, int grp, uint8_t*,
+  __device__ void operator()(int64_t m, bool valid, int j0, float (&v)[C], float* sPart, int grp, uint8_t*,
                              int64_t, int64_t) const {
     const int row = threadIdx.x & 127;
     float o = 0.0f;
@@ -920,18 +894,10 @@ __global__ void kAdam(float* __restrict__ P, float* __restrict__ Mo, float* __re
   P[i] -= lr * (m / c1) / (sqrtf(v / c2) + eps);
 }
 
-template <int N, class Epi>
-static its_status gemm(its_ctx* ctx, const bf16* A, int64_t lda, int64_t M, const bf16* B, int64_t ldb, int64_t K,
-                       int splits, const Epi& epi, int* err) {
-  static bool configured = false;
-  if (!configured) {
-    ITS_CU(ctx, cudaFuncSetAttribute(kUmmaGemm<N, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     GemmSmem<N>::kBytes));
-    configured = true;
-  }
-  const int64_t kPer = ((K / splits + 63) / 64) * 64;
-  dim3 grid((unsigned)((M + 127) / 128), 1, (unsigned)splits);
-  kUmmaGemm<N, Epi><<<grid, kGemmThreads, GemmSmem<N>::kBytes, ctx->stream>>>(A, lda, M, B, ldb, K, kPer, epi, err);
+template <class Epi>
+static its_status gemm(its_ctx* ctx, const bf16* A, int64_t M, const bf16* B, int K, const Epi& epi, int* err) {
+  ITS_CU(ctx, cudaFuncSetAttribute(kUmmaGemm<Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem));
+  kUmmaGemm<Epi><<<gridFor(M, 128), kGemmThreads, kGemmSmem, ctx->stream>>>(A, M, B, K, epi, err);
   ITS_LAUNCHED(ctx);
   return ITS_OK;
 }
@@ -982,11 +948,11 @@ static its_status mlpCast(its_mlp* h) {
 static its_status mlpForward(its_mlp* h, int64_t n, float* out) {
   its_ctx* ctx = h->ctx;
   its_status st;
-  if ((st = gemm<kHid>(ctx, h->Xb, kIn, n, h->W1, kIn, kIn, 1, EpiHidden{h->P + kOffB1, h->H1}, h->err)) != ITS_OK ||
-      (st = gemm<kHid>(ctx, h->H1, kHid, n, h->W2, kHid, kHid, 1, EpiHidden{h->P + kOffB2, h->H2}, h->err)) != ITS_OK)
+  if ((st = gemm(ctx, h->Xb, n, h->W1, kIn, EpiHidden{h->P + kOffB1, h->H1}, h->err)) != ITS_OK ||
+      (st = gemm(ctx, h->H1, n, h->W2, kHid, EpiHidden{h->P + kOffB2, h->H2}, h->err)) != ITS_OK)
     return st;
   const EpiOutput e3{h->P + kOffB3, h->w4r, h->P + kOffB4, out};
-  return gemm<kHid>(ctx, h->H2, kHid, n, h->W3, kHid, kHid, 1, e3, h->err);
+  return gemm(ctx, h->H2, n, h->W3, kHid, e3, h->err);
 }
 
 // Gradient of the mean squared error over n rows of X (targets y), drawn as rows says, into h->G.
