@@ -424,10 +424,7 @@ __global__ void __launch_bounds__(128) kWideNodes(BvhDevice B, const BoxF* __res
     w.leaves = -1;
     if (j < k) {
       const int32_t c = slot[j];
-      // one triangle alone has no box (its leaf never climbs): the whole space
-      const float inf = __int_as_float(0x7f800000);
-      BoxF b{{-inf, -inf, -inf}, {inf, inf, inf}};
-      if (n > 1) b = box[c < 0 ? (n - 1) + (-(int64_t)c - 1) : c];
+      const BoxF b = box[c < 0 ? (n - 1) + (-(int64_t)c - 1) : c];
       for (int a = 0; a < 3; ++a) {
         w.lo[a] = b.lo[a];
         w.hi[a] = b.hi[a];

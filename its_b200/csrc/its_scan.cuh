@@ -1,4 +1,5 @@
-// Exclusive prefix sums (reduce-then-scan, three launches, no inter-block waiting).
+// Exclusive prefix sums (reduce-then-scan, no inter-block waiting): one launch for a few tiles, three
+// (sums, spine, prefixes) in general, five where the spine is long enough for tiles of its own.
 // The input is produced by a functor so that flags, popcounts or counts need not be
 // materialised. Used for stream compaction of Morton codes, lattice ranks, CSR row
 // pointers and marching-cubes offsets.
