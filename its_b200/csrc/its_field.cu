@@ -173,6 +173,13 @@ constexpr int kBrickThreads = 256, kTileCap = 640;
 // inputs, equal IEEE results); all quotients use divRn. Depths whose corner box has no
 // corner are skipped; depths whose box exceeds the tile (grids much coarser than the octree)
 // fall back to per-point lookups.
+// The cell at distance a from the lattice's first point; one outside the lattice's cells 0 .. lim touches no
+// corner and is kept next to them, so that boxes stay small.
+__device__ __forceinline__ int64_t cellOf(double a, double w, double wi, int64_t lim) {
+  const int64_t c = (int64_t)floor(divRn(a, w, wi));
+  return c < -2 ? -2 : (c > lim + 1 ? lim + 1 : c);
+}
+
 template <int kBrickX, int kBrickY, int kZPer>
 __global__ void __launch_bounds__(kBrickThreads, 2)
     kEvalGridBricks(const __grid_constant__ EvalParams P, const double* __restrict__ lambda, double3 o, double3 vs,
@@ -208,12 +215,13 @@ __global__ void __launch_bounds__(kBrickThreads, 2)
       const double oa = a == 0 ? o.x : a == 1 ? o.y : o.z, va = a == 0 ? vs.x : a == 1 ? vs.y : vs.z;
       const double ga = a == 0 ? P.g.x : a == 1 ? P.g.y : P.g.z;
       const double pa = oa + (double)cl * va;
-      box[tid] = (int64_t)floor(divRn(pa - ga, w, wi));
+      box[tid] = cellOf(pa - ga, w, wi, lim);
     }
     __syncthreads();
     const int64_t cx0 = box[0], cy0 = box[2], cz0 = box[4];
     const int nx = (int)(box[1] - cx0 + 2), ny = (int)(box[3] - cy0 + 2), nz = (int)(box[5] - cz0 + 2);
-    const bool tiled = (int64_t)nx * ny * nz <= kTileCap;  // block-uniform
+    // block-uniform (a lattice that runs backwards has no box)
+    const bool tiled = nx > 1 && ny > 1 && nz > 1 && (int64_t)nx * ny * nz <= kTileCap;
     int any = 1;
     if (tiled) {
       int mine = 0;
@@ -244,7 +252,7 @@ __global__ void __launch_bounds__(kBrickThreads, 2)
       __syncthreads();
     }
     if (any && inXY) {
-      const int64_t cx = (int64_t)floor(divRn(px - gx, w, wi)), cy = (int64_t)floor(divRn(py - gy, w, wi));
+      const int64_t cx = cellOf(px - gx, w, wi, lim), cy = cellOf(py - gy, w, wi, lim);
       // the lattice factors of this column's cell: x and y shared by its 4 points
       const double fx[2] = {hat1r(px, latticePos(P.g.x, w, (uint32_t)cx), w, wi),
                             hat1r(px, latticePos(P.g.x, w, (uint32_t)(cx + 1)), w, wi)};
@@ -254,7 +262,7 @@ __global__ void __launch_bounds__(kBrickThreads, 2)
       for (int q = 0; q < kZPer; ++q) {
         if (zb + q >= M) break;
         const double pzq = pz[q];
-        const int64_t cz = (int64_t)floor(divRn(pzq - gz, w, wi));
+        const int64_t cz = cellOf(pzq - gz, w, wi, lim);
         const double fz[2] = {hat1r(pzq, latticePos(P.g.z, w, (uint32_t)cz), w, wi),
                               hat1r(pzq, latticePos(P.g.z, w, (uint32_t)(cz + 1)), w, wi)};
         double s = sum[q];
@@ -1050,7 +1058,7 @@ static its_status launchBricks(its_ctx* ctx, const EvalParams& P, const double* 
 
 // Corners per axis of the cell box that n consecutive lattice points span at the finest depth
 // (one more than the exact bound, for the rounding of the cell quotients).
-static int64_t boxCorners(int n, double v, double w0) { return (int64_t)std::floor((n - 1) * v / w0) + 3; }
+static double boxCorners(int n, double v, double w0) { return std::floor((n - 1) * std::fabs(v) / w0) + 3; }
 
 template <typename T>
 static its_status evalGridTuned(its_ctx* ctx, const SvoDevice& d, const double* lam, double3 o, double3 vs, int res,
@@ -1062,7 +1070,7 @@ static its_status evalGridTuned(its_ctx* ctx, const SvoDevice& d, const double* 
   // separable kernel's two shapes. Coarser grids: the separable kernel with the large tile, the
   // deeper brick by default where its box fits (torus of 99,000 faces, octree 256, grid 256: 3.52
   // ms point by point in bricks of 32 x 4 x 8).
-  auto boxFits = [&](int z, int64_t cap) {
+  auto boxFits = [&](int z, int cap) {
     return boxCorners(kSepX, vs.x, d.unit[0]) * boxCorners(kSepY, vs.y, d.unit[0]) * boxCorners(z, vs.z, d.unit[0]) <=
            cap;
   };
