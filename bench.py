@@ -895,7 +895,7 @@ def run_batch(ctx, net, norm, timed, tol, world, rank, steps, pg):
            "speedup": round(tot["plain_ms"] / tot["learned_ms"], 2),
            "sharding": ("LPT by faces over %d ranks" % world) if world > 1 else "single",
            "mc_256": {"ms": round(tot["mc_ms"], 2), "mvox_s": round(256 * R ** 3 / (tot["mc_ms"] * 1e-3) / 1e6, 1),
-                      "triangles": int(tot["triangles"]), "iso": 0.0, "field": "FP64, point by point (its_eval_grid)"},
+                      "triangles": int(tot["triangles"]), "iso": 0.0, "field": "FP64, bit-exact (its_eval_grid)"},
            "mc_256_fast": {"ms": round(tot["mc_fast_ms"], 2),
                            "mvox_s": round(256 * R ** 3 / (tot["mc_fast_ms"] * 1e-3) / 1e6, 1),
                            "triangles": int(tot["triangles_fast"]), "iso": 0.0,

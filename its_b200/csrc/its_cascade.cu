@@ -191,7 +191,7 @@ static its_status evalGridFast(its_svo* sv, const double* lambda, const double o
   its_ctx* ctx = sv->ctx;
   ITS_CU(ctx, cudaSetDevice(ctx->device));
   int s = 0;
-  if (!alignedLattice(sv->d, origin, width, res, &s)) {  // any other lattice: point by point
+  if (!alignedLattice(sv->d, origin, width, res, &s)) {  // any other lattice: the exact field
     if (sizeof(T) == 8) return its_eval_grid(sv, lambda, origin, width, res, (double*)field);
     return its_eval_grid_f32(sv, lambda, origin, width, res, (float*)field);
   }
